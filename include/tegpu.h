@@ -367,12 +367,12 @@ int te_evolver_krylov_matrix(te_evolver ev, double* diag, double* offdiag, doubl
 
 /* Evolver options (no counterpart in the reference).
  * TE_OPT_FUSED_LANCZOS: run the three-term Lanczos iterations of a Krylov step
- * as one persistent cooperative kernel with grid barriers instead of two
- * launches per iteration (same step sequence; the norm sums round
- * differently).  0: never; 1 (default): for matrices of fewer than 2048
- * 32-row chunks, where launch costs dominate (measured on GB300: 20% faster
- * at dim 6435, equal at dim 92378, slower from dim 352716); 2: always, where
- * a cooperative launch of the matrix's schedule is possible. */
+ * as one persistent cooperative kernel that exchanges its sums between all
+ * blocks, instead of two launches per iteration (same step sequence; the sums
+ * round differently).  0: never; 1 (default): for every matrix without long
+ * rows whose rows fit the kernels' registers (369 664 rows on 152 SMs;
+ * measured on GB300, per iteration: 31 against 11.5 us at dim 92378); 2: the
+ * same with the FP64 SpMV, whatever TE_OPT_FIXED_SPMV says. */
 #define TE_OPT_FUSED_LANCZOS 1
 /* TE_OPT_FIXED_SPMV: the SpMV of the three-term Lanczos passes in integer
  * arithmetic instead of FP64 FMAs (GB300 issues FP64 at 1/58 of its FP32
@@ -383,15 +383,15 @@ int te_evolver_krylov_matrix(te_evolver ev, double* diag, double* offdiag, doubl
  * row of k entries below (1.25 k 2^-56 + (k + 1) 2^-61) R U + 2^-53 |y| for
  * real H, (5 k 2^-56 + (2 k + 1) 2^-61) R U + 2^-53 |y| for complex H, against
  * FP64's k 2^-53 sum|h||u|.  The recurrence and all reductions stay FP64.
- * Applies to the per-iteration passes of matrices of at least 2048 32-row
- * chunks (smaller ones run the persistent FP64 kernel); see
+ * Applies to matrices of at least 2048 32-row chunks (smaller ones run the
+ * persistent FP64 kernel); see
  * te_matrix_fixed_layout for the forms (value dictionary, column blocks).
  * 0: FP64 SpMV; 1 (default): fixed point. */
 #define TE_OPT_FIXED_SPMV 2
 /* Options that bound or exercise the failure paths (no counterpart in the
  * reference, which exits or keeps going where these return an error):
- * TE_OPT_BARRIER_SPIN_LIMIT: polls (each a load and a short sleep) before a
- * grid-barrier wait of the persistent Lanczos kernel gives up; the run then
+ * TE_OPT_BARRIER_SPIN_LIMIT: polls (each a load) before a grid-barrier wait of
+ * the persistent Lanczos kernels gives up; the run then
  * returns TE_ERR_DEVICE_TIMEOUT and the evolver can be reset and run again.
  * Default 2^22 (seconds; a co-resident grid arrives in microseconds).
  * TE_OPT_BARRIER_EXTRA_ARRIVALS: 1 makes every barrier of that kernel wait

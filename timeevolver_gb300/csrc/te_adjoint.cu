@@ -419,6 +419,7 @@ int make_evolver(te_adjoint a, double exp_factor, const std::vector<double>* tim
   te_evolver ev = nullptr;
   int rc = te_evolver_create(a->Hth, a->v0.data(), &p, &ev);
   if (rc != TE_OK) return rc;
+  te_evolver_set_resident(ev, false);
   if (times) rc = te_evolver_set_schedule(ev, times->data(), (int64_t)times->size(), store, a->n);
   if (rc == TE_OK && with_obs) rc = te_evolver_add_sparse_observable(ev, a->O);
   if (rc != TE_OK) {

@@ -73,6 +73,11 @@ struct te_evolver_s {
   int qr_sweeps = 0;                      // TE_OPT_QR_SWEEP_LIMIT (0: 40 m + 40)
   int4* X = nullptr;      // fixed-point copies of the Krylov vectors (m x n rows)
   longlong2* fx_acc = nullptr;  // column-blocked fixed-point SpMV: exact row sums (n rows)
+  TeResidentSync* res_sync = nullptr;  // words of the resident Lanczos kernel
+  unsigned int res_launch = 0;         // its launches so far
+  TeStepSync* step_sync = nullptr;     // words of the small matrices' Lanczos kernel
+  unsigned int step_launch = 0;        // its launches so far
+  bool resident = true;                // te_evolver_set_resident
   TeSegCarry seg;               // carries of H's split long rows (this evolver's passes)
   int batch_cap = 0;         // states the batch buffer holds
   size_t results_cap = 0;    // doubles the results buffer holds
@@ -234,6 +239,8 @@ void free_evolver(te_evolver ev) {
   te_free_host(ev->host_state);
   te_free(ev->slab);
   te_free(ev->X);
+  te_free(ev->res_sync);
+  te_free(ev->step_sync);
   te_seg_carry_free(&ev->seg);
   te_free(ev->fx_acc);
   te_free(ev->batch);
@@ -352,8 +359,17 @@ int run(te_evolver ev, te_result* out) {
   // matrices large enough for the per-iteration passes
   // (its own schedule, one lane per row); otherwise the FP64 passes, whose
   // lanes per row are tuned once per matrix on first use
-  bool fix = ev->fixed_spmv != 0 && ev->p.reorth == 0 && ev->p.exp_factor != 0.0 &&
-             ev->H->sell.n_chunks >= 2048 && ev->fused_lanczos != 2;
+  // all m iterations in one launch: the small matrices' kernel below 2048
+  // chunks, the resident kernel from there on for every matrix that fits,
+  // unless the caller pinned another number of lanes per row.  (per step of
+  // 40 iterations: see te_step.cu, te_resident.cu)
+  const TeSell& sell = ev->H->sell;
+  const bool one_launch = ev->fused_lanczos != 0 && ev->p.reorth == 0 && ev->p.exp_factor != 0.0 && sell.n_long == 0 &&
+                          (sell.lanes == 1 || !(sell.lanes_pinned || sell.lanes_timed));
+  const bool small = one_launch && sell.n_chunks < 2048;
+  const bool resident = one_launch && !small && ev->resident && te_resident_fits(sell);
+  bool fix = ev->fixed_spmv != 0 && ev->p.reorth == 0 && ev->p.exp_factor != 0.0 && sell.n_chunks >= 2048 &&
+             ev->fused_lanczos != 2;
   if (fix) {
     // the fixed-point form and its vectors; without memory for them the
     // evolution runs the FP64 passes instead
@@ -369,6 +385,14 @@ int run(te_evolver ev, te_result* out) {
     }
   }
   if (!fix && (rc = te_tune_sell_lanes(ev->H)) != TE_OK) return rc;
+  if (small && !ev->step_sync) {
+    TE_CUDA(te_malloc(&ev->step_sync, sizeof(TeStepSync)));
+    TE_CUDA(cudaMemsetAsync(ev->step_sync, 0, sizeof(TeStepSync), st));
+  }
+  if (resident && !ev->res_sync) {
+    TE_CUDA(te_malloc(&ev->res_sync, sizeof(TeResidentSync)));
+    TE_CUDA(cudaMemsetAsync(ev->res_sync, 0, sizeof(TeResidentSync), st));
+  }
   while (!S->done) {
     if (S->fatal) break;
     if (++guard > ((int64_t)1 << 40)) break;
@@ -378,21 +402,22 @@ int run(te_evolver ev, te_result* out) {
     const bool cgs2 = ev->p.reorth != 0;
     const bool fold = !cgs2 && ev->p.exp_factor != 0.0;
     bool fused = false;
-    // all m iterations in one persistent launch: measured faster than the
-    // per-iteration passes only while launch costs dominate (dim 6435: -20%;
-    // dim 92378: equal; dim >= 352716: slower), hence the automatic size rule
-    const bool want_fused = ev->fused_lanczos == 2 || (ev->fused_lanczos == 1 && ev->H->sell.n_chunks < 2048);
-    if (fold && want_fused) {
-      ProfScope ps(ev, 0);
-      fused = te_launch_lanczos_step(ev->H->sell, ev->H->is_real, ev->cols, m, ev->w, ev->ds, ev->partials, st,
-                                     ev->barrier_spins, ev->barrier_extra);
-      if (fused) ++ev->launches;
-    }
-    const bool fix_step = fix && fold && !fused;
+    const bool fix_step = fix && fold;
     if (fix_step) {
       ProfScope ps(ev, 3);
       te_launch_fix_start(n, ev->cols[0], ev->X, ev->ds, ev->partials, st);
       ev->launches += 2;
+    }
+    if (small) {
+      ProfScope ps(ev, 0);
+      fused = te_launch_lanczos_step(sell, ev->H->is_real, ev->cols, m, ev->w, ev->ds, ev->step_sync, ev->step_launch,
+                                     st, ev->barrier_spins, ev->barrier_extra);
+      if (fused) ++ev->launches, ++ev->step_launch;
+    } else if (resident) {
+      ProfScope ps(ev, 0);
+      fused = te_launch_lanczos_resident(sell, ev->H->is_real, fix_step, ev->H->norm1, ev->cols, m, ev->X, ev->ds,
+                                         ev->res_sync, ev->res_launch, st, ev->barrier_spins, ev->barrier_extra);
+      if (fused) ++ev->launches, ++ev->res_launch;
     }
     for (int j = 0; j < m && !fused; ++j) {
       {
@@ -840,6 +865,8 @@ int te_evolver_set_schedule(te_evolver ev, const double* times_host, int64_t cou
   ev->store_ld = store_ld;
   return TE_OK;
 }
+
+void te_evolver_set_resident(te_evolver ev, bool on) { ev->resident = on; }
 
 extern "C" int te_evolver_reset(te_evolver ev, const double* v, int v_is_device) {
   if (!ev || !v) {

@@ -134,10 +134,13 @@ struct TeSell {
   int32_t* warp_chunk = nullptr;
   int grid = 0;
   bool saturated = false;  // the grid is capped at every SM's resident blocks
+  int warp_chunks = 0;     // most chunks of one warp of the schedule
+  int64_t block_slots = 0; // most slots of one block of the schedule
   // lanes per row of the SpMV passes (1, 2 or 4), chosen by te_tune_sell_lanes
   // or set through te_matrix_set_spmv_lanes; lanes_fixed once chosen
   int lanes = 1;
   bool lanes_fixed = false;
+  bool lanes_pinned = false;  // 1, 2 or 4 set by the caller
   bool lanes_timed = false;  // chosen by timing the variants (te_matrix_set_spmv_lanes(A, -1))
   // Long rows: rows longer than max(1024, 32 x mean length) -- the first n_long
   // rows of the sorted order -- have no slots in the chunks (one of them would
@@ -381,15 +384,34 @@ void te_launch_lanczos_apply_fix(const TeSell& A, const int4* X, const double2* 
 void te_sell_schedule(const std::vector<int64_t>& off, int64_t n_chunks, int blocks_per_sm,
                       bool real, int& grid, bool& saturated, std::vector<int32_t>& wc);
 // All m three-term Lanczos iterations of one Krylov step in one cooperative
-// launch (te_lanczos.cu).  Returns false (nothing launched) when the matrix's
-// static schedule does not fit the persistent kernel's residency, or the
-// device has no cooperative launch; the caller then runs the per-iteration
-// passes.  cols[j]: the basis columns of the step.
-// spin_limit: polls before a grid-barrier wait gives up (TE_ERR_DEVICE_TIMEOUT);
-// extra_arrivals > 0 makes every barrier wait for arrivals that never come
-// (the failure-path test of TE_OPT_BARRIER_EXTRA_ARRIVALS).
+// launch, for matrices of fewer than 2048 chunks (te_step.cu).  Returns false
+// (nothing launched) when the matrix's static schedule does not fit the
+// kernel's residency, or the device has no cooperative launch; the caller then
+// runs the per-iteration passes.  cols[j]: the basis columns of the step.
+// spin_limit: polls before an exchange gives up (TE_ERR_DEVICE_TIMEOUT);
+// extra_arrivals > 0 makes every exchange wait for a block that never comes
+// (the failure-path test of TE_OPT_BARRIER_EXTRA_ARRIVALS).  launch counts the
+// launches on this sync block.
+#define TE_STEP_BLOCKS 256  // 2048 chunks, 8 warps per block
+struct TeStepSync {
+  ulonglong2 alpha[TE_STEP_BLOCKS][2];  // tagged halves of the block's <u_j, w'> (re, im)
+  ulonglong2 norm[TE_STEP_BLOCKS];      // and of its ||u'_{j+1}||^2
+};
 bool te_launch_lanczos_step(const TeSell& A, bool is_real, double2* const* cols, int m, double2* w, TeDevState* ds,
-                            double* partials, cudaStream_t st, unsigned int spin_limit, unsigned int extra_arrivals);
+                            TeStepSync* sync, unsigned int launch, cudaStream_t st, unsigned int spin_limit,
+                            unsigned int extra_arrivals);
+// The same iterations with the rows in registers (te_resident.cu), for
+// matrices of at most te_resident_fits rows; fixed: the fixed-point SpMV
+// (te_launch_fix_start done, X the copies of the basis; u_1.. are then not
+// stored), else the FP64 SpMV.  launch counts the launches on this sync block.
+struct TeResidentSync {
+  unsigned long long words[2][TE_MMAX][32];  // sums, by launch parity and iteration
+  unsigned long long umax[256];              // tagged max|u_0|, one per block
+};
+bool te_resident_fits(const TeSell& A);
+bool te_launch_lanczos_resident(const TeSell& A, bool is_real, bool fixed, double norm1, double2* const* cols, int m,
+                                int4* X, TeDevState* ds, TeResidentSync* sync, unsigned int launch,
+                                cudaStream_t st, unsigned int spin_limit, unsigned int extra_arrivals);
 // Device-side stop conditions: after a batch of samples, ds->stop_flag = k + 1
 // for the first sample k of the batch at which results[obs][sample] >= threshold
 // (direction > 0) or <= threshold (direction < 0) for any condition (te_sample.cu).
@@ -427,6 +449,11 @@ void te_launch_krylov_batch(TeDevState* states, int n_instances, int mode, cudaS
 // internal: explicit sample times and stored sampled states (te_evolver.cu)
 int te_evolver_set_schedule(te_evolver ev, const double* times_host, int64_t count, double2* store_dev,
                             int64_t store_ld);
+// internal: whether the evolver may run the resident Lanczos kernel (default
+// on).  A gradient is a difference of nearly cancelling terms: at its
+// tolerance the last Krylov coefficients carry amplified rounding, so the
+// adjoint's evolutions keep the arithmetic, sum for sum, of the passes
+void te_evolver_set_resident(te_evolver ev, bool on);
 struct TeCombineArgs {
   const double2* cols[TE_MMAX];
   int m;

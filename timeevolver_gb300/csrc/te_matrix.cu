@@ -640,6 +640,12 @@ int sell_schedule(TeSell& S, const std::vector<int64_t>& off, bool real) {
                                                    TE_THREADS, 0));
   std::vector<int32_t> wc;
   te_sell_schedule(off, S.n_chunks, bps, real, S.grid, S.saturated, wc);
+  constexpr int kWarps = TE_THREADS / 32;
+  S.warp_chunks = 0;
+  S.block_slots = 0;
+  for (size_t w = 0; w + 1 < wc.size(); ++w) S.warp_chunks = std::max(S.warp_chunks, (int)(wc[w + 1] - wc[w]));
+  for (int b = 0; b < S.grid; ++b)
+    S.block_slots = std::max(S.block_slots, off[wc[(b + 1) * kWarps]] - off[wc[b * kWarps]]);
   return upload(&S.warp_chunk, wc.data(), wc.size());
 }
 
@@ -1471,6 +1477,7 @@ extern "C" int te_matrix_set_spmv_lanes(te_matrix A, int lanes) {
   }
   A->sell.lanes = lanes <= 0 ? 1 : lanes;
   A->sell.lanes_fixed = lanes > 0;
+  A->sell.lanes_pinned = lanes > 0;
   A->sell.lanes_timed = lanes == -1;
   return TE_OK;
 }

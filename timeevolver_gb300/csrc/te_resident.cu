@@ -1,0 +1,613 @@
+// te_resident.cu -- all three-term Lanczos iterations of a Krylov step in one
+// cooperative launch with the recurrence's rows in registers.
+//
+// Replaces, for matrices whose rows fit (te_resident_fits), the loop of
+// arnoldiAlgorithm (core/krylovTimeEvolver.cpp:523-571).  What bounds an
+// iteration of such a matrix is not bandwidth but the chain apply -> <u_j, w'>
+// over all rows -> update -> all rows visible -> next apply, so the kernel is
+// laid out for the length of that chain:
+//  * one block per SM; a warp owns CPW chunks of 32 rows for the whole step
+//    and keeps u_j, u_{j-1} and w' of its rows in registers.  Only the vector
+//    that other SMs gather (u_j, or its fixed-point copy X_j) goes through
+//    memory, and the matrix slots are read through L1, which holds a block's
+//    share of a small matrix from one iteration to the next;
+//  * chunk c belongs to block c mod gridDim.x: rows are sorted by length, so
+//    every block gets the same mix of lengths;
+//  * the two grid-wide sums are exact integers (as on the per-pass
+//    fixed-point path): each warp adds its lanes' values as 24-bit limbs
+//    (redux.sync), each block its warps', and one lane per limb adds the
+//    block's sum to a 64-bit word whose upper 16 bits count the blocks.  A
+//    reader knows from the word itself that its sum is complete, so the sum
+//    is its own barrier: no separate arrival counter, and no FP64 reduction
+//    tree (a warp-wide FP64 instruction costs 64 cycles here);
+//  * maxima (the fixed-point scale, and the units of the sums) travel in the
+//    same line as counts of exponents: a sum can carry them, a maximum could not;
+//  * every scalar of the recurrence is a product of ||u_j||^2 and its
+//    reciprocal: c_w = (beta_j / e)^2 = S_{j-1} ||u_j||^2, alpha_j / e =
+//    S_j <u_j, w'> with S_j = s_j^2 = 1 / ||u_j||^2, so the chain holds no
+//    square root and no division: one spare warp computes S_j, beta_j and s_j
+//    while the others gather.
+//
+// Times on GB300, per iteration: Bose-Hubbard L=10 (dim 92 378) 31 us as two
+// passes, 11.5 us here; an exchange takes 2 to 4 thousand cycles, the gathers
+// 6 700, the rows' FP64 recurrence 4 100 of an iteration's 23 000.  With the
+// rows' sums of all 152 blocks in tagged words instead (one line per 16
+// blocks) the polls themselves took the L2 slices' time: 16 us.
+#include <algorithm>
+#include <cmath>
+
+#include "te_fixed.cuh"
+#include "te_internal.cuh"
+
+namespace {
+
+constexpr int kResWarps = 19;     // worker warps per block at most
+constexpr int kResMaxCpw = 4;     // chunks per worker warp at most
+constexpr int kAlphaWords = 10;   // <u_j, w'>: re, im (4 limbs of 24 bits each), 2 words of exponent counts
+constexpr int kNormWords = 7;     // ||u_{j+1}||^2: 5 limbs, 2 words of exponent counts
+constexpr int kCountShift = 48;   // blocks counted in bits 48..63 of a word
+constexpr unsigned long long kTopBias = 1ull << 34;  // per block, keeps a signed top limb's sum positive
+
+// exponent x with |v| < 2^x (from the high word; zero and subnormals give -1022)
+__device__ __forceinline__ int exp_above(unsigned int hiword) { return (int)((hiword >> 20) & 0x7ffu) - 1022; }
+__device__ __forceinline__ int exp_above(double v) { return exp_above(te_fix_hiword(v)); }
+// 2^x, at least the smallest normal number
+__device__ __forceinline__ double pow2(int x) { return __hiloint2double((min(max(x, -1022), 1023) + 1023) << 20, 0); }
+
+struct ResShared {
+  unsigned long long part[kResWarps][8];  // per-warp limb sums
+  unsigned int pmax[kResWarps];
+  double cw, gr, gi;
+  int k1, k2, xs;    // units of the two sums, fixed-point scale of u_{j+1}
+  int ew, eu;        // exponents that the maxima of w' and u_{j+1} are counted from
+  int go, go_start;  // 1 continue, 0 leave (timeout; lucky breakdown)
+  double norm2[TE_MMAX + 1], cws[TE_MMAX + 1];  // ||u_j||^2 and (beta_j / e)^2 of the step
+};
+
+// A warp's sum of limbs (24 bits each); lane l < N keeps limb l.
+template <int N>
+__device__ __forceinline__ void warp_limbs(const int (&limb)[N], unsigned long long* out) {
+  const int lane = threadIdx.x & 31;
+  long long mine = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int s = __reduce_add_sync(0xffffffffu, limb[i]);
+    if (lane == i) mine = s;
+  }
+  if (lane < N) out[lane] = (unsigned long long)mine;
+}
+
+__device__ __forceinline__ void limbs4(unsigned long long lo, unsigned long long hi, int* l) {
+  l[0] = (int)(lo & 0xffffffull);
+  l[1] = (int)((lo >> 24) & 0xffffffull);
+  l[2] = (int)(((lo >> 48) | (hi << 16)) & 0xffffffull);
+  l[3] = (int)((long long)hi >> 8);  // signed; the caller's units keep it below 2^23
+}
+
+// Counts of exponents: a maximum below 2^e0 is counted in one of 11 bins (bin
+// b: below 2^(e0 - b), the last one open below), 6 bins of 8 bits in the
+// first word, 5 in the second, whose sixth counts non-finite values.
+__device__ __forceinline__ unsigned long long exp_count(unsigned int hiword, int e0, int word) {
+  if (hiword >= 0x7ff00000u) return word == 1 ? 1ull << 40 : 0ull;
+  const int bin = min(max(e0 - exp_above(hiword), 0), 10);
+  return bin / 6 == word ? 1ull << (8 * (bin % 6)) : 0ull;
+}
+// The exponent of the largest counted value, or INT_MAX for a non-finite one.
+__device__ __forceinline__ int exp_of_counts(unsigned long long w0, unsigned long long w1, int e0) {
+  const unsigned long long mask = (1ull << kCountShift) - 1;
+  w0 &= mask;
+  w1 &= mask;
+  if (w1 >> 40) return 0x7fffffff;
+  if (w0) return e0 - (__ffsll((long long)w0) - 1) / 8;
+  return e0 - 6 - (w1 ? (__ffsll((long long)w1) - 1) / 8 : 4);
+}
+
+// Sum over limb words (weights 2^24i, the top one biased) as a 128-bit integer.
+template <int N>
+__device__ __forceinline__ void limbs_join(const unsigned long long (&t)[N], unsigned long long bias,
+                                           unsigned long long& lo, unsigned long long& hi) {
+  const unsigned long long mask = (1ull << kCountShift) - 1;
+  lo = hi = 0;
+#pragma unroll
+  for (int i = N - 1; i >= 0; --i) {
+    // {hi, lo} = {hi, lo} << 24 + t_i
+    hi = (hi << 24) | (lo >> 40);
+    lo <<= 24;
+    const long long v = (long long)(t[i] & mask) - (i == N - 1 ? (long long)bias : 0ll);
+    const unsigned long long add = (unsigned long long)v;
+    lo += add;
+    hi += (v < 0 ? ~0ull : 0ull) + (lo < add ? 1ull : 0ull);
+  }
+}
+
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void red_add(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+}  // namespace
+
+struct TeResidentArgs {
+  int64_t n;
+  int n_chunks, n_workers, m;
+  const int64_t* chunk_off;
+  const int32_t* col;
+  const double* val;   // FP64 slots
+  const int2* hv;      // fixed point: real limbs
+  const int4* hv4;     // fixed point: complex limbs
+  const uint32_t* pk;  // fixed point: value dictionary
+  const int2* table;
+  int nvals, cbits, sh;
+  int r_exp;           // ||H|| < 2^r_exp
+  int n_exp;           // 2 n < 2^n_exp
+  int4* X;             // fixed point: copies of the basis (m x n)
+  TeResidentSync* sync;
+  int parity;          // which half of sync this launch uses
+  unsigned int epoch;  // tags of this launch's maxima
+  unsigned int spin_limit, arrivals;
+  double2* u[TE_MMAX];
+};
+
+// One lane's row of chunk slots [s, e) times the gathered vector, by format:
+// 0 fixed real limbs, 1 fixed value dictionary, 2 fixed complex limbs,
+// 3 FP64 real, 4 FP64 complex.  UNR slots in flight per lane: registers are
+// plentiful at one block per SM, and the gathers' latency is the chain.
+template <int FMT, int UNR>
+__device__ __forceinline__ double2 res_row(const TeResidentArgs& a, const int2* tab, int s, int e, const void* x,
+                                           int shift) {
+  if (FMT >= 3) {
+    const double2* xv = static_cast<const double2*>(x);
+    double re = 0.0, im = 0.0;
+#pragma unroll UNR
+    for (; s < e; s += 32) {
+      const double2 v = __ldca(xv + __ldg(a.col + s));
+      if (FMT == 3) {
+        const double h = __ldg(a.val + s);
+        re = fma(h, v.x, re);
+        im = fma(h, v.y, im);
+      } else {
+        const double2 h = __ldg(reinterpret_cast<const double2*>(a.val) + s);
+        re = fma(h.x, v.x, re);
+        re = fma(-h.y, v.y, re);
+        im = fma(h.x, v.y, im);
+        im = fma(h.y, v.x, im);
+      }
+    }
+    return make_double2(re, im);
+  }
+  const int4* xv = static_cast<const int4*>(x);
+  int64_t sr = 0, si = 0;
+  if (FMT == 1) {
+    const uint32_t cmask = (1u << a.cbits) - 1u;
+#pragma unroll UNR
+    for (; s < e; s += 32) {
+      const uint32_t wd = __ldg(a.pk + s);
+      te_fix_mac(tab[wd >> a.cbits], __ldca(xv + (wd & cmask)), sr, si);
+    }
+  } else if (FMT == 0) {
+#pragma unroll UNR
+    for (; s < e; s += 32) te_fix_mac(__ldg(a.hv + s), __ldca(xv + __ldg(a.col + s)), sr, si);
+  } else {
+#pragma unroll UNR
+    for (; s < e; s += 32) {
+      const int4 h = __ldg(a.hv4 + s);
+      const int4 v = __ldca(xv + __ldg(a.col + s));
+      sr += te_fix_prod(h.x, h.y, v.x, v.y) - te_fix_prod(h.z, h.w, v.z, v.w);
+      si += te_fix_prod(h.x, h.y, v.z, v.w) + te_fix_prod(h.z, h.w, v.x, v.y);
+    }
+  }
+  return make_double2(te_i64_to_double(sr, 62 - shift), te_i64_to_double(si, 62 - shift));
+}
+
+// The spare warp sends this block's words: its warps' limb sums (N - 2 words;
+// the signed top limbs biased) and its maximum's exponent counts.
+template <int N>
+__device__ __forceinline__ void res_send(const TeResidentArgs& a, ResShared& S, unsigned long long* words, int e0) {
+  const int lane = threadIdx.x & 31, l = lane & 15;
+  unsigned long long v = 0;
+  unsigned int mx = 0;
+  for (int w = 0; w < a.n_workers; ++w) {
+    if (l < N - 2) v += S.part[w][l];
+    mx = max(mx, S.pmax[w]);
+  }
+  if (l >= N - 2) v = exp_count(mx, e0, l - (N - 2));
+  if (l == N - 3 || (N == kAlphaWords && l == 3)) v += kTopBias;
+  v += 1ull << kCountShift;
+  if (lane < N) red_add(words + lane, v);
+}
+
+// The grid's words on lanes 0..N-1 (spare warp); false when the wait gave up.
+template <int N>
+__device__ __forceinline__ bool res_receive(const TeResidentArgs& a, const unsigned long long* words,
+                                            unsigned long long& word, TeDevState* ds) {
+  const int lane = threadIdx.x & 31;
+  word = 0;
+  unsigned int spins = 0;
+  while (true) {
+    bool ok = true;
+    if (lane < N) {
+      word = ld_relaxed(words + lane);
+      ok = (unsigned int)(word >> kCountShift) == a.arrivals;
+    }
+    if (__all_sync(0xffffffffu, ok)) return true;
+    if (++spins > a.spin_limit) {
+      if (lane == 0) atomicExch(&ds->fatal, TE_ERR_DEVICE_TIMEOUT);
+      return false;
+    }
+  }
+}
+
+// max|u_0| over the grid (FP64 rows, whose start has no encoding pass).
+__device__ __forceinline__ bool res_start_max(const TeResidentArgs& a, const ResShared& S, unsigned int tag,
+                                              unsigned int& gmax, TeDevState* ds) {
+  const int lane = threadIdx.x & 31;
+  unsigned int mx = 0;
+  for (int w = 0; w < a.n_workers; ++w) mx = max(mx, S.pmax[w]);
+  if (lane == 0) st_relaxed(a.sync->umax + blockIdx.x, ((unsigned long long)tag << 32) | mx);
+  unsigned int spins = 0;
+  while (true) {
+    bool ok = (unsigned int)gridDim.x == a.arrivals;
+    unsigned int m = 0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) {
+      const unsigned long long t = ld_relaxed(a.sync->umax + b);
+      ok = ok && (unsigned int)(t >> 32) == tag;
+      m = max(m, (unsigned int)t);
+    }
+    if (__all_sync(0xffffffffu, ok)) {
+      gmax = __reduce_max_sync(0xffffffffu, m);
+      return true;
+    }
+    if (++spins > a.spin_limit) {
+      if (lane == 0) atomicExch(&ds->fatal, TE_ERR_DEVICE_TIMEOUT);
+      return false;
+    }
+  }
+}
+
+template <int FMT, int CPW>
+__global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kernel(TeResidentArgs a, TeDevState* ds) {
+  constexpr bool FIX = FMT < 3;
+  __shared__ ResShared S;
+  extern __shared__ int2 tab[];  // FMT 1: the value table
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int G = gridDim.x;
+  const bool leader = blockIdx.x == 0;
+  TeResidentSync& sy = *a.sync;
+  if (leader)  // the other half, for the next launch (no launch in flight uses it)
+    for (int i = threadIdx.x; i < TE_MMAX * 32; i += blockDim.x) (&sy.words[a.parity ^ 1][0][0])[i] = 0ull;
+  if (ds->fatal != 0 || ds->done != 0 || ds->breakdown != 0) return;
+  if (FMT == 1)
+    for (int i = threadIdx.x; i < a.nvals; i += blockDim.x) tab[i] = a.table[i];
+  const int m = min(a.m, ds->m_cur);
+  const double e = ds->exp_factor;
+  const bool spare = warp == a.n_workers;
+  // this lane's rows: chunks blockIdx.x + (warp + i n_workers) G
+  int s0[CPW], s1[CPW];
+  int row[CPW];
+  double2 u[CPW], up[CPW], w[CPW];
+  unsigned int mx = 0;
+#pragma unroll
+  for (int i = 0; i < CPW; ++i) {
+    const int64_t c = blockIdx.x + (int64_t)(warp + i * a.n_workers) * G;
+    const bool have = !spare && c < a.n_chunks;
+    s0[i] = have ? (int)__ldg(a.chunk_off + c) + lane : 0;
+    s1[i] = have ? (int)__ldg(a.chunk_off + c + 1) : 0;
+    const int64_t r = c * 32 + lane;
+    row[i] = have && r < a.n ? (int)r : -1;
+    u[i] = row[i] >= 0 ? a.u[0][row[i]] : make_double2(0.0, 0.0);
+    up[i] = make_double2(0.0, 0.0);
+    if (!FIX) mx = max(mx, max(te_fix_hiword(u[i].x), te_fix_hiword(u[i].y)));
+  }
+  // scalars of the spare warp (the same in every block): S_j = s_j^2 and
+  // ||u_j||^2, exponents above max|u_j| and max|u_{j-1}|
+  double Sj = 1.0, norm2 = 1.0;
+  int eu = 0, eup = -4000;
+  int xs = FIX ? ds->fx_xs[0] : 0;
+  const double bd2 = (ds->tol_rate / e) * (ds->tol_rate / e);
+  int last_j = m;
+  bool broke = false;
+  if (FIX) {
+    eu = exp_above(ds->fx_umax[0]);
+    __syncthreads();  // the value table
+  } else {
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (!spare && lane == 0) S.pmax[warp] = mx;
+    __syncthreads();
+    if (spare) {
+      unsigned int um = 0;
+      const bool ok = res_start_max(a, S, a.epoch, um, ds);
+      eu = exp_above(um);
+      if (lane == 0) S.go = ok ? 1 : 0;
+    }
+    __syncthreads();
+    if (!S.go) return;
+  }
+  for (int j = 0; j < m; ++j) {
+    unsigned long long* words = sy.words[a.parity][j];
+    // apply: y = H u_j for the workers; the spare warp finishes the previous
+    // norm meanwhile
+    if (!spare) {
+      const void* x = FIX ? (const void*)(a.X + (int64_t)j * a.n) : (const void*)a.u[j];
+#pragma unroll
+      for (int i = 0; i < CPW; ++i) w[i] = res_row<FMT, CPW == 1 ? 8 : 4>(a, tab, s0[i], s1[i], x, a.sh + xs);
+    } else {
+      const double cw = j > 0 ? Sj * norm2 : 0.0;  // (beta_j / e)^2
+      const bool go = !(cw < bd2) || j == 0;       // else the lucky breakdown (:551-555)
+      const int ecw = j > 0 ? exp_above(cw) : -4000;
+      if (lane == 0) {
+        S.cw = cw;
+        S.go_start = go ? 1 : 0;
+        // units 2^-k1 of <u_j, w'>: |<u_j, w'>| <= ||u_j||^2 (||H|| + beta_j / e),
+        // beta_j / e <= ||H|| for the Hermitian H of an evolution; 12 bits to spare.
+        // ||u_0|| is only bounded through max|u_0|
+        const int ex = j == 0 ? 2 * eu + a.n_exp : exp_above(norm2);
+        S.k1 = 82 - ex - max(a.r_exp, (ecw + 2) / 2);
+        // |w'| <= ||H||_inf max|u_j| + c_w max|u_{j-1}|
+        S.ew = max(a.r_exp + eu, ecw + eup) + 1;
+        if (leader && j > 0) {
+          S.norm2[j] = norm2;
+          S.cws[j] = cw;
+        }
+      }
+      if (j > 0) Sj = 1.0 / norm2;
+    }
+    __syncthreads();
+    if (!S.go_start) {
+      last_j = j;
+      broke = true;
+      break;
+    }
+    if (!spare) {
+      const double cw = S.cw;
+      double dr = 0.0, di = 0.0;
+      mx = 0;
+#pragma unroll
+      for (int i = 0; i < CPW; ++i) {
+        if (row[i] >= 0) {
+          // w' = -i H u_j + c_w u_{j-1}; <u_j, w'> += conj(u_j) w'
+          const double2 y = w[i];
+          if (j > 0) {
+            w[i].x = fma(cw, up[i].x, y.y);
+            w[i].y = fma(cw, up[i].y, -y.x);
+          } else {
+            w[i] = make_double2(y.y, -y.x);
+          }
+          dr = fma(u[i].x, w[i].x, fma(u[i].y, w[i].y, dr));
+          di = fma(u[i].x, w[i].y, fma(-u[i].y, w[i].x, di));
+          mx = max(mx, max(te_fix_hiword(w[i].x), te_fix_hiword(w[i].y)));
+        }
+      }
+      int limb[8];
+      unsigned long long lo, hi;
+      te_fix_encode128(dr, S.k1, lo, hi);
+      limbs4(lo, hi, limb);
+      te_fix_encode128(di, S.k1, lo, hi);
+      limbs4(lo, hi, limb + 4);
+      warp_limbs<8>(limb, S.part[warp]);
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      if (lane == 0) S.pmax[warp] = mx;
+    }
+    __syncthreads();
+    if (spare) {
+      res_send<kAlphaWords>(a, S, words, S.ew);
+      unsigned long long word;
+      const bool ok = res_receive<kAlphaWords>(a, words, word, ds);
+      if (ok) {
+        // lane 0 (and every even lane) joins re, the odd lanes im
+        const int im = lane & 1;
+        unsigned long long t[4], lo, hi;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) t[i] = __shfl_sync(0xffffffffu, word, i + 4 * im);
+        const int ew = exp_of_counts(__shfl_sync(0xffffffffu, word, 8), __shfl_sync(0xffffffffu, word, 9), S.ew);
+        limbs_join<4>(t, (unsigned long long)G * kTopBias, lo, hi);
+        double g = Sj * te_i128_to_double(lo, hi, -S.k1);
+        if (ew == 0x7fffffff || eu > 1024) g = __longlong_as_double(0x7ff8000000000000ll);
+        const double go = __shfl_xor_sync(0xffffffffu, g, 1);
+        // |u_{j+1}| < B: the fixed-point scale, and the units of ||u_{j+1}||^2
+        const double B = fma(fabs(g) + fabs(go), pow2(eu), pow2(ew)) * (1.0 + 1e-12);
+        const int eb = exp_above(B);
+        xs = te_fix_scale(B);
+        if (lane == 0) {
+          S.gr = g;
+          S.gi = go;
+          S.xs = xs;
+          S.k2 = FIX ? 2 * xs - 62 : 117 - (2 * eb + a.n_exp);
+          S.eu = eb;
+          if (leader) {
+            ds->alpha[j] = make_double2(g * e, go * e);
+            if (FIX) ds->fx_xs[j + 1] = xs;
+          }
+        }
+      }
+      if (lane == 0) S.go = ok ? 1 : 0;
+    }
+    __syncthreads();
+    if (!S.go) return;
+    xs = S.xs;
+    if (!spare) {
+      // update: u_{j+1} = w' - (alpha_j / e) u_j
+      const double gr = S.gr, gi = S.gi;
+      unsigned long long lo = 0, hi = 0;
+      double nr = 0.0;
+      mx = 0;
+#pragma unroll
+      for (int i = 0; i < CPW; ++i) {
+        if (row[i] >= 0) {
+          double2 o;
+          o.x = fma(-gr, u[i].x, fma(gi, u[i].y, w[i].x));
+          o.y = fma(-gr, u[i].y, fma(-gi, u[i].x, w[i].y));
+          up[i] = u[i];
+          u[i] = o;
+          mx = max(mx, max(te_fix_hiword(o.x), te_fix_hiword(o.y)));
+          if (FIX) {
+            const int64_t er = te_fix_encode(o.x, xs), ei = te_fix_encode(o.y, xs);
+            if (j + 1 < m) {
+              const int2 p = te_fix_split(er), q = te_fix_split(ei);
+              a.X[(int64_t)(j + 1) * a.n + row[i]] = make_int4(p.x, p.y, q.x, q.y);
+            }
+            const unsigned long long sq = te_fix_sq(er) + te_fix_sq(ei);
+            lo += sq;
+            hi += lo < sq ? 1ull : 0ull;
+          } else {
+            if (j + 1 < m) a.u[j + 1][row[i]] = o;
+            nr = fma(o.x, o.x, fma(o.y, o.y, nr));
+          }
+        }
+      }
+      if (!FIX) te_fix_encode128(nr, S.k2, lo, hi);
+      int limb[kNormWords - 2];
+      limb[0] = (int)(lo & 0xffffffull);
+      limb[1] = (int)((lo >> 24) & 0xffffffull);
+      limb[2] = (int)(((lo >> 48) | (hi << 16)) & 0xffffffull);
+      limb[3] = (int)((hi >> 8) & 0xffffffull);
+      limb[4] = (int)((hi >> 32) & 0xffffffull);
+      warp_limbs<kNormWords - 2>(limb, S.part[warp]);
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      if (lane == 0) S.pmax[warp] = mx;
+    }
+    __syncthreads();
+    const bool last = j + 1 == m;
+    if (spare) {
+      fence_gpu();  // the rows this block stored, before its sums
+      res_send<kNormWords>(a, S, words + 16, S.eu);
+      unsigned long long word;
+      bool ok = true;
+      if (!last || leader) {
+        ok = res_receive<kNormWords>(a, words + 16, word, ds);
+        fence_gpu();  // the other blocks' rows, after their sums
+      }
+      if (ok && (!last || leader)) {
+        unsigned long long t[kNormWords - 2], lo, hi;
+#pragma unroll
+        for (int i = 0; i < kNormWords - 2; ++i) t[i] = __shfl_sync(0xffffffffu, word, i);
+        const int en = exp_of_counts(__shfl_sync(0xffffffffu, word, kNormWords - 2),
+                                     __shfl_sync(0xffffffffu, word, kNormWords - 1), S.eu);
+        limbs_join<kNormWords - 2>(t, (unsigned long long)G * kTopBias, lo, hi);
+        norm2 = te_u128_to_double(hi, lo, -S.k2);
+        if (en == 0x7fffffff) norm2 = __longlong_as_double(0x7ff8000000000000ll);
+        eup = eu;
+        eu = en;
+        if (last && lane == 0) {
+          S.cws[m] = Sj * norm2;
+          S.norm2[m] = norm2;
+        }
+      }
+      if (lane == 0) S.go = ok ? 1 : 0;
+    }
+    __syncthreads();
+    if (!S.go) return;
+  }
+  // the step's coefficients: beta_j = |e| sqrt((beta_j / e)^2), s_j = +-1 / ||u_j||
+  // (s_j = e s_{j-1} / beta_j); the last one is h, or the breakdown's
+  if (!leader) return;
+  for (int j = 1 + (int)threadIdx.x; j <= last_j; j += blockDim.x) {
+    const double b = fabs(e) * sqrt(S.cws[j]);
+    if (j < last_j) {
+      const double sn = 1.0 / sqrt(S.norm2[j]);
+      ds->beta[j] = b;
+      ds->s[j] = e < 0.0 && (j & 1) ? -sn : sn;
+    } else {
+      ds->h = b;
+      ds->m_eff = j;
+      if (broke || S.cws[j] < bd2) ds->breakdown = 1;
+    }
+  }
+}
+
+namespace {
+
+using ResKernel = void (*)(TeResidentArgs, TeDevState*);
+
+template <int FMT>
+ResKernel res_kernel_cpw(int cpw) {
+  switch (cpw) {
+    case 1: return lanczos_resident_kernel<FMT, 1>;
+    case 2: return lanczos_resident_kernel<FMT, 2>;
+    case 3: return lanczos_resident_kernel<FMT, 3>;
+    default: return lanczos_resident_kernel<FMT, 4>;
+  }
+}
+
+ResKernel res_kernel(int fmt, int cpw) {
+  switch (fmt) {
+    case 0: return res_kernel_cpw<0>(cpw);
+    case 1: return res_kernel_cpw<1>(cpw);
+    case 2: return res_kernel_cpw<2>(cpw);
+    case 3: return res_kernel_cpw<3>(cpw);
+    default: return res_kernel_cpw<4>(cpw);
+  }
+}
+
+}  // namespace
+
+// Rows that fit the registers of one block per SM: kResWarps warps of
+// kResMaxCpw chunks (369 664 rows on 152 SMs).
+bool te_resident_fits(const TeSell& A) {
+  if (A.n_long > 0 || A.n < 1 || A.fix_nblk > 0 || te_num_sms() > 255) return false;
+  if (A.slots >= ((int64_t)1 << 31) - 256) return false;  // 32-bit slot counters
+  return A.n_chunks <= (int64_t)te_num_sms() * kResWarps * kResMaxCpw;
+}
+
+bool te_launch_lanczos_resident(const TeSell& A, bool is_real, bool fixed, double norm1, double2* const* cols, int m,
+                                int4* X, TeDevState* ds, TeResidentSync* sync, unsigned int launch,
+                                cudaStream_t st, unsigned int spin_limit, unsigned int extra_arrivals) {
+  if (m < 1 || m > TE_MMAX || !te_resident_fits(A)) return false;
+  TeResidentArgs a{};
+  const int fmt = fixed ? (A.fix_val4 ? 2 : (A.fix_pk ? 1 : 0)) : (is_real ? 3 : 4);
+  const size_t smem = fmt == 1 ? sizeof(int2) * A.fix_nvals : 0;
+  const int G = (int)std::min<int64_t>(te_num_sms(), A.n_chunks);
+  const int per_block = (int)((A.n_chunks + G - 1) / G);
+  const int cpw = (per_block + kResWarps - 1) / kResWarps;
+  const int workers = (per_block + cpw - 1) / cpw;
+  a.n = A.n;
+  a.n_chunks = (int)A.n_chunks;
+  a.n_workers = workers;
+  a.m = m;
+  a.chunk_off = A.chunk_off;
+  a.col = A.col;
+  a.val = A.val;
+  a.hv = A.fix_val;
+  a.hv4 = A.fix_val4;
+  a.pk = A.fix_pk;
+  a.table = A.fix_table;
+  a.nvals = A.fix_nvals;
+  a.cbits = A.fix_cbits;
+  a.sh = A.fix_sh;
+  int ex = 0;
+  std::frexp(norm1 > 0.0 && norm1 < 1e300 ? norm1 : 1.0, &ex);
+  if (fixed) ex = std::max(ex, 61 - A.fix_sh);  // ||H||_inf < 2^(61 - sh)
+  a.r_exp = ex;
+  a.n_exp = 2;
+  while (((int64_t)1 << (a.n_exp - 2)) < A.n) ++a.n_exp;
+  a.X = X;
+  a.sync = sync;
+  a.parity = (int)(launch & 1u);
+  a.epoch = launch + 1u;
+  a.spin_limit = spin_limit;
+  a.arrivals = (unsigned int)G + extra_arrivals;
+  for (int j = 0; j < TE_MMAX; ++j) a.u[j] = j < m ? cols[j] : nullptr;
+  const ResKernel k = res_kernel(fmt, cpw);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(G);
+  cfg.blockDim = dim3((workers + 1) * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, k, a, ds) != cudaSuccess) {
+    cudaGetLastError();  // a refused launch is not an error of the evolution: the caller falls back
+    return false;
+  }
+  return true;
+}
