@@ -1,4 +1,4 @@
-// te_krylov.cu -- the Krylov-space part of one time step, on one thread block.
+// te_krylov.cu -- the Krylov-space part of one time step, on one cluster of blocks.
 //
 // Replaces, per Krylov step of krylovTimeEvolver::timeEvolve
 // (core/krylovTimeEvolver.cpp:261-512):
@@ -31,9 +31,28 @@
 // Quadrature.  Tanh-sinh with the level rule shared with the CPU oracle
 // (nodes t in [-3, 3], level k adds odd multiples of 2^-k, stop at the first
 // level k >= 2 with |I_k - I_{k-1}| <= 1e-3 L1_k, at most level 8); levels
-// 0..4 are evaluated together (97 abscissae).  Gauss-Legendre 15/7 for
-// fastIntegration.  The step-size search runs the reference's control flow
-// with every integral block-parallel; all threads follow the same branches.
+// 0..3 are evaluated together (49 abscissae; the integrand rises like x^(m-1)
+// and stops there).  Gauss-Legendre 15/7 for fastIntegration.
+//
+// Layout.  A step is a chain of short FP64 sequences, and a warp issues one
+// FP64 instruction per 64 cycles however many lanes it uses (one warp per
+// scheduler: 4 warps a block).  So the work is spread for latency:
+//  * a cluster of blocks runs the reference's step-size search (all blocks and
+//    threads follow the same branches): the integral asked for and the ones
+//    the search is likely to ask for next (the following substeps, the next
+//    halvings or doublings) are evaluated at the same time, one per block, and
+//    exchanged through distributed shared memory.  The search takes the
+//    results it needs from that list and starts another round when one is
+//    missing, so its decisions and values are those of the serial search;
+//  * the outputs of a step (next start vector, samples) are spread over the
+//    blocks as well;
+//  * two lanes share an abscissa's Bessel recurrence (J_k and the sums on one,
+//    the factor 2 k / z and the normalisation on the other: one FP64
+//    instruction does a step of both), three lanes a table's.
+// Measured on GB300 per Krylov step, against one block of 256 threads with the
+// integrals in sequence, results the same bit for bit: Bose-Hubbard L=6 170 ->
+// 95 us, L=8 (9 integrals a step) 294 -> 103 us, L=10 219 -> 131 us, L=12 169
+// -> 93 us.
 #include <cfloat>
 #include <cmath>
 #include <vector>
@@ -44,6 +63,19 @@
 __constant__ TeQuadTables c_quad;
 
 #define TE_KBUF 8  // outputs per coefficient group
+#define TE_KTHREADS 128  // threads per block: one warp per scheduler
+#define TE_KCLUSTER 8    // blocks of a cluster at most
+
+// One integral of the search: its interval and rule (method < 0: none), the
+// same in every block, and what the block that evaluated it found.
+struct KIntegral {
+  double a, b;
+  int method;
+};
+struct KValue {
+  double value;
+  int state;  // 4 round + 1, or + 3 when the quadrature missed its accuracy
+};
 
 struct KSmem {
   double tc[(TE_NCHEB + 1) * TE_MMAX];  // Chebyshev vectors, row n
@@ -54,9 +86,15 @@ struct KSmem {
   double d[TE_MMAX], e[TE_MMAX], dd[TE_MMAX], ee[TE_MMAX];
   double gs[TE_NCHEB + 8];              // signed, doubled last components of t_n
   double rc[TE_MMAX], rs[TE_MMAX];      // rotations of one QR sweep
-  double red[64];
+  double lev[TE_TS_KMAX + 1][2];        // level sums of the tanh-sinh rule
+  int bad[TE_TS_KMAX + 1];
   double bc[16];
   int ibc[16];
+  KIntegral spec[TE_KCLUSTER];          // the last round of integrals (this block's copy)
+  KValue found[2][TE_KCLUSTER];         // their values, by round parity, stored by the blocks that evaluated them
+  double dts[TE_SCAP + 1];              // outputs of this launch: times and slots
+  int slots[TE_SCAP + 1];
+  double trig[TE_KBUF][2];
 };
 
 static_assert(sizeof(KSmem) + 4096 <= 232448, "Krylov kernel shared memory exceeds the per-block limit");
@@ -83,6 +121,8 @@ __device__ __forceinline__ bool needs_rescale(double v) {
 struct KCtx {
   TeDevState* ds;
   KSmem* sm;
+  int rank, size;  // block of the cluster; rank 0 writes the state
+  int round;       // rounds of integrals so far
   int m;
   double h, rho, c;
   int cheb_n;     // Chebyshev vectors available up to this degree
@@ -140,85 +180,91 @@ __device__ void ensure_cheb(KCtx& C, int K) {
   __syncthreads();
 }
 
-// Integrand h |e_m^T exp(-i x T) e_1| by Chebyshev-Bessel, K iterations.
+// Integrand h |e_m^T exp(-i x T) e_1| by Chebyshev-Bessel, K iterations, on a
+// pair of lanes (all lanes of the warp call it): the even lane runs
+// J_{k-1} = f_k J_k - J_{k+1} and the sums R, I of the signed components, the
+// odd lane f_{k-1} = f_k - 2 / z and the normalisation.  The value is returned
+// to both.
 __device__ double integrand_cheb(const KCtx& C, double x, int K) {
-  const double z = x * C.rho;
+  const bool jl = (threadIdx.x & 1) == 0;
   const double* gs = C.sm->gs;
-  if (!(z > 1e-200)) return (C.m == 1) ? C.h * fabs(gs[0]) : 0.0;
+  double z = x * C.rho;
+  const bool tiny = !(z > 1e-200);
+  if (tiny) z = 1.0;
   const double inv2z = 2.0 / z;
-  double jp1 = 0.0, jk = 1e-200;
-  double R = 0.0, I = 0.0, nrm = 0.0;
-  double f = (double)K * inv2z;
+  // v: J_k / f_k; c: -J_{k+1} / -2 / z; even: R / normalisation; odd: I / unused
+  double v = jl ? 1e-200 : (double)K * inv2z;
+  double c = jl ? -0.0 : -inv2z;
+  double even = 0.0, odd = 0.0;
   for (int k = K; k >= 4; k -= 4) {
-    // k = 4q
-    R = fma(gs[k], jk, R);
-    nrm = fma(2.0, jk, nrm);
-    double jm = fma(f, jk, -jp1);
-    f -= inv2z;
-    jp1 = jk;
-    jk = jm;
-    // k - 1
-    I = fma(gs[k - 1], jk, I);
-    jm = fma(f, jk, -jp1);
-    f -= inv2z;
-    jp1 = jk;
-    jk = jm;
-    // k - 2
-    R = fma(gs[k - 2], jk, R);
-    nrm = fma(2.0, jk, nrm);
-    jm = fma(f, jk, -jp1);
-    f -= inv2z;
-    jp1 = jk;
-    jk = jm;
-    // k - 3
-    I = fma(gs[k - 3], jk, I);
-    jm = fma(f, jk, -jp1);
-    f -= inv2z;
-    jp1 = jk;
-    jk = jm;
-    if (needs_rescale(jk)) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const double o = __shfl_xor_sync(0xffffffffu, v, 1);
+      const double jk = jl ? v : o;
+      const double w = jl ? gs[k - q] : 2.0;
+      if (q & 1)
+        odd = fma(w, jk, odd);
+      else
+        even = fma(w, jk, even);
+      const double nv = fma(jl ? o : 1.0, v, c);
+      if (jl) c = -v;
+      v = nv;
+    }
+    if (needs_rescale(__shfl_sync(0xffffffffu, v, (threadIdx.x & 31) & ~1))) {
       const double sc = 0x1p-600;
-      jk *= sc;
-      jp1 *= sc;
-      R *= sc;
-      I *= sc;
-      nrm *= sc;
+      even *= sc;
+      if (jl) {
+        v *= sc;
+        c *= sc;
+        odd *= sc;
+      }
     }
   }
-  // jk = J_0 (unnormalised)
-  nrm += jk;
-  R = fma(gs[0], jk, R);
+  // v = J_0 (unnormalised) on the even lane
+  const double j0 = __shfl_sync(0xffffffffu, v, (threadIdx.x & 31) & ~1);
+  even = fma(jl ? gs[0] : 1.0, j0, even);
+  const double R = __shfl_sync(0xffffffffu, even, (threadIdx.x & 31) & ~1);
+  const double nrm = __shfl_sync(0xffffffffu, even, threadIdx.x | 1);
+  const double I = __shfl_sync(0xffffffffu, odd, (threadIdx.x & 31) & ~1);
+  if (tiny) return (C.m == 1) ? C.h * fabs(gs[0]) : 0.0;
   return C.h * hypot(R, I) / fabs(nrm);
 }
 
-// Bessel values J_0..J_K(z), normalised, into out[] (one thread).
-__device__ void bessel_table(double z, int K, double* out) {
-  if (!(z > 1e-200)) {
-    for (int k = 0; k <= K; ++k) out[k] = (k == 0) ? 1.0 : 0.0;
-    return;
-  }
+// Bessel values J_0..J_K(z) into out[], unnormalised, on a group of 4 lanes
+// (all lanes of the warp call it): lane 0 of the group runs
+// J_{k-1} = f_k J_k - J_{k+1}, lane 1 f_k, lane 2 the normalisation, whose
+// value is returned to the group.
+__device__ double bessel_table(double z, int K, double* out, bool active) {
+  const int g = threadIdx.x & 3, l0 = (threadIdx.x & 31) & ~3;
+  const bool tiny = !(z > 1e-200);
+  if (tiny) z = 1.0;
   const double inv2z = 2.0 / z;
-  double jp1 = 0.0, jk = 1e-200, nrm = 0.0;
-  double f = (double)K * inv2z;
-  out[K] = jk;
+  // v: J_k / f_k / sum; c: -J_{k+1} / -2 / z / sum
+  double v = g == 0 ? 1e-200 : (g == 1 ? (double)K * inv2z : 0.0);
+  double c = g == 0 ? -0.0 : (g == 1 ? -inv2z : 0.0);
+  const bool w = active && !tiny && g == 0;
+  if (w) out[K] = v;
   for (int k = K; k >= 1; --k) {
-    if ((k & 1) == 0) nrm = fma(2.0, jk, nrm);
-    double jm = fma(f, jk, -jp1);
-    f -= inv2z;
-    jp1 = jk;
-    jk = jm;
-    out[k - 1] = jk;
-    if (needs_rescale(jk)) {
+    const double jk = __shfl_sync(0xffffffffu, v, l0), f = __shfl_sync(0xffffffffu, v, l0 + 1);
+    if (g == 2) c = v;
+    const double x = g == 0 ? f : (g == 1 ? 1.0 : ((k & 1) == 0 ? 2.0 : 0.0));
+    const double y = g == 2 ? jk : v;
+    const double nv = fma(x, y, c);
+    if (g == 0) c = -v;
+    v = nv;
+    if (w) out[k - 1] = v;
+    if (needs_rescale(__shfl_sync(0xffffffffu, v, l0))) {
       const double sc = 0x1p-600;
-      for (int q = k - 1; q <= K; ++q) out[q] *= sc;
-      jk = out[k - 1];
-      jp1 *= sc;
-      nrm *= sc;
+      if (w)
+        for (int q = k - 1; q <= K; ++q) out[q] *= sc;
+      if (g == 0) c *= sc;
+      if (g != 1) v *= sc;
     }
   }
-  nrm += jk;
-  const double inv = 1.0 / nrm;
-  for (int k = 0; k <= K; ++k) out[k] *= inv;
+  const double j0 = __shfl_sync(0xffffffffu, v, l0), nrm = __shfl_sync(0xffffffffu, v, l0 + 2) + j0;
+  if (tiny && active && g == 0)
+    for (int k = 0; k <= K; ++k) out[k] = (k == 0) ? 1.0 : 0.0;
+  return tiny ? 1.0 : nrm;
 }
 
 // ------------------------------------------------------------ eigen path
@@ -341,84 +387,84 @@ struct IntResult {
 };
 
 // Evaluate the integrand at the abscissae of nodes [n0, n1) of the tanh-sinh
-// table on [a, b] into sm->fp / sm->fm (block-cooperative).
+// table on [a, b] into sm->fp / sm->fm (block-cooperative), two lanes each.
 __device__ void eval_ts_nodes(KCtx& C, double a, double b, int n0, int n1, bool use_eig, int K) {
   KSmem* S = C.sm;
   const double c = 0.5 * (a + b), d = 0.5 * (b - a);
   const int nev = 2 * (n1 - n0);
-  for (int e = threadIdx.x; e < nev; e += blockDim.x) {
-    const int node = n0 + (e >> 1);
+  const int w0 = (threadIdx.x & ~31) >> 1;  // first evaluation of this warp
+  for (int e0 = w0; e0 < nev; e0 += blockDim.x >> 1) {
+    const int e = e0 + ((threadIdx.x & 31) >> 1);
+    const int node = n0 + (min(e, nev - 1) >> 1);
     const bool minus = e & 1;
-    if (minus && node == 0) continue;  // t = 0 is evaluated once
     const double u = c_quad.ts_u[node];
     const double x = minus ? c - d * u : c + d * u;
     const double f = use_eig ? integrand_eig(C, x) : integrand_cheb(C, x, K);
-    if (minus)
-      S->fm[node] = f;
-    else
-      S->fp[node] = f;
+    // t = 0 is evaluated once
+    if (e < nev && (threadIdx.x & 1) == 0 && !(minus && node == 0)) (minus ? S->fm : S->fp)[node] = f;
   }
   __syncthreads();
 }
 
+// The level's weighted sums on one warp.
+__device__ void ts_level_sum(KCtx& C, int k) {
+  KSmem* S = C.sm;
+  const int* lb = c_quad.ts_level_begin;
+  double s = 0.0, sa = 0.0;
+  bool bad = false;
+  for (int node = lb[k] + (int)(threadIdx.x & 31); node < lb[k + 1]; node += 32) {
+    const double w = c_quad.ts_w[node];
+    if (node == 0) {
+      double fv = S->fp[0];
+      s = fma(w, fv, s);
+      sa = fma(w, fabs(fv), sa);
+      bad |= !isfinite(fv);
+    } else {
+      double f1 = S->fp[node], f2 = S->fm[node];
+      s = fma(w, f1 + f2, s);
+      sa = fma(w, fabs(f1) + fabs(f2), sa);
+      bad |= !isfinite(f1) || !isfinite(f2);
+    }
+  }
+  s = warp_sum_all(s);
+  sa = warp_sum_all(sa);
+  bad = __any_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 31) == 0) {
+    S->lev[k][0] = s;
+    S->lev[k][1] = sa;
+    S->bad[k] = bad ? 1 : 0;
+  }
+}
+
 // Tanh-sinh integral of the error integrand on [a, b].
-__device__ IntResult ts_integrate(KCtx& C, double a, double b) {
+__device__ IntResult ts_integrate(KCtx& C, double a, double b, int K, bool use_eig) {
   KSmem* S = C.sm;
   IntResult res = {0.0, 0.0, false};
   if (!(b > a)) return res;
-  const double zmax = fmax(fabs(a), fabs(b)) * C.rho;
-  int K = bessel_start(zmax, C.m);
-  const bool use_eig = K > TE_NCHEB;
   if (use_eig)
     ensure_eig(C);
   else
     ensure_cheb(C, K);
   const double d = 0.5 * (b - a);
   const int* lb = c_quad.ts_level_begin;
-  // levels 0..4 at once
-  eval_ts_nodes(C, a, b, 0, lb[5], use_eig, K);
+  constexpr int kFirst = 3;  // levels evaluated at once
+  eval_ts_nodes(C, a, b, 0, lb[kFirst + 1], use_eig, K);
+  const int warp = threadIdx.x >> 5;
+  if (warp <= kFirst) ts_level_sum(C, warp);
+  __syncthreads();
   double sum = 0.0, sum_abs = 0.0, prev = 0.0;
   bool nonfinite = false;
-  int evaluated = 4;
   const int kmax = C.ds->ts_kmax >= TE_TS_KMIN && C.ds->ts_kmax < TE_TS_KMAX ? C.ds->ts_kmax : TE_TS_KMAX;
   for (int k = 0; k <= kmax; ++k) {
-    if (k > evaluated) {
+    if (k > kFirst) {
       eval_ts_nodes(C, a, b, lb[k], lb[k + 1], use_eig, K);
-      evaluated = k;
+      if (warp == 0) ts_level_sum(C, k);
+      __syncthreads();
     }
-    // level sum on warp 0, broadcast through shared memory
-    if (threadIdx.x < 32) {
-      double s = 0.0, sa = 0.0;
-      bool bad = false;
-      for (int node = lb[k] + (int)threadIdx.x; node < lb[k + 1]; node += 32) {
-        const double w = c_quad.ts_w[node];
-        if (node == 0) {
-          double fv = S->fp[0];
-          s = fma(w, fv, s);
-          sa = fma(w, fabs(fv), sa);
-          bad |= !isfinite(fv);
-        } else {
-          double f1 = S->fp[node], f2 = S->fm[node];
-          s = fma(w, f1 + f2, s);
-          sa = fma(w, fabs(f1) + fabs(f2), sa);
-          bad |= !isfinite(f1) || !isfinite(f2);
-        }
-      }
-      s = warp_sum_all(s);
-      sa = warp_sum_all(sa);
-      bad = __any_sync(0xffffffffu, bad);
-      if (threadIdx.x == 0) {
-        S->bc[0] = s;
-        S->bc[1] = sa;
-        S->ibc[1] = bad ? 1 : 0;
-      }
-    }
-    __syncthreads();
-    sum += S->bc[0];
-    sum_abs += S->bc[1];
-    nonfinite |= S->ibc[1] != 0;
-    __syncthreads();
-    const double hk = ldexp(1.0, -k);
+    sum += S->lev[k][0];
+    sum_abs += S->lev[k][1];
+    nonfinite |= S->bad[k] != 0;
+    const double hk = __hiloint2double((1023 - k) << 20, 0);  // 2^-k
     const double Ik = d * hk * sum;
     const double L1 = d * hk * sum_abs;
     res.value = Ik;
@@ -429,28 +475,26 @@ __device__ IntResult ts_integrate(KCtx& C, double a, double b) {
     prev = Ik;
   }
   res.nonfinite = nonfinite;
+  __syncthreads();
   return res;
 }
 
-__device__ double gauss_integrate(KCtx& C, double a, double b, int npts) {
+__device__ double gauss_integrate(KCtx& C, double a, double b, int npts, int K, bool use_eig) {
   KSmem* S = C.sm;
   const double* xs = npts == 15 ? c_quad.g15_x : c_quad.g7_x;
   const double* ws = npts == 15 ? c_quad.g15_w : c_quad.g7_w;
   const double c = 0.5 * (a + b), d = 0.5 * (b - a);
-  const double zmax = fmax(fabs(a), fabs(b)) * C.rho;
-  int K = bessel_start(zmax, C.m);
-  const bool use_eig = K > TE_NCHEB;
   if (use_eig)
     ensure_eig(C);
   else
     ensure_cheb(C, K);
   if (threadIdx.x < 32) {
-    double s = 0.0;
-    if ((int)threadIdx.x < npts) {
-      double x = c + d * xs[threadIdx.x];
-      double f = use_eig ? integrand_eig(C, x) : integrand_cheb(C, x, K);
-      s = ws[threadIdx.x] * f;
-    }
+    const int i = threadIdx.x >> 1;  // two lanes per abscissa
+    double x = c + d * xs[min(i, npts - 1)];
+    double f = use_eig ? integrand_eig(C, x) : integrand_cheb(C, x, K);
+    // abscissa i's term on lane i
+    double t = __shfl_sync(0xffffffffu, f, (2 * threadIdx.x) & 31);
+    double s = (int)threadIdx.x < npts ? ws[threadIdx.x] * t : 0.0;
     s = warp_sum_all(s);
     if (threadIdx.x == 0) S->bc[0] = s;
   }
@@ -460,29 +504,128 @@ __device__ double gauss_integrate(KCtx& C, double a, double b, int npts) {
   return r;
 }
 
-// integrateError (core/krylovTimeEvolver.cpp:584-618); uniform across the block.
-__device__ double integrate_error(KCtx& C, double a, double b, int method, double tolRate, bool& successful) {
+// One integral of the search on this block (integrateError,
+// core/krylovTimeEvolver.cpp:584-618); only the block that runs the
+// eigen-decomposition path (rank 0) evaluates arguments beyond the series.
+// Returns whether the quadrature was accurate.
+__device__ bool eval_integral(KCtx& C, const KIntegral& q, double tolRate, double& ret) {
   TeDevState* ds = C.ds;
-  if (threadIdx.x == 0) ds->n_integrals++;
-  double ret, error = 0.0;
-  bool success = true;
-  if (method == 0) {
-    ret = gauss_integrate(C, a, b, 15);
-  } else if (method == 1) {
-    ret = gauss_integrate(C, a, b, 7);
+  const double a = q.a, b = q.b;
+  const int K = bessel_start(fmax(fabs(a), fabs(b)) * C.rho, C.m);
+  const bool use_eig = K > TE_NCHEB;
+  double error = 0.0;
+  if (q.method == 0) {
+    ret = gauss_integrate(C, a, b, 15, K, use_eig);
+  } else if (q.method == 1) {
+    ret = gauss_integrate(C, a, b, 7, K, use_eig);
   } else {
-    IntResult r = ts_integrate(C, a, b);
+    IntResult r = ts_integrate(C, a, b, K, use_eig);
     if (r.nonfinite) {
       ret = ds->tol * 10.0;  // the reference's response to a failed quadrature (:601-605)
-      error = 0.0;
     } else {
       ret = r.value;
       error = r.err;
     }
-    if (error / ret > 1e-3 && ret > 1e-3 * (b - a) * tolRate) success = false;
   }
-  successful = successful && success;
-  return ret;
+  return !(q.method == 2 && error / ret > 1e-3 && ret > 1e-3 * (b - a) * tolRate);
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned int cluster_addr(const void* p, int rank) {
+  unsigned int a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned int)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+
+// What the search may ask for next, after [0, t] (from = 0: and the doublings
+// or the halvings and substeps that follow) or substep n of t.
+struct KNext {
+  double t, t_max, s;
+  int n;        // 0: an interval [0, t]; else substep n
+  bool doubling;
+  int method_long, method_short;
+};
+
+// The value of one integral the search asks for: from the last round when it
+// is there, else a new round with it and the likely next ones, one per block.
+__device__ double integrate_error(KCtx& C, double a, double b, int method, double tolRate, bool& successful,
+                                  const KNext& nx) {
+  KSmem* S = C.sm;
+  if (threadIdx.x == 0 && C.rank == 0) C.ds->n_integrals++;
+  int hit = -1;
+  for (int i = 0; i < C.size; ++i) {
+    const KIntegral& q = S->spec[i];
+    if (q.method == method && __double_as_longlong(q.a) == __double_as_longlong(a) &&
+        __double_as_longlong(q.b) == __double_as_longlong(b) && (S->found[C.round & 1][i].state >> 2) == C.round) {
+      hit = i;
+      break;
+    }
+  }
+  if (hit < 0) {
+    ++C.round;
+    __syncthreads();
+    if ((int)threadIdx.x < C.size) {
+      const int i = threadIdx.x;
+      KIntegral q{a, b, method};
+      bool use = true;
+      if (i > 0) {
+        int n = nx.n + i;  // substeps after substep n
+        if (nx.n == 0 && nx.doubling) {
+          n = 0;
+          double t = nx.t;
+          for (int k = 0; k < i; ++k) t *= 2;
+          // the doubling loop stops at t_max: only its first clipped value counts
+          use = t < 2 * nx.t_max;
+          q.a = 0.0;
+          q.b = t > nx.t_max ? nx.t_max : t;
+        } else if (nx.n == 0) {
+          n = i - 1;
+          if (i == 1) {
+            q.a = 0.0;
+            q.b = nx.t / 2.0;
+          }
+          use = i == 1 || nx.t < nx.t_max;
+        }
+        if (n > 0) {
+          q.a = nx.t + (n - 1) * nx.s;
+          q.b = nx.t + n * nx.s;
+          q.method = nx.method_short;
+        }
+        // arguments beyond the series take the eigen-decomposition: only when asked for
+        use = use && bessel_start(fmax(fabs(q.a), fabs(q.b)) * C.rho, C.m) <= TE_NCHEB;
+      }
+      if (!use) q.method = -1;
+      S->spec[i] = q;
+    }
+    __syncthreads();
+    const KIntegral mine = S->spec[C.rank];
+    if (mine.method >= 0) {
+      double v;
+      const bool good = eval_integral(C, mine, tolRate, v);
+      if ((int)threadIdx.x < C.size) {
+        KValue* f = &S->found[C.round & 1][C.rank];
+        const int st = 4 * C.round + (good ? 1 : 3);
+        if (C.size > 1) {
+          asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cluster_addr(&f->value, threadIdx.x)), "d"(v) : "memory");
+          asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(cluster_addr(&f->state, threadIdx.x)), "r"(st)
+                       : "memory");
+        } else {
+          f->value = v;
+          f->state = st;
+        }
+      }
+    }
+    if (C.size > 1)
+      cluster_barrier();
+    else
+      __syncthreads();
+    hit = 0;
+  }
+  const KValue& f = S->found[C.round & 1][hit];
+  if ((f.state & 2) != 0) successful = false;
+  return f.value;
 }
 
 // findMaximalStepSize (core/krylovTimeEvolver.cpp:153-254).  Returns the
@@ -501,7 +644,12 @@ __device__ int find_step(KCtx& C, double tolRate, double t_stepSuggestion, doubl
     t_step = t_step_max;
     skipSubsteps = true;
   }
-  double err_step = integrate_error(C, 0.0, t_step, mlong, tolRate, ok);
+  // candidates for the other blocks: what follows an interval [0, t] or substep n
+  auto next = [&](double t, int n, bool doubling) {
+    return KNext{t, t_step_max, t / n_substeps, n, doubling, mlong, mshort};
+  };
+  double err_step =
+      integrate_error(C, 0.0, t_step, mlong, tolRate, ok, next(t_step, 0, increaseStep && !skipSubsteps));
   if (increaseStep && !skipSubsteps) {
     double err_new = err_step, t_new = t_step;
     int guard = 0;
@@ -514,13 +662,13 @@ __device__ int find_step(KCtx& C, double tolRate, double t_stepSuggestion, doubl
       }
       t_new *= 2;
       if (t_new > t_step_max) t_new = t_step_max;
-      err_new = integrate_error(C, 0.0, t_new, mlong, tolRate, ok);
+      err_new = integrate_error(C, 0.0, t_new, mlong, tolRate, ok, next(t_new, 0, true));
     }
   }
   while (err_step > tolRate * t_step) {
     nbReductions++;
     t_step = t_step / 2.0;
-    err_step = integrate_error(C, 0.0, t_step, mlong, tolRate, ok);
+    err_step = integrate_error(C, 0.0, t_step, mlong, tolRate, ok, next(t_step, 0, false));
     if (nbReductions == GO_MAX) return -1;
     skipSubsteps = false;
   }
@@ -533,7 +681,8 @@ __device__ int find_step(KCtx& C, double tolRate, double t_stepSuggestion, doubl
       n_s++;
       if (t_step + (n_s - 1) * s >= t_step_max) break;
       if (n_s > (1 << 22)) return -2;
-      deltaError = integrate_error(C, t_step + (n_s - 1) * s, t_step + n_s * s, mshort, tolRate, ok);
+      deltaError =
+          integrate_error(C, t_step + (n_s - 1) * s, t_step + n_s * s, mshort, tolRate, ok, next(t_step, n_s, false));
     }
     t_step += (n_s - 1) * s;
   }
@@ -548,9 +697,10 @@ __device__ int find_step(KCtx& C, double tolRate, double t_stepSuggestion, doubl
 
 // ------------------------------------------------------- coefficient vectors
 
-// Y[slot] = s_j i^j [exp(-i dt T) e_1]_j for the listed outputs
-// (block-cooperative; at most TE_KBUF outputs per call).
-__device__ void output_coefficients(KCtx& C, const double* dts, const int* slots, int count) {
+// Y[slot] = s_j i^j [exp(-i dt T) e_1]_j for a group of outputs (at most
+// TE_KBUF) that shares one series length; this block computes outputs first,
+// first + stride, ... of it.
+__device__ void output_coefficients(KCtx& C, const double* dts, const int* slots, int count, int first, int stride) {
   KSmem* S = C.sm;
   TeDevState* ds = C.ds;
   const int m = C.m;
@@ -558,41 +708,68 @@ __device__ void output_coefficients(KCtx& C, const double* dts, const int* slots
   for (int o = 0; o < count; ++o) zmax = fmax(zmax, fabs(dts[o]) * C.rho);
   const int K = bessel_start(zmax, m);
   const bool use_eig = K > TE_NCHEB;
+  if (use_eig) {  // one eigen-decomposition, on rank 0
+    if (C.rank != 0) return;
+    first = 0;
+    stride = 1;
+  }
+  const int own = first < count ? (count - 1 - first) / stride + 1 : 0;
+  if (own == 0) return;
   if (use_eig)
     ensure_eig(C);
   else
     ensure_cheb(C, K);
   if (!use_eig) {
-    if ((int)threadIdx.x < count) bessel_table(dts[threadIdx.x] * C.rho, K, S->J[threadIdx.x]);
+    const int warp = threadIdx.x >> 5;
+    if (warp == 0) {
+      const int i = threadIdx.x >> 2;  // 8 groups of 4 lanes
+      const double nrm = bessel_table(dts[first + min(i, own - 1) * stride] * C.rho, K, S->J[i], i < own);
+      const double inv = 1.0 / nrm;
+      if (i < own && (threadIdx.x & 3) == 0) S->bc[4 + i] = inv;
+    } else if (warp == 1 && (int)(threadIdx.x & 31) < own) {
+      const int i = threadIdx.x & 31;
+      sincos(dts[first + i * stride] * C.c, &S->trig[i][0], &S->trig[i][1]);
+    }
     __syncthreads();
     // signed coefficients a_n = eps_n sigma_n J_n (sigma: + for n%4 in {0,3}, - otherwise)
-    for (int i = threadIdx.x; i < count * (K + 1); i += blockDim.x) {
+    for (int i = threadIdx.x; i < own * (K + 1); i += blockDim.x) {
       int o = i / (K + 1), n = i % (K + 1);
       int r = n & 3;
       double sg = (r == 0 || r == 3) ? 1.0 : -1.0;
-      S->J[o][n] *= (n == 0) ? 1.0 : 2.0 * sg;
+      S->J[o][n] = (S->J[o][n] * S->bc[4 + o]) * ((n == 0) ? 1.0 : 2.0 * sg);
     }
     __syncthreads();
-  }
-  for (int i = threadIdx.x; i < count * m; i += blockDim.x) {
-    const int o = i / m, j = i % m;
-    const double dt = dts[o];
-    double re = 0.0, im = 0.0;
-    if (!use_eig) {
+    // the even terms (re) and the odd ones (im) of a component on their own
+    // lanes, then times e^{-i dt c}
+    for (int i0 = 0; i0 < 2 * own * m; i0 += blockDim.x) {
+      const int i = min(i0 + (int)threadIdx.x, 2 * own * m - 1);
+      const bool live = i0 + (int)threadIdx.x < 2 * own * m;
+      const int c = i & 1, o = (i >> 1) / m, j = (i >> 1) % m;
       const double* a = S->J[o];
-      for (int n = 0; n + 1 <= K; n += 2) {
-        re = fma(a[n], S->tc[n * TE_MMAX + j], re);
-        im = fma(a[n + 1], S->tc[(n + 1) * TE_MMAX + j], im);
+      double v = 0.0;
+      for (int n = c; n <= K; n += 2) v = fma(a[n], S->tc[n * TE_MMAX + j], v);
+      const double w = __shfl_xor_sync(0xffffffffu, v, 1);
+      const double sn = S->trig[o][0], cs = S->trig[o][1];
+      // re' = re cs + im sn, im' = im cs - re sn
+      const double x = v * cs, y = w * sn;
+      const double t = c == 0 ? x + y : x - y;
+      // times i^j, then the column scale s_j of the unnormalised basis
+      const double other = __shfl_xor_sync(0xffffffffu, t, 1);
+      const double re = c == 0 ? t : other, im = c == 0 ? other : t;
+      double yv;
+      switch (j & 3) {
+        case 0: yv = c == 0 ? re : im; break;
+        case 1: yv = c == 0 ? -im : re; break;
+        case 2: yv = c == 0 ? -re : -im; break;
+        default: yv = c == 0 ? im : -re; break;
       }
-      if ((K & 1) == 0) re = fma(a[K], S->tc[K * TE_MMAX + j], re);
-      // times e^{-i dt c}
-      double sn, cs;
-      sincos(dt * C.c, &sn, &cs);
-      double r2 = re * cs + im * sn;
-      double i2 = im * cs - re * sn;
-      re = r2;
-      im = i2;
-    } else {
+      if (live) reinterpret_cast<double*>(&ds->Y[slots[first + o * stride] * TE_MMAX + j])[c] = yv * ds->s[j];
+    }
+  } else {
+    for (int i = threadIdx.x; i < own * m; i += blockDim.x) {
+      const int o = i / m, j = i % m;
+      const double dt = dts[o];
+      double re = 0.0, im = 0.0;
       for (int k = 0; k < m; ++k) {
         double q = S->Q[k * TE_MMAX + j] * S->Q[k * TE_MMAX];
         double sn, cs;
@@ -600,76 +777,78 @@ __device__ void output_coefficients(KCtx& C, const double* dts, const int* slots
         re = fma(q, cs, re);
         im = fma(-q, sn, im);
       }
+      double yr, yi;
+      switch (j & 3) {
+        case 0: yr = re; yi = im; break;
+        case 1: yr = -im; yi = re; break;
+        case 2: yr = -re; yi = -im; break;
+        default: yr = im; yi = -re; break;
+      }
+      const double sj = ds->s[j];
+      ds->Y[slots[o] * TE_MMAX + j] = make_double2(yr * sj, yi * sj);
     }
-    // times i^j, then the column scale s_j of the unnormalised basis
-    double yr, yi;
-    switch (j & 3) {
-      case 0: yr = re; yi = im; break;
-      case 1: yr = -im; yi = re; break;
-      case 2: yr = -re; yi = -im; break;
-      default: yr = im; yi = -re; break;
-    }
-    const double sj = ds->s[j];
-    ds->Y[slots[o] * TE_MMAX + j] = make_double2(yr * sj, yi * sj);
   }
   __syncthreads();
 }
 
 // Schedule the next batch of samples of the current Krylov space (the
-// while-condition of :405) and compute their coefficients.  When the batch
-// exhausts the step, advance t_now and err (:440-441) and open the next step.
-__device__ void schedule_batch(KCtx& C) {
+// while-condition of :405) and compute their coefficients, with the step's
+// next start vector (want_w: at t_step) before them.  When the batch exhausts
+// the step, advance t_now and err (:440-441) and open the next step.
+__device__ void schedule_batch(KCtx& C, double t_step, bool want_w) {
   TeDevState* ds = C.ds;
   KSmem* S = C.sm;
-  __shared__ double dts[TE_SCAP];
-  __shared__ int cnt_s, pending_s;
-  if (threadIdx.x == 0) {
-    const double t = ds->t, ss = ds->sampling_step, t_now = ds->t_now, t_step = ds->t_step;
-    const int ns = ds->n_samples;
-    int idx = ds->index_samples;
-    double ts = ds->t_sampling;
-    int cnt = 0;
-    ds->sample_base = idx;
-    const double* times = ds->sample_times;
-    auto cond = [&](int i, double tsv) {
-      if (i >= ns) return false;
-      const double next = times ? times[i] : tsv + ss;
-      return next <= t_now + t_step || (i == ns - 1 && fabs(t_now + t_step - t) <= DBL_EPSILON);
-    };
-    while (cnt < ds->max_batch && cond(idx, ts)) {
-      ts = times ? times[idx] : ts + ss;
-      dts[cnt] = ts - t_now;
-      ++cnt;
-      ++idx;
+  // every block finds the batch's times; rank 0 alone writes the state, once
+  // all have read it
+  int idx = ds->index_samples, cnt = 0;
+  double ts = ds->t_sampling;
+  const int base = idx;
+  const double t = ds->t, ss = ds->sampling_step, t_now = ds->t_now;
+  const int ns = ds->n_samples;
+  const double* times = ds->sample_times;
+  auto cond = [&](int i, double tsv) {
+    if (i >= ns) return false;
+    const double next = times ? times[i] : tsv + ss;
+    return next <= t_now + t_step || (i == ns - 1 && fabs(t_now + t_step - t) <= DBL_EPSILON);
+  };
+  while (cnt < ds->max_batch && cond(idx, ts)) {
+    ts = times ? times[idx] : ts + ss;
+    if (threadIdx.x == 0) {
+      S->dts[1 + cnt] = ts - t_now;
+      S->slots[1 + cnt] = 1 + cnt;
     }
-    const bool pending = cond(idx, ts);
+    ++cnt;
+    ++idx;
+  }
+  const bool pending = cond(idx, ts);
+  if (threadIdx.x == 0) {
+    S->dts[0] = t_step;
+    S->slots[0] = 0;
+  }
+  __syncthreads();
+  if (C.size > 1) cluster_barrier();
+  if (C.rank == 0 && threadIdx.x == 0) {
+    ds->sample_base = base;
     ds->t_sampling = ts;
     ds->index_samples = idx;
     ds->samples_in_batch = cnt;
     ds->samples_pending = pending ? 1 : 0;
-    cnt_s = cnt;
-    pending_s = pending ? 1 : 0;
-  }
-  __syncthreads();
-  const int cnt = cnt_s;
-  for (int o0 = 0; o0 < cnt; o0 += TE_KBUF) {
-    int slots[TE_KBUF];
-    const int k = min(TE_KBUF, cnt - o0);
-    for (int o = 0; o < k; ++o) slots[o] = 1 + o0 + o;
-    output_coefficients(C, dts + o0, slots, k);
-  }
-  if (threadIdx.x == 0 && !pending_s) {
-    ds->t_now += ds->t_step;
-    ds->err += ds->err_step;
-    if (ds->index_samples < ds->n_samples) {
-      ds->n_steps++;
-      ds->breakdown = 0;
-    } else {
-      ds->done = 1;
+    if (!pending) {
+      ds->t_now += ds->t_step;
+      ds->err += ds->err_step;
+      if (idx < ns) {
+        ds->n_steps++;
+        ds->breakdown = 0;
+      } else {
+        ds->done = 1;
+      }
     }
   }
-  (void)S;
-  __syncthreads();
+  // the outputs over the blocks: the start vector on the last one, samples
+  // round the others
+  if (want_w) output_coefficients(C, S->dts, S->slots, 1, C.rank == C.size - 1 ? 0 : 1, 1);
+  for (int o0 = 0; o0 < cnt; o0 += TE_KBUF)
+    output_coefficients(C, S->dts + 1 + o0, S->slots + 1 + o0, min(TE_KBUF, cnt - o0), C.rank, C.size);
 }
 
 // Load T from the Lanczos coefficients and set up the Chebyshev data.
@@ -681,8 +860,10 @@ __device__ void setup_krylov_matrix(KCtx& C) {
     int j = threadIdx.x;
     S->d[j] = j < m ? -ds->alpha[j].y : 0.0;
     S->e[j] = j + 1 < m ? ds->beta[j + 1] : 0.0;
-    ds->d[j] = S->d[j];
-    ds->e[j] = S->e[j];
+    if (C.rank == 0) {
+      ds->d[j] = S->d[j];
+      ds->e[j] = S->e[j];
+    }
   }
   __syncthreads();
   // Gershgorin interval on warp 0
@@ -718,10 +899,11 @@ __device__ void setup_krylov_matrix(KCtx& C) {
 }
 
 // Persist Chebyshev / eigen data for the later batch launches.
-__device__ void save_krylov_data(KCtx& C) {
+__device__ void save_krylov_data(KCtx& C, bool pending) {
   TeDevState* ds = C.ds;
   KSmem* S = C.sm;
-  for (int i = threadIdx.x; i < (C.cheb_n + 1) * TE_MMAX; i += blockDim.x) ds->cheb_t[i] = S->tc[i];
+  if (pending)  // only a further batch of samples reads them
+    for (int i = threadIdx.x; i < (C.cheb_n + 1) * TE_MMAX; i += blockDim.x) ds->cheb_t[i] = S->tc[i];
   if (C.eig_ok) {
     for (int i = threadIdx.x; i < TE_MMAX * TE_MMAX; i += blockDim.x) ds->eig_Q[i] = S->Q[i];
     if (threadIdx.x < TE_MMAX) ds->eig_lam[threadIdx.x] = S->lam[threadIdx.x];
@@ -765,14 +947,16 @@ __device__ void load_krylov_data(KCtx& C) {
   __syncthreads();
 }
 
-// One Krylov-space step of one evolution (block-cooperative).
+// One Krylov-space step of one evolution, by the blocks of a cluster (rank,
+// size; size 1: one block of any size).
 // mode 0: full step (matrix setup, step search, w, first sample batch);
 // mode 1: next sample batch of the same Krylov space.
-__device__ void krylov_step_body(TeDevState* ds, int mode, KSmem* S) {
+__device__ void krylov_step_body(TeDevState* ds, int mode, KSmem* S, int rank, int size) {
   if (ds->fatal != 0) return;
   if ((mode == 0 && ds->done != 0) || (mode == 1 && ds->samples_pending == 0)) {
     // nothing to do for this evolution: make the combine/observable passes skip it
-    if (threadIdx.x == 0) {
+    if (size > 1) cluster_barrier();  // all blocks have read the state
+    if (threadIdx.x == 0 && rank == 0) {
       ds->samples_in_batch = 0;
       ds->want_w = 0;
     }
@@ -781,23 +965,45 @@ __device__ void krylov_step_body(TeDevState* ds, int mode, KSmem* S) {
   KCtx C;
   C.ds = ds;
   C.sm = S;
+  C.rank = rank;
+  C.size = size;
+  C.round = 0;
+  if ((int)threadIdx.x < TE_KCLUSTER) {
+    S->spec[threadIdx.x].method = -1;
+    S->found[0][threadIdx.x].state = S->found[1][threadIdx.x].state = 0;
+  }
+  // every block runs, and has read the state, before any stores into the
+  // others' shared memory or writes the state
+  if (size > 1)
+    cluster_barrier();
+  else
+    __syncthreads();
   C.m = ds->m_eff;
   C.h = ds->h;
   C.fatal = 0;
+  const bool writer = rank == 0 && threadIdx.x == 0;
   if (mode == 1) {
     load_krylov_data(C);
-    if (threadIdx.x == 0) ds->want_w = 0;
-    schedule_batch(C);
-    save_krylov_data(C);
+    schedule_batch(C, ds->t_step, false);
+    if (rank == 0) {
+      if (threadIdx.x == 0) ds->want_w = 0;
+      __syncthreads();
+      save_krylov_data(C, ds->samples_pending != 0);
+    }
+    if (size > 1) cluster_barrier();
     return;
   }
-  if (threadIdx.x == 0) ds->n_integrals = 0;
-  setup_krylov_matrix(C);
   const bool hbd = ds->breakdown != 0;
+  double t_step = 0.0;
+  int code = 0;
+  if (writer) ds->n_integrals = 0;
+  setup_krylov_matrix(C);
   if (hbd) {
     // lucky breakdown (:342-363): the remaining time in one step, m reduced for good
-    if (threadIdx.x == 0) {
-      ds->t_step = ds->t - ds->t_now;
+    t_step = ds->t - ds->t_now;
+    if (size > 1) cluster_barrier();
+    if (writer) {
+      ds->t_step = t_step;
       ds->err_step = 0.0;
       ds->m_cur = C.m;
       ds->status = TE_STATUS_LUCKY_BREAKDOWN;
@@ -806,26 +1012,23 @@ __device__ void krylov_step_body(TeDevState* ds, int mode, KSmem* S) {
     }
   } else {
     const double s0 = 0.97 * ds->t_step;
-    double t_step = 0.0, err_step = 0.0;
-    int code = find_step(C, ds->tol_rate, s0, ds->t - ds->t_now, 50, ds->num_err_est, ds->t_now == 0.0, &t_step,
-                         &err_step);
+    double err_step = 0.0;
+    code = find_step(C, ds->tol_rate, s0, ds->t - ds->t_now, 50, ds->num_err_est, ds->t_now == 0.0, &t_step,
+                     &err_step);
+    if (size > 1) cluster_barrier();
     if (code < 0) {
-      if (threadIdx.x == 0) ds->fatal = code == -1 ? TE_ERR_NO_STEP : TE_ERR_UNSUPPORTED;
+      if (writer) ds->fatal = code == -1 ? TE_ERR_NO_STEP : TE_ERR_UNSUPPORTED;
       return;
     }
-    if (threadIdx.x == 0) {
+    if (writer) {
       ds->t_step = t_step;
       ds->err_step = err_step;
       ds->err_code_find = code;
       ds->want_w = 1;
       ds->new_start = 1;
     }
-    __syncthreads();
-    double dts[1] = {t_step};
-    int slots[1] = {0};
-    output_coefficients(C, dts, slots, 1);
   }
-  if (threadIdx.x == 0) {
+  if (writer) {
     switch (ds->err_code_find) {  // :386-399 (a breakdown step re-counts the previous code)
       case 1: ds->nb_err_roundoff++; break;
       case 20: ds->nb_err_int++; break;
@@ -837,23 +1040,26 @@ __device__ void krylov_step_body(TeDevState* ds, int mode, KSmem* S) {
     }
   }
   __syncthreads();
-  if (ds->fatal != 0) return;
-  schedule_batch(C);
-  save_krylov_data(C);
+  schedule_batch(C, t_step, !hbd);
+  if (rank == 0) {
+    __syncthreads();
+    save_krylov_data(C, ds->samples_pending != 0);
+  }
+  if (size > 1) cluster_barrier();  // no block leaves while others may store into its shared memory
 }
 
 // One block (one per SM at most: the shared memory of KSmem), so the whole
 // register file is available; at the default budget of 64 registers the
 // kernel spilled 260 bytes.
-__global__ void __launch_bounds__(TE_THREADS, 1) krylov_kernel(TeDevState* ds, int mode) {
+__global__ void __launch_bounds__(TE_KTHREADS, 1) krylov_kernel(TeDevState* ds, int mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  krylov_step_body(ds, mode, reinterpret_cast<KSmem*>(smem_raw));
+  krylov_step_body(ds, mode, reinterpret_cast<KSmem*>(smem_raw), blockIdx.x, gridDim.x);
 }
 
-// Batched evolutions: block b runs the step of instance b.
-__global__ void __launch_bounds__(TE_THREADS, 1) krylov_batch_kernel(TeDevState* states, int mode) {
+// Batched evolutions: cluster b (of `size` blocks) runs the step of instance b.
+__global__ void __launch_bounds__(TE_KTHREADS, 1) krylov_batch_kernel(TeDevState* states, int mode, int size) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  krylov_step_body(states + blockIdx.x, mode, reinterpret_cast<KSmem*>(smem_raw));
+  krylov_step_body(states + blockIdx.x / size, mode, reinterpret_cast<KSmem*>(smem_raw), blockIdx.x % size, size);
 }
 
 // ---------------------------------------------------------------------------
@@ -923,7 +1129,7 @@ __global__ void __launch_bounds__(TE_BATCH_PTHREADS, 1) batch_persistent_kernel(
     }
     int pending, all_done, fatal;
     for (int mode = 0;; mode = 1) {
-      for (int i = blockIdx.x; i < n_inst; i += G) krylov_step_body(a.states + i, mode, S);
+      for (int i = blockIdx.x; i < n_inst; i += G) krylov_step_body(a.states + i, mode, S, 0, 1);
       if (!bar()) return;
       batch_combine_body<true>(a.g, a.V, a.spare, a.sampled, a.states, 0, pw, PW);
       if (!bar()) return;
@@ -944,6 +1150,7 @@ __global__ void __launch_bounds__(TE_BATCH_PTHREADS, 1) batch_persistent_kernel(
 // ---------------------------------------------------------------- host side
 
 static bool g_tables_uploaded = false;
+static int g_cluster = 1;  // blocks per cluster of the Krylov kernels (te_upload_quad_tables)
 
 int te_upload_quad_tables() {
   if (g_tables_uploaded) return TE_OK;
@@ -1007,20 +1214,57 @@ int te_upload_quad_tables() {
   TE_CUDA(cudaMemcpyToSymbol(c_quad, &T, sizeof(T)));
   TE_CUDA(cudaFuncSetAttribute(krylov_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KSmem)));
   TE_CUDA(cudaFuncSetAttribute(krylov_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KSmem)));
+  // the largest cluster whose blocks (one per SM: their shared memory) can run together
+  for (int size = TE_KCLUSTER; size > 1; size /= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(TE_KTHREADS);
+    cfg.dynamicSmemBytes = sizeof(KSmem);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, krylov_kernel, &cfg) != cudaSuccess) cudaGetLastError();
+    if (clusters >= 1) {
+      g_cluster = size;
+      break;
+    }
+  }
   g_tables_uploaded = true;
   return TE_OK;
 }
 
-void te_launch_krylov_step(TeDevState* ds, cudaStream_t st) {
-  krylov_kernel<<<1, TE_THREADS, sizeof(KSmem), st>>>(ds, 0);
+template <typename... KArgs, typename... Args>
+static void launch_clusters(void (*kernel)(KArgs...), int clusters, int size, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(clusters * size);
+  cfg.blockDim = dim3(TE_KTHREADS);
+  cfg.dynamicSmemBytes = sizeof(KSmem);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+
+void te_launch_krylov_step(TeDevState* ds, cudaStream_t st) { launch_clusters(krylov_kernel, 1, g_cluster, st, ds, 0); }
 
 void te_launch_schedule_samples(TeDevState* ds, cudaStream_t st) {
-  krylov_kernel<<<1, TE_THREADS, sizeof(KSmem), st>>>(ds, 1);
+  launch_clusters(krylov_kernel, 1, g_cluster, st, ds, 1);
 }
 
+// Blocks per instance: as many as leave all clusters resident at once (a
+// block takes a whole SM's shared memory); finished instances leave at once.
 void te_launch_krylov_batch(TeDevState* states, int n_instances, int mode, cudaStream_t st) {
-  krylov_batch_kernel<<<n_instances, TE_THREADS, sizeof(KSmem), st>>>(states, mode);
+  int size = g_cluster;
+  while (size > 1 && n_instances * size > te_num_sms()) size /= 2;
+  launch_clusters(krylov_batch_kernel, n_instances, size, st, states, mode, size);
 }
 
 int te_batch_persistent_grid(bool is_real) {
