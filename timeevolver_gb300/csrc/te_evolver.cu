@@ -6,8 +6,8 @@
 // and status counters live in TeDevState); the host only enqueues one Krylov
 // step at a time (2m Lanczos passes, one Krylov-space kernel, one combine
 // pass, one observable pass), reads back a few scalars and decides whether a
-// further sample batch or step is needed.  Observables that cannot be fused
-// (non-diagonal sparse matrices, host callbacks) are evaluated per sample.
+// further sample batch or step is needed.  Observables are evaluated for a
+// whole batch of samples per launch; host callbacks see one sample at a time.
 #include <cfloat>
 #include <cstddef>
 #include <cmath>
@@ -147,9 +147,9 @@ int read_summary(te_evolver ev) {
   return TE_OK;
 }
 
-// Observables of the current batch: fused reductions on the device, then the
-// per-sample general / callback observables.  *stop_at receives the batch
-// index of a stop request (or -1).
+// Observables of the current batch: fused reductions, then the general, dense
+// and callback observables.  *stop_at receives the batch index of a stop
+// request (or -1).
 int process_batch(te_evolver ev, int* stop_at, bool synced) {
   *stop_at = -1;
   // fused passes (up to TE_FUSED_DIAG diagonal + TE_FUSED_VEC vector observables per pass)
@@ -183,46 +183,40 @@ int process_batch(te_evolver ev, int* stop_at, bool synced) {
     }
     ++ev->launches;
   }
-  bool need_host = false;
-  for (auto& o : ev->obs) need_host |= (o.kind == 2 || o.kind == 3 || o.kind == 4);
-  if (!need_host) {
-    if (ev->stops.count) {
-      te_launch_stop_check(ev->stops, ev->results, (int)ev->n_samples, ev->ds, ev->st);
+  // the others in the order they were added; callbacks see one sample per
+  // batch (run), on the host
+  bool callbacks = false;
+  for (auto& o : ev->obs) callbacks |= o.kind == 3;
+  if (callbacks) {
+    if (!synced) {
+      int rc = read_summary(ev);
+      if (rc != TE_OK) return rc;
+    }
+    if (ev->sum->samples_in_batch > 0) {
+      te_launch_permute(ev->n, ev->H->sell.iperm, ev->batch, ev->orig_tmp, ev->st);
       ++ev->launches;
     }
-    return TE_OK;
   }
-  if (!synced) {
-    int rc = read_summary(ev);
-    if (rc != TE_OK) return rc;
-  }
-  const int S = ev->sum->samples_in_batch;
-  for (int s = 0; s < S; ++s) {
-    te_launch_permute(ev->n, ev->H->sell.iperm, ev->batch + (int64_t)s * ev->n, ev->orig_tmp, ev->st);
-    ++ev->launches;
-    for (size_t i = 0; i < ev->obs.size(); ++i) {
-      HostObs& o = ev->obs[i];
-      if (o.kind == 2) {
-        te_launch_general_obs(*o.O, ev->orig_tmp, ev->ds, s, ev->partials, ev->results + i * ev->n_samples, ev->st);
-        ++ev->launches;
-      } else if (o.kind == 4) {
-        te_launch_dense_obs(ev->n, o.dense, ev->orig_tmp, ev->ds, s, ev->partials, ev->results + i * ev->n_samples,
-                            ev->st);
-        ++ev->launches;
-      } else if (o.kind == 3) {
-        TE_CUDA(cudaMemcpyAsync(ev->host_state, ev->orig_tmp, sizeof(double2) * ev->n, cudaMemcpyDeviceToHost,
-                                ev->st));
-        TE_CUDA(cudaStreamSynchronize(ev->st));
-        double value = 0.0;
-        int stop = o.fn(o.user, reinterpret_cast<const double*>(ev->host_state), ev->n, &value);
-        if (stop) {
-          *stop_at = s;
-          return TE_OK;
-        }
-        TE_CUDA(cudaMemcpyAsync(ev->results + i * ev->n_samples + ev->sum->sample_base + s, &value, sizeof(double),
-                                cudaMemcpyHostToDevice, ev->st));
-        TE_CUDA(cudaStreamSynchronize(ev->st));
+  for (size_t i = 0; i < ev->obs.size(); ++i) {
+    HostObs& o = ev->obs[i];
+    double* row = ev->results + i * ev->n_samples;
+    if (o.kind == 2) {
+      te_launch_general_obs(*o.O, ev->H->sell.iperm, ev->batch, ev->ds, ev->partials, row, ev->st);
+      ++ev->launches;
+    } else if (o.kind == 4) {
+      te_launch_dense_obs(ev->n, o.dense, ev->H->sell.iperm, ev->batch, ev->ds, ev->partials, row, ev->st);
+      ++ev->launches;
+    } else if (o.kind == 3 && ev->sum->samples_in_batch > 0) {
+      TE_CUDA(cudaMemcpyAsync(ev->host_state, ev->orig_tmp, sizeof(double2) * ev->n, cudaMemcpyDeviceToHost, ev->st));
+      TE_CUDA(cudaStreamSynchronize(ev->st));
+      double value = 0.0;
+      int stop = o.fn(o.user, reinterpret_cast<const double*>(ev->host_state), ev->n, &value);
+      if (stop) {
+        *stop_at = 0;
+        return TE_OK;
       }
+      TE_CUDA(cudaMemcpyAsync(row + ev->sum->sample_base, &value, sizeof(double), cudaMemcpyHostToDevice, ev->st));
+      TE_CUDA(cudaStreamSynchronize(ev->st));
     }
   }
   if (ev->stops.count) {
@@ -277,9 +271,11 @@ int run(te_evolver ev, te_result* out) {
   cudaStream_t st = ev->st;
   ev->launches = 0;
   ev->trace.clear();
-  bool need_host = false;
-  for (auto& o : ev->obs) need_host |= (o.kind == 2 || o.kind == 3 || o.kind == 4);
-  ev->max_batch = need_host ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(TE_SCAP, ((int64_t)256 << 20) / (16 * n)));
+  // host callbacks see one sample at a time, and so does a stop condition
+  // beside observables that are not fused
+  bool single = false;
+  for (auto& o : ev->obs) single |= o.kind == 3 || (ev->stops.count > 0 && (o.kind == 2 || o.kind == 4));
+  ev->max_batch = single ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(TE_SCAP, ((int64_t)256 << 20) / (16 * n)));
   if (ev->max_batch > ev->batch_cap) {  // kept across runs while large enough
     te_free(ev->batch);
     ev->batch = nullptr;

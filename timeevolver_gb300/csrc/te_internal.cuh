@@ -25,7 +25,7 @@
 #define TE_TS_KMAX 8          // tanh-sinh refinement levels 0..8
 #define TE_TS_KMIN 2
 #define TE_TS_NODES 769       // nodes with t >= 0 over levels 0..8
-#define TE_FUSED_DIAG 4       // diagonal observables per fused reduction pass
+#define TE_FUSED_DIAG 8       // diagonal observables per fused reduction pass
 #define TE_FUSED_VEC 2        // vector observables per fused reduction pass
 #define TE_FUSED_VALS (TE_FUSED_DIAG + 2 * TE_FUSED_VEC)
 
@@ -424,8 +424,9 @@ struct TeStopConds {
 };
 void te_launch_stop_check(const TeStopConds& c, const double* results, int n_samples_total, TeDevState* ds,
                           cudaStream_t st);
-// Re <psi|O|psi> of a dense column-major O on the original ordering (te_sample.cu).
-void te_launch_dense_obs(int64_t n, const double2* O, const double2* psi_orig, TeDevState* ds, int sample_in_batch,
+// Re <psi|O|psi> of a dense column-major O (original ordering) for the batch's
+// samples psi (the evolver's row order, iperm: original -> evolver) (te_sample.cu).
+void te_launch_dense_obs(int64_t n, const double2* O, const int32_t* iperm, const double2* psi, TeDevState* ds,
                          double* partials, double* results_row, cudaStream_t st);
 // Choose the lanes per row of a square matrix's SpMV passes (te_lanczos.cu).
 int te_tune_sell_lanes(te_matrix_s* A);
@@ -474,6 +475,6 @@ struct TeFusedObs {
 };
 void te_launch_fused_obs(int64_t n, const double2* psi, const TeFusedObs& f, TeDevState* ds, double* partials,
                          double* results, int n_samples_total, cudaStream_t st);
-void te_launch_general_obs(const te_matrix_s& O, const double2* psi_orig, TeDevState* ds, int sample_in_batch,
+void te_launch_general_obs(const te_matrix_s& O, const int32_t* iperm, const double2* psi, TeDevState* ds,
                            double* partials, double* results_row, cudaStream_t st);
 void te_launch_norm2(int64_t n, const double2* x, double* partials, TeDevState* ds, cudaStream_t st);
