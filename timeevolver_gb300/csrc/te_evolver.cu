@@ -389,6 +389,8 @@ int run(te_evolver ev, te_result* out) {
     TE_CUDA(te_malloc(&ev->res_sync, sizeof(TeResidentSync)));
     TE_CUDA(cudaMemsetAsync(ev->res_sync, 0, sizeof(TeResidentSync), st));
   }
+  unsigned long long* gs_acc = reinterpret_cast<unsigned long long*>(ev->partials + kPartials);
+  if (ev->p.reorth) TE_CUDA(cudaMemsetAsync(gs_acc, 0, sizeof(unsigned long long) * TE_GS_ACC, st));
   while (!S->done) {
     if (S->fatal) break;
     if (++guard > ((int64_t)1 << 40)) break;
@@ -398,6 +400,10 @@ int run(te_evolver ev, te_result* out) {
     const bool cgs2 = ev->p.reorth != 0;
     const bool fold = !cgs2 && ev->p.exp_factor != 0.0;
     bool fused = false;
+    if (cgs2) {
+      te_launch_norm2(n, ev->cols[0], ev->partials, ev->ds, st);
+      ++ev->launches;
+    }
     const bool fix_step = fix && fold;
     if (fix_step) {
       ProfScope ps(ev, 3);
@@ -443,10 +449,12 @@ int run(te_evolver ev, te_result* out) {
         TeBasisPtrs V{};
         for (int i = 0; i <= j; ++i) V.u[i] = ev->cols[i];
         ProfScope ps(ev, 1);
-        te_launch_gs_project(n, V, j + 1, ev->w, ev->ds, ev->partials, st);
-        te_launch_gs_update_project(n, V, j + 1, ev->w, ev->ds, ev->partials, st);
-        te_launch_gs_update_norm(n, V, j + 1, ev->w, j + 1 < m ? ev->cols[j + 1] : nullptr, ev->ds, ev->partials, j,
-                                 st);
+        double2* next = j + 1 < m ? ev->cols[j + 1] : nullptr;
+        if (!te_launch_gs_small(n, V, j + 1, ev->w, next, ev->ds, ev->partials, gs_acc, ev->H->norm1, j, st)) {
+          te_launch_gs_project(n, V, j + 1, ev->w, ev->ds, ev->partials, st);
+          te_launch_gs_update_project(n, V, j + 1, ev->w, ev->ds, ev->partials, st);
+          te_launch_gs_update_norm(n, V, j + 1, ev->w, next, ev->ds, ev->partials, j, st);
+        }
         ev->launches += 4;
       }
     }
@@ -634,7 +642,7 @@ extern "C" int te_evolver_create(te_matrix H, const double* v_host, const te_par
   ev->spare = ev->slab + (int64_t)m * n;
   ev->w = ev->slab + (int64_t)(m + 1) * n;
   ev->sampled = ev->slab + (int64_t)(m + 2) * n;
-  if ((rc = te_cuda_check(te_malloc(&ev->partials, sizeof(double) * kPartials), "partials")) != TE_OK)
+  if ((rc = te_cuda_check(te_malloc(&ev->partials, sizeof(double) * (kPartials + TE_GS_ACC)), "partials")) != TE_OK)
     return fail(rc);
   if ((rc = te_cuda_check(te_malloc(&ev->orig_tmp, sizeof(double2) * n), "tmp")) != TE_OK) return fail(rc);
   // v (original order) -> permuted start vector

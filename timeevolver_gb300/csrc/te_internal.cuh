@@ -441,6 +441,13 @@ void te_launch_gs_update_project(int64_t n, const TeBasisPtrs& V, int nvec, doub
                                  double* partials, cudaStream_t st);
 void te_launch_gs_update_norm(int64_t n, const TeBasisPtrs& V, int nvec, const double2* w, double2* u_next,
                               TeDevState* ds, double* partials, int j, cudaStream_t st);
+// All three passes of iteration j for dimensions below TE_GS_ROWS rows per SM
+// (false: not launched); acc: TE_GS_ACC words, zero before an evolution's
+// first iteration; ds->norm2_final holds ||u_0||^2 of the step
+// (te_launch_norm2).
+#define TE_GS_ACC (8 * TE_MMAX + 1)
+bool te_launch_gs_small(int64_t n, const TeBasisPtrs& V, int nvec, double2* w, double2* u_next, TeDevState* ds,
+                        double* partials, unsigned long long* acc, double norm1, int j, cudaStream_t st);
 // te_krylov.cu
 int te_upload_quad_tables();
 void te_launch_krylov_step(TeDevState* ds, cudaStream_t st);
