@@ -46,13 +46,15 @@
 //    missing, so its decisions and values are those of the serial search;
 //  * the outputs of a step (next start vector, samples) are spread over the
 //    blocks as well;
-//  * two lanes share an abscissa's Bessel recurrence (J_k and the sums on one,
-//    the factor 2 k / z and the normalisation on the other: one FP64
-//    instruction does a step of both), three lanes a table's.
+//  * two warps share the Bessel recurrence of 32 abscissae, one running J_k and
+//    its factor, the other the sums, 16 steps behind through shared memory.
+//    (Two lanes sharing it, one FP64 instruction for both, is slower: a value
+//    that leaves the FP64 pipe for a shuffle or a select takes ~150 cycles,
+//    one that stays in it 65.)
 // Measured on GB300 per Krylov step, against one block of 256 threads with the
 // integrals in sequence, results the same bit for bit: Bose-Hubbard L=6 170 ->
-// 95 us, L=8 (9 integrals a step) 294 -> 103 us, L=10 219 -> 131 us, L=12 169
-// -> 93 us.
+// 69 us, L=8 (9 integrals a step) 294 -> 88 us, L=10 219 -> 108 us, L=12 169
+// -> 83 us.
 #include <cfloat>
 #include <cmath>
 #include <vector>
@@ -61,6 +63,11 @@
 #include "te_internal.cuh"
 
 __constant__ TeQuadTables c_quad;
+// The abscissae and weights again in global memory: lanes read different nodes
+// at once, which constant memory serves one by one.
+__device__ TeQuadTables g_quad;
+constexpr int kTsFirst = 3;        // tanh-sinh levels evaluated at once
+constexpr int kTsFirstNodes = 25;  // their nodes
 
 #define TE_KBUF 8  // outputs per coefficient group
 #define TE_KTHREADS 128  // threads per block: one warp per scheduler
@@ -71,6 +78,7 @@ __constant__ TeQuadTables c_quad;
 struct KIntegral {
   double a, b;
   int method;
+  int K;  // series length at the interval's end
 };
 struct KValue {
   double value;
@@ -81,10 +89,18 @@ struct KSmem {
   double tc[(TE_NCHEB + 1) * TE_MMAX];  // Chebyshev vectors, row n
   double fp[TE_TS_NODES], fm[TE_TS_NODES];
   double Q[TE_MMAX * TE_MMAX];          // eigenvectors (col-major), fallback path
-  double J[TE_KBUF][TE_NCHEB + 8];      // Bessel values per output
+  union {
+    double J[TE_SCAP + 1][TE_NCHEB + 8];  // Bessel values per output
+    struct {  // integrals: J_k between the two warps of an argument set (2 blocks of 16 steps, J_0)
+      double ring[2][2][17][32];
+      int rescaled[2][2][4][32];  // after every fourth step of a block
+    };
+  };
   double lam[TE_MMAX];
   double d[TE_MMAX], e[TE_MMAX], dd[TE_MMAX], ee[TE_MMAX];
   double gs[TE_NCHEB + 8];              // signed, doubled last components of t_n
+  double s[TE_MMAX];                    // column scales
+  double tsu[kTsFirstNodes], tsw[kTsFirstNodes];  // tanh-sinh nodes and weights of the first levels
   double rc[TE_MMAX], rs[TE_MMAX];      // rotations of one QR sweep
   double lev[TE_TS_KMAX + 1][2];        // level sums of the tanh-sinh rule
   int bad[TE_TS_KMAX + 1];
@@ -92,9 +108,10 @@ struct KSmem {
   int ibc[16];
   KIntegral spec[TE_KCLUSTER];          // the last round of integrals (this block's copy)
   KValue found[2][TE_KCLUSTER];         // their values, by round parity, stored by the blocks that evaluated them
-  double dts[TE_SCAP + 1];              // outputs of this launch: times and slots
-  int slots[TE_SCAP + 1];
-  double trig[TE_KBUF][2];
+  double dts[TE_SCAP + 1];              // times of this launch's outputs
+  double trig[TE_SCAP + 1][2];
+  double inv[TE_SCAP + 1];              // 1 / normalisation of the tables
+  int outK[3];                          // series lengths: start vector, samples 0..7, samples 8..15
 };
 
 static_assert(sizeof(KSmem) + 4096 <= 232448, "Krylov kernel shared memory exceeds the per-block limit");
@@ -123,6 +140,8 @@ struct KCtx {
   KSmem* sm;
   int rank, size;  // block of the cluster; rank 0 writes the state
   int round;       // rounds of integrals so far
+  int n_integrals;
+  int ts_kmax;     // deepest tanh-sinh level
   int m;
   double h, rho, c;
   int cheb_n;     // Chebyshev vectors available up to this degree
@@ -180,91 +199,116 @@ __device__ void ensure_cheb(KCtx& C, int K) {
   __syncthreads();
 }
 
-// Integrand h |e_m^T exp(-i x T) e_1| by Chebyshev-Bessel, K iterations, on a
-// pair of lanes (all lanes of the warp call it): the even lane runs
-// J_{k-1} = f_k J_k - J_{k+1} and the sums R, I of the signed components, the
-// odd lane f_{k-1} = f_k - 2 / z and the normalisation.  The value is returned
-// to both.
-__device__ double integrand_cheb(const KCtx& C, double x, int K) {
-  const bool jl = (threadIdx.x & 1) == 0;
-  const double* gs = C.sm->gs;
-  double z = x * C.rho;
-  const bool tiny = !(z > 1e-200);
-  if (tiny) z = 1.0;
-  const double inv2z = 2.0 / z;
-  // v: J_k / f_k; c: -J_{k+1} / -2 / z; even: R / normalisation; odd: I / unused
-  double v = jl ? 1e-200 : (double)K * inv2z;
-  double c = jl ? -0.0 : -inv2z;
-  double even = 0.0, odd = 0.0;
-  for (int k = K; k >= 4; k -= 4) {
+// Integrand h |e_m^T exp(-i x T) e_1| by Chebyshev-Bessel, K iterations (a
+// multiple of 4), at nev arguments x = arg(e), results through put(e, value)
+// (block-cooperative).  Warps 0..3 form two sets of 32 arguments: the even warp
+// of a set runs J_{k-1} = f_k J_k - J_{k+1}, f_{k-1} = f_k - 2 / z, the odd one
+// the sums of the signed components and the normalisation.
+template <class Arg, class Put>
+__device__ void integrand_series(const KCtx& C, int nev, int K, Arg arg, Put put) {
+  KSmem* S = C.sm;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, set = warp >> 1;
+  if (warp < 4) {
+    // named barriers of the set: ring block b full / empty again
+    auto sync = [&](int id) { asm volatile("bar.sync %0, 64;" ::"r"(id + 4 * set) : "memory"); };
+    auto arrive = [&](int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id + 4 * set) : "memory"); };
+    const int blocks = (K + 15) / 16;
+    for (int e0 = 32 * set; e0 < nev; e0 += 64) {
+      const double x = arg(min(e0 + lane, nev - 1));
+      double z = x * C.rho;
+      const bool tiny = !(z > 1e-200);
+      if (tiny) z = 1.0;
+      if ((warp & 1) == 0) {
+        const double inv2z = 2.0 / z;
+        double jp1 = 0.0, jk = 1e-200, f = (double)K * inv2z;
+        for (int b = 0; b < blocks; ++b) {
+          if (b >= 2) sync(3 + (b & 1));
+          double(*J)[32] = S->ring[set][b & 1];
+          const int steps = min(16, K - 16 * b);
+          for (int q4 = 0; q4 < steps; q4 += 4) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const double o = __shfl_xor_sync(0xffffffffu, v, 1);
-      const double jk = jl ? v : o;
-      const double w = jl ? gs[k - q] : 2.0;
-      if (q & 1)
-        odd = fma(w, jk, odd);
-      else
-        even = fma(w, jk, even);
-      const double nv = fma(jl ? o : 1.0, v, c);
-      if (jl) c = -v;
-      v = nv;
-    }
-    if (needs_rescale(__shfl_sync(0xffffffffu, v, (threadIdx.x & 31) & ~1))) {
-      const double sc = 0x1p-600;
-      even *= sc;
-      if (jl) {
-        v *= sc;
-        c *= sc;
-        odd *= sc;
+            for (int q = 0; q < 4; ++q) {
+              J[q4 + q][lane] = jk;
+              const double jm = fma(f, jk, -jp1);
+              f -= inv2z;
+              jp1 = jk;
+              jk = jm;
+            }
+            const bool big = needs_rescale(jk);
+            S->rescaled[set][b & 1][q4 >> 2][lane] = big;
+            if (big) {
+              jk *= 0x1p-600;
+              jp1 *= 0x1p-600;
+            }
+          }
+          J[16][lane] = jk;  // J_0 in the last block
+          arrive(1 + (b & 1));
+        }
+      } else {
+        const double* gs = S->gs;
+        double R = 0.0, I = 0.0, nrm = 0.0;
+        for (int b = 0; b < blocks; ++b) {
+          sync(1 + (b & 1));
+          double(*J)[32] = S->ring[set][b & 1];
+          const int steps = min(16, K - 16 * b);
+          for (int q4 = 0; q4 < steps; q4 += 4) {
+            const int k = K - 16 * b - q4;
+            const double j0 = J[q4][lane], j2 = J[q4 + 2][lane];
+            R = fma(gs[k], j0, R);
+            nrm = fma(2.0, j0, nrm);
+            I = fma(gs[k - 1], J[q4 + 1][lane], I);
+            R = fma(gs[k - 2], j2, R);
+            nrm = fma(2.0, j2, nrm);
+            I = fma(gs[k - 3], J[q4 + 3][lane], I);
+            if (S->rescaled[set][b & 1][q4 >> 2][lane]) {
+              R *= 0x1p-600;
+              I *= 0x1p-600;
+              nrm *= 0x1p-600;
+            }
+          }
+          if (b + 1 == blocks) {
+            const double j0 = J[16][lane];  // unnormalised
+            nrm += j0;
+            R = fma(gs[0], j0, R);
+          }
+          if (b + 2 < blocks) arrive(3 + (b & 1));
+        }
+        const double v = tiny ? ((C.m == 1) ? C.h * fabs(gs[0]) : 0.0) : C.h * hypot(R, I) / fabs(nrm);
+        if (e0 + lane < nev) put(e0 + lane, v);
       }
+      sync(3);  // the ring is free for the next arguments
     }
   }
-  // v = J_0 (unnormalised) on the even lane
-  const double j0 = __shfl_sync(0xffffffffu, v, (threadIdx.x & 31) & ~1);
-  even = fma(jl ? gs[0] : 1.0, j0, even);
-  const double R = __shfl_sync(0xffffffffu, even, (threadIdx.x & 31) & ~1);
-  const double nrm = __shfl_sync(0xffffffffu, even, threadIdx.x | 1);
-  const double I = __shfl_sync(0xffffffffu, odd, (threadIdx.x & 31) & ~1);
-  if (tiny) return (C.m == 1) ? C.h * fabs(gs[0]) : 0.0;
-  return C.h * hypot(R, I) / fabs(nrm);
+  __syncthreads();
 }
 
-// Bessel values J_0..J_K(z) into out[], unnormalised, on a group of 4 lanes
-// (all lanes of the warp call it): lane 0 of the group runs
-// J_{k-1} = f_k J_k - J_{k+1}, lane 1 f_k, lane 2 the normalisation, whose
-// value is returned to the group.
-__device__ double bessel_table(double z, int K, double* out, bool active) {
-  const int g = threadIdx.x & 3, l0 = (threadIdx.x & 31) & ~3;
-  const bool tiny = !(z > 1e-200);
-  if (tiny) z = 1.0;
+// Bessel values J_0..J_K(z), unnormalised, into out[] (one thread); returns
+// their normalisation.
+__device__ double bessel_table(double z, int K, double* out) {
+  if (!(z > 1e-200)) {
+    for (int k = 0; k <= K; ++k) out[k] = (k == 0) ? 1.0 : 0.0;
+    return 1.0;
+  }
   const double inv2z = 2.0 / z;
-  // v: J_k / f_k / sum; c: -J_{k+1} / -2 / z / sum
-  double v = g == 0 ? 1e-200 : (g == 1 ? (double)K * inv2z : 0.0);
-  double c = g == 0 ? -0.0 : (g == 1 ? -inv2z : 0.0);
-  const bool w = active && !tiny && g == 0;
-  if (w) out[K] = v;
+  double jp1 = 0.0, jk = 1e-200, nrm = 0.0;
+  double f = (double)K * inv2z;
+  out[K] = jk;
   for (int k = K; k >= 1; --k) {
-    const double jk = __shfl_sync(0xffffffffu, v, l0), f = __shfl_sync(0xffffffffu, v, l0 + 1);
-    if (g == 2) c = v;
-    const double x = g == 0 ? f : (g == 1 ? 1.0 : ((k & 1) == 0 ? 2.0 : 0.0));
-    const double y = g == 2 ? jk : v;
-    const double nv = fma(x, y, c);
-    if (g == 0) c = -v;
-    v = nv;
-    if (w) out[k - 1] = v;
-    if (needs_rescale(__shfl_sync(0xffffffffu, v, l0))) {
+    if ((k & 1) == 0) nrm = fma(2.0, jk, nrm);
+    double jm = fma(f, jk, -jp1);
+    f -= inv2z;
+    jp1 = jk;
+    jk = jm;
+    out[k - 1] = jk;
+    if (needs_rescale(jk)) {
       const double sc = 0x1p-600;
-      if (w)
-        for (int q = k - 1; q <= K; ++q) out[q] *= sc;
-      if (g == 0) c *= sc;
-      if (g != 1) v *= sc;
+      for (int q = k - 1; q <= K; ++q) out[q] *= sc;
+      jk = out[k - 1];
+      jp1 *= sc;
+      nrm *= sc;
     }
   }
-  const double j0 = __shfl_sync(0xffffffffu, v, l0), nrm = __shfl_sync(0xffffffffu, v, l0 + 2) + j0;
-  if (tiny && active && g == 0)
-    for (int k = 0; k <= K; ++k) out[k] = (k == 0) ? 1.0 : 0.0;
-  return tiny ? 1.0 : nrm;
+  return nrm + jk;
 }
 
 // ------------------------------------------------------------ eigen path
@@ -387,22 +431,25 @@ struct IntResult {
 };
 
 // Evaluate the integrand at the abscissae of nodes [n0, n1) of the tanh-sinh
-// table on [a, b] into sm->fp / sm->fm (block-cooperative), two lanes each.
+// table on [a, b] into sm->fp / sm->fm (block-cooperative); t = 0 once.
 __device__ void eval_ts_nodes(KCtx& C, double a, double b, int n0, int n1, bool use_eig, int K) {
   KSmem* S = C.sm;
   const double c = 0.5 * (a + b), d = 0.5 * (b - a);
-  const int nev = 2 * (n1 - n0);
-  const int w0 = (threadIdx.x & ~31) >> 1;  // first evaluation of this warp
-  for (int e0 = w0; e0 < nev; e0 += blockDim.x >> 1) {
-    const int e = e0 + ((threadIdx.x & 31) >> 1);
-    const int node = n0 + (min(e, nev - 1) >> 1);
-    const bool minus = e & 1;
-    const double u = c_quad.ts_u[node];
-    const double x = minus ? c - d * u : c + d * u;
-    const double f = use_eig ? integrand_eig(C, x) : integrand_cheb(C, x, K);
-    // t = 0 is evaluated once
-    if (e < nev && (threadIdx.x & 1) == 0 && !(minus && node == 0)) (minus ? S->fm : S->fp)[node] = f;
+  const int skip = n0 == 0 ? 1 : 0;  // node 0 has no minus side
+  const int nev = 2 * (n1 - n0) - skip;
+  auto node = [&](int e) { return n0 + ((e + skip) >> 1); };
+  auto minus = [&](int e) { return ((e + skip) & 1) != 0 && node(e) != 0; };
+  auto arg = [&](int e) {
+    const int i = node(e);
+    const double u = i < kTsFirstNodes ? S->tsu[i] : g_quad.ts_u[i];
+    return minus(e) ? c - d * u : c + d * u;
+  };
+  auto put = [&](int e, double f) { (minus(e) ? S->fm : S->fp)[node(e)] = f; };
+  if (!use_eig) {
+    integrand_series(C, nev, K, arg, put);
+    return;
   }
+  for (int e = threadIdx.x; e < nev; e += blockDim.x) put(e, integrand_eig(C, arg(e)));
   __syncthreads();
 }
 
@@ -413,7 +460,7 @@ __device__ void ts_level_sum(KCtx& C, int k) {
   double s = 0.0, sa = 0.0;
   bool bad = false;
   for (int node = lb[k] + (int)(threadIdx.x & 31); node < lb[k + 1]; node += 32) {
-    const double w = c_quad.ts_w[node];
+    const double w = node < kTsFirstNodes ? S->tsw[node] : g_quad.ts_w[node];
     if (node == 0) {
       double fv = S->fp[0];
       s = fma(w, fv, s);
@@ -447,20 +494,45 @@ __device__ IntResult ts_integrate(KCtx& C, double a, double b, int K, bool use_e
     ensure_cheb(C, K);
   const double d = 0.5 * (b - a);
   const int* lb = c_quad.ts_level_begin;
-  constexpr int kFirst = 3;  // levels evaluated at once
-  eval_ts_nodes(C, a, b, 0, lb[kFirst + 1], use_eig, K);
+  eval_ts_nodes(C, a, b, 0, kTsFirstNodes, use_eig, K);
   const int warp = threadIdx.x >> 5;
-  if (warp <= kFirst) ts_level_sum(C, warp);
+  if (warp <= kTsFirst) ts_level_sum(C, warp);
   __syncthreads();
   double sum = 0.0, sum_abs = 0.0, prev = 0.0;
   bool nonfinite = false;
-  const int kmax = C.ds->ts_kmax >= TE_TS_KMIN && C.ds->ts_kmax < TE_TS_KMAX ? C.ds->ts_kmax : TE_TS_KMAX;
-  for (int k = 0; k <= kmax; ++k) {
-    if (k > kFirst) {
-      eval_ts_nodes(C, a, b, lb[k], lb[k + 1], use_eig, K);
-      if (warp == 0) ts_level_sum(C, k);
+  const int kmax = C.ts_kmax;
+  // levels 0..3 side by side: lane k of every warp holds the sums up to level
+  // k (added in order), so their estimates take one round of FP64 instructions
+  const int lane = threadIdx.x & 31, kl = min(lane, kTsFirst);
+  double s = 0.0, sa = 0.0;
+#pragma unroll
+  for (int k = 0; k <= kTsFirst; ++k) {
+    const double ns = s + S->lev[k][0], nsa = sa + S->lev[k][1];
+    if (k <= kl) s = ns, sa = nsa;
+  }
+  {
+    const double hk = __hiloint2double((1023 - kl) << 20, 0);  // 2^-k
+    const double Ik = d * hk * s, L1 = d * hk * sa;
+    const double err = fabs(Ik - __shfl_up_sync(0xffffffffu, Ik, 1));
+    const bool stop = kl >= TE_TS_KMIN && err <= 1e-3 * L1;
+    const unsigned int done = __ballot_sync(0xffffffffu, (stop || kl == kmax) && lane <= kTsFirst);
+    const int k = done ? __ffs(done) - 1 : kTsFirst;
+    res.value = __shfl_sync(0xffffffffu, Ik, k);
+    res.err = __shfl_sync(0xffffffffu, err, k);
+    for (int i = 0; i <= k; ++i) nonfinite |= S->bad[i] != 0;
+    sum = __shfl_sync(0xffffffffu, s, k);
+    sum_abs = __shfl_sync(0xffffffffu, sa, k);
+    prev = res.value;
+    if (done) {
+      res.nonfinite = nonfinite;
       __syncthreads();
+      return res;
     }
+  }
+  for (int k = kTsFirst + 1; k <= kmax; ++k) {
+    eval_ts_nodes(C, a, b, lb[k], lb[k + 1], use_eig, K);
+    if (warp == 0) ts_level_sum(C, k);
+    __syncthreads();
     sum += S->lev[k][0];
     sum_abs += S->lev[k][1];
     nonfinite |= S->bad[k] != 0;
@@ -468,10 +540,8 @@ __device__ IntResult ts_integrate(KCtx& C, double a, double b, int K, bool use_e
     const double Ik = d * hk * sum;
     const double L1 = d * hk * sum_abs;
     res.value = Ik;
-    if (k >= 1) {
-      res.err = fabs(Ik - prev);
-      if (k >= TE_TS_KMIN && res.err <= 1e-3 * L1) break;
-    }
+    res.err = fabs(Ik - prev);
+    if (res.err <= 1e-3 * L1) break;
     prev = Ik;
   }
   res.nonfinite = nonfinite;
@@ -488,13 +558,15 @@ __device__ double gauss_integrate(KCtx& C, double a, double b, int npts, int K, 
     ensure_eig(C);
   else
     ensure_cheb(C, K);
+  auto arg = [&](int e) { return c + d * xs[e]; };
+  if (use_eig) {
+    if ((int)threadIdx.x < npts) S->fp[threadIdx.x] = integrand_eig(C, arg(threadIdx.x));
+    __syncthreads();
+  } else {
+    integrand_series(C, npts, K, arg, [&](int e, double f) { S->fp[e] = f; });
+  }
   if (threadIdx.x < 32) {
-    const int i = threadIdx.x >> 1;  // two lanes per abscissa
-    double x = c + d * xs[min(i, npts - 1)];
-    double f = use_eig ? integrand_eig(C, x) : integrand_cheb(C, x, K);
-    // abscissa i's term on lane i
-    double t = __shfl_sync(0xffffffffu, f, (2 * threadIdx.x) & 31);
-    double s = (int)threadIdx.x < npts ? ws[threadIdx.x] * t : 0.0;
+    double s = (int)threadIdx.x < npts ? ws[threadIdx.x] * S->fp[threadIdx.x] : 0.0;
     s = warp_sum_all(s);
     if (threadIdx.x == 0) S->bc[0] = s;
   }
@@ -511,7 +583,7 @@ __device__ double gauss_integrate(KCtx& C, double a, double b, int npts, int K, 
 __device__ bool eval_integral(KCtx& C, const KIntegral& q, double tolRate, double& ret) {
   TeDevState* ds = C.ds;
   const double a = q.a, b = q.b;
-  const int K = bessel_start(fmax(fabs(a), fabs(b)) * C.rho, C.m);
+  const int K = q.K;
   const bool use_eig = K > TE_NCHEB;
   double error = 0.0;
   if (q.method == 0) {
@@ -542,7 +614,8 @@ __device__ __forceinline__ unsigned int cluster_addr(const void* p, int rank) {
 // What the search may ask for next, after [0, t] (from = 0: and the doublings
 // or the halvings and substeps that follow) or substep n of t.
 struct KNext {
-  double t, t_max, s;
+  double t, t_max;
+  int n_substeps;
   int n;        // 0: an interval [0, t]; else substep n
   bool doubling;
   int method_long, method_short;
@@ -553,7 +626,7 @@ struct KNext {
 __device__ double integrate_error(KCtx& C, double a, double b, int method, double tolRate, bool& successful,
                                   const KNext& nx) {
   KSmem* S = C.sm;
-  if (threadIdx.x == 0 && C.rank == 0) C.ds->n_integrals++;
+  ++C.n_integrals;
   int hit = -1;
   for (int i = 0; i < C.size; ++i) {
     const KIntegral& q = S->spec[i];
@@ -568,7 +641,7 @@ __device__ double integrate_error(KCtx& C, double a, double b, int method, doubl
     __syncthreads();
     if ((int)threadIdx.x < C.size) {
       const int i = threadIdx.x;
-      KIntegral q{a, b, method};
+      KIntegral q{a, b, method, 0};
       bool use = true;
       if (i > 0) {
         int n = nx.n + i;  // substeps after substep n
@@ -589,14 +662,15 @@ __device__ double integrate_error(KCtx& C, double a, double b, int method, doubl
           use = i == 1 || nx.t < nx.t_max;
         }
         if (n > 0) {
-          q.a = nx.t + (n - 1) * nx.s;
-          q.b = nx.t + n * nx.s;
+          const double s = nx.t / nx.n_substeps;
+          q.a = nx.t + (n - 1) * s;
+          q.b = nx.t + n * s;
           q.method = nx.method_short;
         }
-        // arguments beyond the series take the eigen-decomposition: only when asked for
-        use = use && bessel_start(fmax(fabs(q.a), fabs(q.b)) * C.rho, C.m) <= TE_NCHEB;
       }
-      if (!use) q.method = -1;
+      q.K = bessel_start(fmax(fabs(q.a), fabs(q.b)) * C.rho, C.m);
+      // arguments beyond the series take the eigen-decomposition: only when asked for
+      if (!use || (i > 0 && q.K > TE_NCHEB)) q.method = -1;
       S->spec[i] = q;
     }
     __syncthreads();
@@ -646,7 +720,7 @@ __device__ int find_step(KCtx& C, double tolRate, double t_stepSuggestion, doubl
   }
   // candidates for the other blocks: what follows an interval [0, t] or substep n
   auto next = [&](double t, int n, bool doubling) {
-    return KNext{t, t_step_max, t / n_substeps, n, doubling, mlong, mshort};
+    return KNext{t, t_step_max, n_substeps, n, doubling, mlong, mshort};
   };
   double err_step =
       integrate_error(C, 0.0, t_step, mlong, tolRate, ok, next(t_step, 0, increaseStep && !skipSubsteps));
@@ -697,96 +771,114 @@ __device__ int find_step(KCtx& C, double tolRate, double t_stepSuggestion, doubl
 
 // ------------------------------------------------------- coefficient vectors
 
-// Y[slot] = s_j i^j [exp(-i dt T) e_1]_j for a group of outputs (at most
-// TE_KBUF) that shares one series length; this block computes outputs first,
-// first + stride, ... of it.
-__device__ void output_coefficients(KCtx& C, const double* dts, const int* slots, int count, int first, int stride) {
+// Y[slot] = s_j i^j [exp(-i dt T) e_1]_j for the outputs of a launch: S->dts[0]
+// (slot 0) when want_w, and the samples S->dts[1..cnt] (slot = index).  The
+// start vector and each group of TE_KBUF samples share a series length.  The
+// start vector goes to the last block of the cluster, samples round the blocks;
+// each block runs all its tables at once (a warp per group).
+__device__ void output_coefficients(KCtx& C, bool want_w, int cnt) {
   KSmem* S = C.sm;
   TeDevState* ds = C.ds;
   const int m = C.m;
-  double zmax = 0.0;
-  for (int o = 0; o < count; ++o) zmax = fmax(zmax, fabs(dts[o]) * C.rho);
-  const int K = bessel_start(zmax, m);
-  const bool use_eig = K > TE_NCHEB;
-  if (use_eig) {  // one eigen-decomposition, on rank 0
-    if (C.rank != 0) return;
-    first = 0;
-    stride = 1;
+  if (threadIdx.x < 3) {
+    const int q = threadIdx.x, o0 = q == 0 ? 0 : 1 + (q - 1) * TE_KBUF;
+    const int o1 = q == 0 ? (want_w ? 1 : 0) : min(o0 + TE_KBUF, cnt + 1);
+    double zmax = 0.0;
+    for (int o = o0; o < o1; ++o) zmax = fmax(zmax, fabs(S->dts[o]) * C.rho);
+    S->outK[q] = o1 > o0 ? bessel_start(zmax, m) : 0;
   }
-  const int own = first < count ? (count - 1 - first) / stride + 1 : 0;
-  if (own == 0) return;
-  if (use_eig)
+  __syncthreads();
+  auto group = [](int o) { return o == 0 ? 0 : 1 + (o - 1) / TE_KBUF; };
+  // own outputs: o = first, first + size, ...; the start vector on the last block
+  const bool own_w = want_w && C.rank == C.size - 1;
+  const int first = 1 + C.rank;
+  const int own = (own_w ? 1 : 0) + (first <= cnt ? (cnt - first) / C.size + 1 : 0);
+  auto output = [&](int i) { return own_w ? (i == 0 ? 0 : first + (i - 1) * C.size) : first + i * C.size; };
+  int K = 0;
+  bool eig = false;
+  for (int q = 0; q < 3; ++q) {
+    if (S->outK[q] > TE_NCHEB)
+      eig = true;
+    else
+      K = max(K, S->outK[q]);
+  }
+  if (eig && C.rank == 0) {  // one eigen-decomposition, on rank 0, for whole groups
     ensure_eig(C);
-  else
-    ensure_cheb(C, K);
-  if (!use_eig) {
-    const int warp = threadIdx.x >> 5;
-    if (warp == 0) {
-      const int i = threadIdx.x >> 2;  // 8 groups of 4 lanes
-      const double nrm = bessel_table(dts[first + min(i, own - 1) * stride] * C.rho, K, S->J[i], i < own);
-      const double inv = 1.0 / nrm;
-      if (i < own && (threadIdx.x & 3) == 0) S->bc[4 + i] = inv;
-    } else if (warp == 1 && (int)(threadIdx.x & 31) < own) {
-      const int i = threadIdx.x & 31;
-      sincos(dts[first + i * stride] * C.c, &S->trig[i][0], &S->trig[i][1]);
+    for (int o = want_w ? 0 : 1; o <= cnt; ++o) {
+      if (S->outK[group(o)] <= TE_NCHEB) continue;
+      for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        const double dt = S->dts[o];
+        double re = 0.0, im = 0.0;
+        for (int k = 0; k < m; ++k) {
+          double q = S->Q[k * TE_MMAX + j] * S->Q[k * TE_MMAX];
+          double sn, cs;
+          sincos(dt * S->lam[k], &sn, &cs);
+          re = fma(q, cs, re);
+          im = fma(-q, sn, im);
+        }
+        double yr, yi;
+        switch (j & 3) {
+          case 0: yr = re; yi = im; break;
+          case 1: yr = -im; yi = re; break;
+          case 2: yr = -re; yi = -im; break;
+          default: yr = im; yi = -re; break;
+        }
+        const double sj = S->s[j];
+        ds->Y[o * TE_MMAX + j] = make_double2(yr * sj, yi * sj);
+      }
     }
+  }
+  if (own == 0 || K == 0) {
     __syncthreads();
-    // signed coefficients a_n = eps_n sigma_n J_n (sigma: + for n%4 in {0,3}, - otherwise)
-    for (int i = threadIdx.x; i < own * (K + 1); i += blockDim.x) {
-      int o = i / (K + 1), n = i % (K + 1);
-      int r = n & 3;
-      double sg = (r == 0 || r == 3) ? 1.0 : -1.0;
-      S->J[o][n] = (S->J[o][n] * S->bc[4 + o]) * ((n == 0) ? 1.0 : 2.0 * sg);
+    return;
+  }
+  ensure_cheb(C, K);
+  // tables: a warp per group, a lane per output; the phases on the last warp
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < 3) {
+    if (lane < own && group(output(lane)) == warp && S->outK[warp] <= TE_NCHEB)
+      S->inv[lane] = 1.0 / bessel_table(S->dts[output(lane)] * C.rho, S->outK[warp], S->J[lane]);
+  } else if (warp == 3 && lane < own) {
+    sincos(S->dts[output(lane)] * C.c, &S->trig[lane][0], &S->trig[lane][1]);
+  }
+  __syncthreads();
+  // signed coefficients eps_n sigma_n J_n (sigma: + for n%4 in {0,3}, - otherwise)
+  for (int i = threadIdx.x; i < own * (K + 1); i += blockDim.x) {
+    const int o = i / (K + 1), n = i % (K + 1);
+    if (n > S->outK[group(output(o))]) continue;
+    const double sg = ((n & 3) == 0 || (n & 3) == 3) ? 1.0 : -1.0;
+    S->J[o][n] = (S->J[o][n] * S->inv[o]) * ((n == 0) ? 1.0 : 2.0 * sg);
+  }
+  __syncthreads();
+  // the even terms (re) and the odd ones (im) of a component on their own
+  // lanes, then times e^{-i dt c}
+  for (int i0 = 0; i0 < 2 * own * m; i0 += blockDim.x) {
+    const int i = min(i0 + (int)threadIdx.x, 2 * own * m - 1);
+    const int c = i & 1, o = (i >> 1) / m, j = (i >> 1) % m;
+    const int out = output(o), Ko = S->outK[group(out)];
+    const bool live = i0 + (int)threadIdx.x < 2 * own * m && Ko <= TE_NCHEB;
+    const double* a = S->J[o];
+    double v = 0.0;
+    if (live) {
+#pragma unroll 4
+      for (int n = c; n <= Ko; n += 2) v = fma(a[n], S->tc[n * TE_MMAX + j], v);
     }
-    __syncthreads();
-    // the even terms (re) and the odd ones (im) of a component on their own
-    // lanes, then times e^{-i dt c}
-    for (int i0 = 0; i0 < 2 * own * m; i0 += blockDim.x) {
-      const int i = min(i0 + (int)threadIdx.x, 2 * own * m - 1);
-      const bool live = i0 + (int)threadIdx.x < 2 * own * m;
-      const int c = i & 1, o = (i >> 1) / m, j = (i >> 1) % m;
-      const double* a = S->J[o];
-      double v = 0.0;
-      for (int n = c; n <= K; n += 2) v = fma(a[n], S->tc[n * TE_MMAX + j], v);
-      const double w = __shfl_xor_sync(0xffffffffu, v, 1);
-      const double sn = S->trig[o][0], cs = S->trig[o][1];
-      // re' = re cs + im sn, im' = im cs - re sn
-      const double x = v * cs, y = w * sn;
-      const double t = c == 0 ? x + y : x - y;
-      // times i^j, then the column scale s_j of the unnormalised basis
-      const double other = __shfl_xor_sync(0xffffffffu, t, 1);
-      const double re = c == 0 ? t : other, im = c == 0 ? other : t;
-      double yv;
-      switch (j & 3) {
-        case 0: yv = c == 0 ? re : im; break;
-        case 1: yv = c == 0 ? -im : re; break;
-        case 2: yv = c == 0 ? -re : -im; break;
-        default: yv = c == 0 ? im : -re; break;
-      }
-      if (live) reinterpret_cast<double*>(&ds->Y[slots[first + o * stride] * TE_MMAX + j])[c] = yv * ds->s[j];
+    const double w = __shfl_xor_sync(0xffffffffu, v, 1);
+    const double sn = S->trig[o][0], cs = S->trig[o][1];
+    // re' = re cs + im sn, im' = im cs - re sn
+    const double x = v * cs, y = w * sn;
+    const double t = c == 0 ? x + y : x - y;
+    // times i^j, then the column scale s_j of the unnormalised basis
+    const double other = __shfl_xor_sync(0xffffffffu, t, 1);
+    const double re = c == 0 ? t : other, im = c == 0 ? other : t;
+    double yv;
+    switch (j & 3) {
+      case 0: yv = c == 0 ? re : im; break;
+      case 1: yv = c == 0 ? -im : re; break;
+      case 2: yv = c == 0 ? -re : -im; break;
+      default: yv = c == 0 ? im : -re; break;
     }
-  } else {
-    for (int i = threadIdx.x; i < own * m; i += blockDim.x) {
-      const int o = i / m, j = i % m;
-      const double dt = dts[o];
-      double re = 0.0, im = 0.0;
-      for (int k = 0; k < m; ++k) {
-        double q = S->Q[k * TE_MMAX + j] * S->Q[k * TE_MMAX];
-        double sn, cs;
-        sincos(dt * S->lam[k], &sn, &cs);
-        re = fma(q, cs, re);
-        im = fma(-q, sn, im);
-      }
-      double yr, yi;
-      switch (j & 3) {
-        case 0: yr = re; yi = im; break;
-        case 1: yr = -im; yi = re; break;
-        case 2: yr = -re; yi = -im; break;
-        default: yr = im; yi = -re; break;
-      }
-      const double sj = ds->s[j];
-      ds->Y[slots[o] * TE_MMAX + j] = make_double2(yr * sj, yi * sj);
-    }
+    if (live) reinterpret_cast<double*>(&ds->Y[out * TE_MMAX + j])[c] = yv * S->s[j];
   }
   __syncthreads();
 }
@@ -804,27 +896,22 @@ __device__ void schedule_batch(KCtx& C, double t_step, bool want_w) {
   double ts = ds->t_sampling;
   const int base = idx;
   const double t = ds->t, ss = ds->sampling_step, t_now = ds->t_now;
-  const int ns = ds->n_samples;
+  const double t_end = t_now + t_step;
+  const int ns = ds->n_samples, max_batch = ds->max_batch;
   const double* times = ds->sample_times;
   auto cond = [&](int i, double tsv) {
     if (i >= ns) return false;
     const double next = times ? times[i] : tsv + ss;
-    return next <= t_now + t_step || (i == ns - 1 && fabs(t_now + t_step - t) <= DBL_EPSILON);
+    return next <= t_end || (i == ns - 1 && fabs(t_end - t) <= DBL_EPSILON);
   };
-  while (cnt < ds->max_batch && cond(idx, ts)) {
+  while (cnt < max_batch && cond(idx, ts)) {
     ts = times ? times[idx] : ts + ss;
-    if (threadIdx.x == 0) {
-      S->dts[1 + cnt] = ts - t_now;
-      S->slots[1 + cnt] = 1 + cnt;
-    }
+    if (threadIdx.x == 0) S->dts[1 + cnt] = ts - t_now;
     ++cnt;
     ++idx;
   }
   const bool pending = cond(idx, ts);
-  if (threadIdx.x == 0) {
-    S->dts[0] = t_step;
-    S->slots[0] = 0;
-  }
+  if (threadIdx.x == 0) S->dts[0] = t_step;
   __syncthreads();
   if (C.size > 1) cluster_barrier();
   if (C.rank == 0 && threadIdx.x == 0) {
@@ -844,11 +931,7 @@ __device__ void schedule_batch(KCtx& C, double t_step, bool want_w) {
       }
     }
   }
-  // the outputs over the blocks: the start vector on the last one, samples
-  // round the others
-  if (want_w) output_coefficients(C, S->dts, S->slots, 1, C.rank == C.size - 1 ? 0 : 1, 1);
-  for (int o0 = 0; o0 < cnt; o0 += TE_KBUF)
-    output_coefficients(C, S->dts + 1 + o0, S->slots + 1 + o0, min(TE_KBUF, cnt - o0), C.rank, C.size);
+  output_coefficients(C, want_w, cnt);
 }
 
 // Load T from the Lanczos coefficients and set up the Chebyshev data.
@@ -856,6 +939,11 @@ __device__ void setup_krylov_matrix(KCtx& C) {
   TeDevState* ds = C.ds;
   KSmem* S = C.sm;
   const int m = C.m;
+  if ((int)threadIdx.x >= TE_MMAX && (int)threadIdx.x < TE_MMAX + kTsFirstNodes) {
+    const int i = threadIdx.x - TE_MMAX;
+    S->tsu[i] = g_quad.ts_u[i];
+    S->tsw[i] = g_quad.ts_w[i];
+  }
   if (threadIdx.x < TE_MMAX) {
     int j = threadIdx.x;
     S->d[j] = j < m ? -ds->alpha[j].y : 0.0;
@@ -874,10 +962,18 @@ __device__ void setup_krylov_matrix(KCtx& C) {
       lo = fmin(lo, S->d[j] - r);
       hi = fmax(hi, S->d[j] + r);
     }
+    // as integers of the same order: minima and maxima off the FP64 pipe
+    auto key = [](double v) {
+      const long long b = __double_as_longlong(v);
+      return b < 0 ? b ^ 0x7fffffffffffffffll : b;
+    };
+    long long klo = key(lo), khi = key(hi);
     for (int o = 16; o > 0; o >>= 1) {
-      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      klo = min(klo, __shfl_xor_sync(0xffffffffu, klo, o));
+      khi = max(khi, __shfl_xor_sync(0xffffffffu, khi, o));
     }
+    lo = __longlong_as_double(klo < 0 ? klo ^ 0x7fffffffffffffffll : klo);
+    hi = __longlong_as_double(khi < 0 ? khi ^ 0x7fffffffffffffffll : khi);
     if (threadIdx.x == 0) {
       double c = 0.5 * (hi + lo), rho = 0.5 * (hi - lo);
       if (!(rho > 1e-300 * fmax(1.0, fabs(c)))) rho = 1.0;
@@ -968,23 +1064,30 @@ __device__ void krylov_step_body(TeDevState* ds, int mode, KSmem* S, int rank, i
   C.rank = rank;
   C.size = size;
   C.round = 0;
+  C.n_integrals = 0;
   if ((int)threadIdx.x < TE_KCLUSTER) {
     S->spec[threadIdx.x].method = -1;
     S->found[0][threadIdx.x].state = S->found[1][threadIdx.x].state = 0;
   }
+  // what the step reads of the state, all loads in flight at once
+  const double t_end = ds->t, t_now = ds->t_now, t_last = ds->t_step, tol_rate = ds->tol_rate, est = ds->num_err_est;
+  const int m_eff = ds->m_eff, bd = ds->breakdown, kmax = ds->ts_kmax;
+  const double h = ds->h;
+  if ((int)threadIdx.x < TE_MMAX) S->s[threadIdx.x] = ds->s[threadIdx.x];
   // every block runs, and has read the state, before any stores into the
   // others' shared memory or writes the state
   if (size > 1)
     cluster_barrier();
   else
     __syncthreads();
-  C.m = ds->m_eff;
-  C.h = ds->h;
+  C.m = m_eff;
+  C.h = h;
+  C.ts_kmax = kmax >= TE_TS_KMIN && kmax < TE_TS_KMAX ? kmax : TE_TS_KMAX;
   C.fatal = 0;
   const bool writer = rank == 0 && threadIdx.x == 0;
   if (mode == 1) {
     load_krylov_data(C);
-    schedule_batch(C, ds->t_step, false);
+    schedule_batch(C, t_last, false);
     if (rank == 0) {
       if (threadIdx.x == 0) ds->want_w = 0;
       __syncthreads();
@@ -993,14 +1096,13 @@ __device__ void krylov_step_body(TeDevState* ds, int mode, KSmem* S, int rank, i
     if (size > 1) cluster_barrier();
     return;
   }
-  const bool hbd = ds->breakdown != 0;
+  const bool hbd = bd != 0;
   double t_step = 0.0;
   int code = 0;
-  if (writer) ds->n_integrals = 0;
   setup_krylov_matrix(C);
   if (hbd) {
     // lucky breakdown (:342-363): the remaining time in one step, m reduced for good
-    t_step = ds->t - ds->t_now;
+    t_step = t_end - t_now;
     if (size > 1) cluster_barrier();
     if (writer) {
       ds->t_step = t_step;
@@ -1011,10 +1113,9 @@ __device__ void krylov_step_body(TeDevState* ds, int mode, KSmem* S, int rank, i
       ds->new_start = 0;
     }
   } else {
-    const double s0 = 0.97 * ds->t_step;
+    const double s0 = 0.97 * t_last;
     double err_step = 0.0;
-    code = find_step(C, ds->tol_rate, s0, ds->t - ds->t_now, 50, ds->num_err_est, ds->t_now == 0.0, &t_step,
-                     &err_step);
+    code = find_step(C, tol_rate, s0, t_end - t_now, 50, est, t_now == 0.0, &t_step, &err_step);
     if (size > 1) cluster_barrier();
     if (code < 0) {
       if (writer) ds->fatal = code == -1 ? TE_ERR_NO_STEP : TE_ERR_UNSUPPORTED;
@@ -1029,6 +1130,7 @@ __device__ void krylov_step_body(TeDevState* ds, int mode, KSmem* S, int rank, i
     }
   }
   if (writer) {
+    ds->n_integrals = C.n_integrals;
     switch (ds->err_code_find) {  // :386-399 (a breakdown step re-counts the previous code)
       case 1: ds->nb_err_roundoff++; break;
       case 20: ds->nb_err_int++; break;
@@ -1211,7 +1313,12 @@ int te_upload_quad_tables() {
   };
   gauss(15, T.g15_x, T.g15_w);
   gauss(7, T.g7_x, T.g7_w);
+  if (T.ts_level_begin[kTsFirst + 1] != kTsFirstNodes) {
+    te_set_error("tanh-sinh table: unexpected first levels");
+    return TE_ERR_UNSUPPORTED;
+  }
   TE_CUDA(cudaMemcpyToSymbol(c_quad, &T, sizeof(T)));
+  TE_CUDA(cudaMemcpyToSymbol(g_quad, &T, sizeof(T)));
   TE_CUDA(cudaFuncSetAttribute(krylov_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KSmem)));
   TE_CUDA(cudaFuncSetAttribute(krylov_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KSmem)));
   // the largest cluster whose blocks (one per SM: their shared memory) can run together
