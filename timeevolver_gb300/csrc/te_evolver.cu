@@ -363,7 +363,6 @@ int run(te_evolver ev, te_result* out) {
   const bool one_launch = ev->fused_lanczos != 0 && ev->p.reorth == 0 && ev->p.exp_factor != 0.0 && sell.n_long == 0 &&
                           (sell.lanes == 1 || !(sell.lanes_pinned || sell.lanes_timed));
   const bool small = one_launch && sell.n_chunks < 2048;
-  const bool resident = one_launch && !small && ev->resident && te_resident_fits(sell);
   bool fix = ev->fixed_spmv != 0 && ev->p.reorth == 0 && ev->p.exp_factor != 0.0 && sell.n_chunks >= 2048 &&
              ev->fused_lanczos != 2;
   if (fix) {
@@ -381,6 +380,8 @@ int run(te_evolver ev, te_result* out) {
     }
   }
   if (!fix && (rc = te_tune_sell_lanes(ev->H)) != TE_OK) return rc;
+  const bool resident =
+      one_launch && !small && ev->resident && (te_resident_fits(sell) || (fix && te_stream_fits(sell)));
   if (small && !ev->step_sync) {
     TE_CUDA(te_malloc(&ev->step_sync, sizeof(TeStepSync)));
     TE_CUDA(cudaMemsetAsync(ev->step_sync, 0, sizeof(TeStepSync), st));

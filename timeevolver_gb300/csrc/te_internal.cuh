@@ -409,6 +409,9 @@ struct TeResidentSync {
   unsigned long long umax[256];              // tagged max|u_0|, one per block
 };
 bool te_resident_fits(const TeSell& A);
+// Larger matrices, fixed point: rows streamed, w' in shared memory
+// (launched by te_launch_lanczos_resident).
+bool te_stream_fits(const TeSell& A);
 bool te_launch_lanczos_resident(const TeSell& A, bool is_real, bool fixed, double norm1, double2* const* cols, int m,
                                 int4* X, TeDevState* ds, TeResidentSync* sync, unsigned int launch,
                                 cudaStream_t st, unsigned int spin_limit, unsigned int extra_arrivals);

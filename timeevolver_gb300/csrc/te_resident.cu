@@ -43,6 +43,17 @@ namespace {
 
 constexpr int kResWarps = 19;     // worker warps per block at most
 constexpr int kResMaxCpw = 4;     // chunks per worker warp at most
+constexpr int kStreamMaxWarps = 31;        // worker warps per block of the streaming kernel at most
+constexpr size_t kStreamSmem = 216 << 10;  // its dynamic shared memory at most
+// Worker warps and slots in flight per lane by format (0 real limbs, 1 value
+// dictionary, 2 complex limbs): more warps leave fewer registers for slots in
+// flight.  Measured per iteration on GB300, dictionary (Bose-Hubbard L=12): 31
+// warps of 2 / 4 / 6 slots 79 / 66 / 63 us, 27 of 6 68, 23 of 8 71; complex
+// (dim 1 000 003, 49 M entries): 31 of 6 235 us, 27 of 6 222, 23 of 8 216.
+template <int FMT>
+constexpr int kStreamWarps = FMT == 1 ? 31 : FMT == 2 ? 23 : 27;
+template <int FMT>
+constexpr int kStreamSlots = FMT == 2 ? 8 : 6;
 constexpr int kAlphaWords = 10;   // <u_j, w'>: re, im (4 limbs of 24 bits each), 2 words of exponent counts
 constexpr int kNormWords = 7;     // ||u_{j+1}||^2: 5 limbs, 2 words of exponent counts
 constexpr int kCountShift = 48;   // blocks counted in bits 48..63 of a word
@@ -55,8 +66,8 @@ __device__ __forceinline__ int exp_above(double v) { return exp_above(te_fix_hiw
 __device__ __forceinline__ double pow2(int x) { return __hiloint2double((min(max(x, -1022), 1023) + 1023) << 20, 0); }
 
 struct ResShared {
-  unsigned long long part[kResWarps][8];  // per-warp limb sums
-  unsigned int pmax[kResWarps];
+  unsigned long long part[kStreamMaxWarps][8];  // per-warp limb sums
+  unsigned int pmax[kStreamMaxWarps];
   double cw, gr, gi;
   int k1, k2, xs;    // units of the two sums, fixed-point scale of u_{j+1}
   int ew, eu;        // exponents that the maxima of w' and u_{j+1} are counted from
@@ -272,6 +283,68 @@ __device__ __forceinline__ bool res_start_max(const TeResidentArgs& a, const Res
   }
 }
 
+// Spare warp, from the grid's words of <u_j, w'> and max|w'|: alpha_j / e =
+// S_j <u_j, w'>, the fixed-point scale of u_{j+1} and the units of its norm.
+__device__ __forceinline__ void res_alpha(const TeResidentArgs& a, ResShared& S, unsigned long long word, double Sj,
+                                          int eu, double e, int j, bool leader, int G, TeDevState* ds) {
+  // the even lanes join re, the odd lanes im
+  const int lane = threadIdx.x & 31, im = lane & 1;
+  unsigned long long t[4], lo, hi;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) t[i] = __shfl_sync(0xffffffffu, word, i + 4 * im);
+  const int ew = exp_of_counts(__shfl_sync(0xffffffffu, word, 8), __shfl_sync(0xffffffffu, word, 9), S.ew);
+  limbs_join<4>(t, (unsigned long long)G * kTopBias, lo, hi);
+  double g = Sj * te_i128_to_double(lo, hi, -S.k1);
+  if (ew == 0x7fffffff || eu > 1024) g = __longlong_as_double(0x7ff8000000000000ll);
+  const double go = __shfl_xor_sync(0xffffffffu, g, 1);
+  // |u_{j+1}| < B
+  const double B = fma(fabs(g) + fabs(go), pow2(eu), pow2(ew)) * (1.0 + 1e-12);
+  const int eb = exp_above(B), xs = te_fix_scale(B);
+  if (lane == 0) {
+    S.gr = g;
+    S.gi = go;
+    S.xs = xs;
+    S.k2 = a.X ? 2 * xs - 62 : 117 - (2 * eb + a.n_exp);
+    S.eu = eb;
+    if (leader) {
+      ds->alpha[j] = make_double2(g * e, go * e);
+      if (a.X) ds->fx_xs[j + 1] = xs;
+    }
+  }
+  __syncwarp();
+}
+
+// ||u_{j+1}||^2 from the grid's words; returns the exponent above max|u_{j+1}|.
+__device__ __forceinline__ int res_norm(const ResShared& S, unsigned long long word, int G, double& norm2) {
+  unsigned long long t[kNormWords - 2], lo, hi;
+#pragma unroll
+  for (int i = 0; i < kNormWords - 2; ++i) t[i] = __shfl_sync(0xffffffffu, word, i);
+  const int en = exp_of_counts(__shfl_sync(0xffffffffu, word, kNormWords - 2),
+                               __shfl_sync(0xffffffffu, word, kNormWords - 1), S.eu);
+  limbs_join<kNormWords - 2>(t, (unsigned long long)G * kTopBias, lo, hi);
+  norm2 = te_u128_to_double(hi, lo, -S.k2);
+  if (en == 0x7fffffff) norm2 = __longlong_as_double(0x7ff8000000000000ll);
+  return en;
+}
+
+// End of a launch, first block: the step's coefficients beta_j = |e| sqrt((beta_j
+// / e)^2), s_j = +-1 / ||u_j|| (s_j = e s_{j-1} / beta_j); the last one is h, or
+// the breakdown's.
+__device__ void res_coefficients(const ResShared& S, int last_j, bool broke, double bd2, double e, TeDevState* ds) {
+  for (int j = 1 + (int)threadIdx.x; j <= last_j; j += blockDim.x) {
+    const double b = fabs(e) * sqrt(S.cws[j]);
+    if (j < last_j) {
+      const double sn = 1.0 / sqrt(S.norm2[j]);
+      ds->beta[j] = b;
+      ds->s[j] = e < 0.0 && (j & 1) ? -sn : sn;
+    } else {
+      ds->h = b;
+      ds->m_eff = j;
+      if (broke || S.cws[j] < bd2) ds->breakdown = 1;
+    }
+  }
+}
+
 template <int FMT, int CPW>
 __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kernel(TeResidentArgs a, TeDevState* ds) {
   constexpr bool FIX = FMT < 3;
@@ -400,33 +473,7 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
       res_send<kAlphaWords>(a, S, words, S.ew);
       unsigned long long word;
       const bool ok = res_receive<kAlphaWords>(a, words, word, ds);
-      if (ok) {
-        // lane 0 (and every even lane) joins re, the odd lanes im
-        const int im = lane & 1;
-        unsigned long long t[4], lo, hi;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) t[i] = __shfl_sync(0xffffffffu, word, i + 4 * im);
-        const int ew = exp_of_counts(__shfl_sync(0xffffffffu, word, 8), __shfl_sync(0xffffffffu, word, 9), S.ew);
-        limbs_join<4>(t, (unsigned long long)G * kTopBias, lo, hi);
-        double g = Sj * te_i128_to_double(lo, hi, -S.k1);
-        if (ew == 0x7fffffff || eu > 1024) g = __longlong_as_double(0x7ff8000000000000ll);
-        const double go = __shfl_xor_sync(0xffffffffu, g, 1);
-        // |u_{j+1}| < B: the fixed-point scale, and the units of ||u_{j+1}||^2
-        const double B = fma(fabs(g) + fabs(go), pow2(eu), pow2(ew)) * (1.0 + 1e-12);
-        const int eb = exp_above(B);
-        xs = te_fix_scale(B);
-        if (lane == 0) {
-          S.gr = g;
-          S.gi = go;
-          S.xs = xs;
-          S.k2 = FIX ? 2 * xs - 62 : 117 - (2 * eb + a.n_exp);
-          S.eu = eb;
-          if (leader) {
-            ds->alpha[j] = make_double2(g * e, go * e);
-            if (FIX) ds->fx_xs[j + 1] = xs;
-          }
-        }
-      }
+      if (ok) res_alpha(a, S, word, Sj, eu, e, j, leader, G, ds);
       if (lane == 0) S.go = ok ? 1 : 0;
     }
     __syncthreads();
@@ -485,14 +532,7 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
         fence_gpu();  // the other blocks' rows, after their sums
       }
       if (ok && (!last || leader)) {
-        unsigned long long t[kNormWords - 2], lo, hi;
-#pragma unroll
-        for (int i = 0; i < kNormWords - 2; ++i) t[i] = __shfl_sync(0xffffffffu, word, i);
-        const int en = exp_of_counts(__shfl_sync(0xffffffffu, word, kNormWords - 2),
-                                     __shfl_sync(0xffffffffu, word, kNormWords - 1), S.eu);
-        limbs_join<kNormWords - 2>(t, (unsigned long long)G * kTopBias, lo, hi);
-        norm2 = te_u128_to_double(hi, lo, -S.k2);
-        if (en == 0x7fffffff) norm2 = __longlong_as_double(0x7ff8000000000000ll);
+        const int en = res_norm(S, word, G, norm2);
         eup = eu;
         eu = en;
         if (last && lane == 0) {
@@ -505,21 +545,255 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
     __syncthreads();
     if (!S.go) return;
   }
-  // the step's coefficients: beta_j = |e| sqrt((beta_j / e)^2), s_j = +-1 / ||u_j||
-  // (s_j = e s_{j-1} / beta_j); the last one is h, or the breakdown's
-  if (!leader) return;
-  for (int j = 1 + (int)threadIdx.x; j <= last_j; j += blockDim.x) {
-    const double b = fabs(e) * sqrt(S.cws[j]);
-    if (j < last_j) {
-      const double sn = 1.0 / sqrt(S.norm2[j]);
-      ds->beta[j] = b;
-      ds->s[j] = e < 0.0 && (j & 1) ? -sn : sn;
-    } else {
-      ds->h = b;
-      ds->m_eff = j;
-      if (broke || S.cws[j] < bd2) ds->breakdown = 1;
+  if (leader) res_coefficients(S, last_j, broke, bd2, e, ds);
+}
+
+// --------------------------------------------------------------------------
+// The same iterations for rows that do not fit the registers (fixed point
+// only): chunk c belongs to block c mod gridDim.x, the block's warps take its
+// chunks in turn (the same ones in every iteration), w' of its rows stays in
+// shared memory, u_j and u_{j-1} are read back. Against the two passes an
+// iteration saves w' through memory, two launches and the serial FP64 start of
+// every block (square root and divisions on the spare warp here).  What bounds
+// it is a warp's own chain per chunk (offsets, words, gathers, rows: 9 000
+// cycles) at 31 warps an SM, then the rows' FP64 recurrence (39% of the pipe's
+// cycles); the slot loop has no predicates (groups of U, then 4, 2, 1) and
+// 32-bit counters, since predicated groups with the next words fetched ahead
+// doubled the instructions (95 us).  Gathers made coalesced, or all from L1,
+// change nothing (61.4, 59.4 us), nor does a value table per lane (62.1).
+// Measured on GB300 per iteration: Bose-Hubbard L=12 (dim 1 352 078, 113 values)
+// 85.6 us in two passes, 61.4 us here; complex, dim 1 000 003, 49 M entries: 293
+// -> 216 us.  In the L=12 iteration's 124 000 cycles the row sums take 85 000,
+// the update 22 000, the two exchanges with their scalars 16 000.
+template <int FMT, int U>
+__device__ __forceinline__ void stream_slots(const TeResidentArgs& a, const int2* tab, int s, const int4* X,
+                                             int64_t& sr, int64_t& si) {
+  int4 x[U];
+  if (FMT == 1) {
+    const uint32_t cmask = (1u << a.cbits) - 1u;
+    uint32_t wd[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) wd[q] = __ldcs(a.pk + s + 32 * q);
+#pragma unroll
+    for (int q = 0; q < U; ++q) x[q] = __ldca(X + (wd[q] & cmask));
+#pragma unroll
+    for (int q = 0; q < U; ++q) te_fix_mac(tab[wd[q] >> a.cbits], x[q], sr, si);
+  } else if (FMT == 0) {
+    int2 h[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      h[q] = __ldcs(a.hv + s + 32 * q);
+      x[q] = __ldca(X + (uint32_t)__ldcs(a.col + s + 32 * q));
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) te_fix_mac(h[q], x[q], sr, si);
+  } else {
+    int4 h[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      h[q] = __ldcs(a.hv4 + s + 32 * q);
+      x[q] = __ldca(X + (uint32_t)__ldcs(a.col + s + 32 * q));
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      sr += te_fix_prod(h[q].x, h[q].y, x[q].x, x[q].y) - te_fix_prod(h[q].z, h[q].w, x[q].z, x[q].w);
+      si += te_fix_prod(h[q].x, h[q].y, x[q].z, x[q].w) + te_fix_prod(h[q].z, h[q].w, x[q].x, x[q].y);
     }
   }
+}
+
+template <int FMT>
+__global__ void __launch_bounds__((kStreamWarps<FMT> + 1) * 32, 1)
+    lanczos_stream_kernel(TeResidentArgs a, TeDevState* ds) {
+  constexpr int W = kStreamWarps<FMT>, U = kStreamSlots<FMT>;
+  __shared__ ResShared S;
+  extern __shared__ __align__(16) unsigned char dyn[];  // w' of the block's rows; FMT 1: the value table
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int G = gridDim.x;
+  const bool leader = blockIdx.x == 0;
+  TeResidentSync& sy = *a.sync;
+  if (leader)  // the other half, for the next launch (no launch in flight uses it)
+    for (int i = threadIdx.x; i < TE_MMAX * 32; i += blockDim.x) (&sy.words[a.parity ^ 1][0][0])[i] = 0ull;
+  if (ds->fatal != 0 || ds->done != 0 || ds->breakdown != 0) return;
+  // chunks blockIdx.x + i G, i < nc; warp w takes i = w, w + W, ...
+  const int nc = (a.n_chunks - (int)blockIdx.x + G - 1) / G;
+  double2* ws = reinterpret_cast<double2*>(dyn);
+  int2* tab = reinterpret_cast<int2*>(ws + nc * 32);
+  if (FMT == 1)
+    for (int i = threadIdx.x; i < a.nvals; i += blockDim.x) tab[i] = a.table[i];
+  const int m = min(a.m, ds->m_cur);
+  const double e = ds->exp_factor;
+  const bool spare = warp == W;
+  const uint32_t n32 = (uint32_t)a.n;
+  double Sj = 1.0, norm2 = 1.0;  // the spare warp's, as in the resident kernel
+  int eu = exp_above(ds->fx_umax[0]), eup = -4000;
+  int xs = ds->fx_xs[0];
+  const double bd2 = (ds->tol_rate / e) * (ds->tol_rate / e);
+  int last_j = m;
+  bool broke = false;
+  __syncthreads();  // the value table
+  for (int j = 0; j < m; ++j) {
+    unsigned long long* words = sy.words[a.parity][j];
+    const int4* X = a.X + (int64_t)j * a.n;
+    const double2 *uj = a.u[j], *up = a.u[j > 0 ? j - 1 : 0];
+    double dr = 0.0, di = 0.0;
+    unsigned int mx = 0;
+    if (spare) {
+      const double cw = j > 0 ? Sj * norm2 : 0.0;  // (beta_j / e)^2
+      const bool go = !(cw < bd2) || j == 0;       // else the lucky breakdown (:551-555)
+      const int ecw = j > 0 ? exp_above(cw) : -4000;
+      if (lane == 0) {
+        S.cw = cw;
+        S.go_start = go ? 1 : 0;
+        const int ex = j == 0 ? 2 * eu + a.n_exp : exp_above(norm2);
+        S.k1 = 82 - ex - max(a.r_exp, (ecw + 2) / 2);
+        S.ew = max(a.r_exp + eu, ecw + eup) + 1;
+        if (leader && j > 0) {
+          S.norm2[j] = norm2;
+          S.cws[j] = cw;
+        }
+      }
+      if (j > 0) Sj = 1.0 / norm2;
+    }
+    // apply; the first chunk's row sums before the scalars are needed
+    bool first = true;
+    double cw = 0.0;
+    if (!spare) {
+      const int shift = a.sh + xs;
+      for (int i = warp; i < nc; i += W) {
+        const int c = (int)blockIdx.x + i * G;
+        int s = (int)__ldg(a.chunk_off + c);
+        int len = ((int)__ldg(a.chunk_off + c + 1) - s) >> 5;
+        s += lane;
+        const uint32_t r = (uint32_t)c * 32u + lane;
+        const bool live = r < n32;
+        int64_t sr = 0, si = 0;
+        for (; len >= U; len -= U, s += 32 * U) stream_slots<FMT, U>(a, tab, s, X, sr, si);
+        if (len >= 4) {
+          stream_slots<FMT, 4>(a, tab, s, X, sr, si);
+          s += 128;
+          len -= 4;
+        }
+        if (len >= 2) {
+          stream_slots<FMT, 2>(a, tab, s, X, sr, si);
+          s += 64;
+          len -= 2;
+        }
+        if (len) stream_slots<FMT, 1>(a, tab, s, X, sr, si);
+        const double yr = te_i64_to_double(sr, 62 - shift), yi = te_i64_to_double(si, 62 - shift);
+        if (first) {  // the spare warp's scalars
+          asm volatile("bar.sync 1, %0;" ::"r"((W + 1) * 32) : "memory");
+          first = false;
+          if (!S.go_start) break;
+          cw = S.cw;
+        }
+        if (live) {
+          // w' = -i H u_j + c_w u_{j-1}; <u_j, w'> += conj(u_j) w'
+          const double2 u = __ldca(uj + r);
+          double2 w = make_double2(yi, -yr);
+          if (j > 0) {
+            const double2 v = __ldca(up + r);
+            w.x = fma(cw, v.x, yi);
+            w.y = fma(cw, v.y, -yr);
+          }
+          ws[i * 32 + lane] = w;
+          dr = fma(u.x, w.x, fma(u.y, w.y, dr));
+          di = fma(u.x, w.y, fma(-u.y, w.x, di));
+          mx = max(mx, max(te_fix_hiword(w.x), te_fix_hiword(w.y)));
+        }
+      }
+    }
+    if (first) asm volatile("bar.sync 1, %0;" ::"r"((W + 1) * 32) : "memory");
+    if (!S.go_start) {
+      last_j = j;
+      broke = true;
+      break;
+    }
+    if (!spare) {
+      int limb[8];
+      unsigned long long lo, hi;
+      te_fix_encode128(dr, S.k1, lo, hi);
+      limbs4(lo, hi, limb);
+      te_fix_encode128(di, S.k1, lo, hi);
+      limbs4(lo, hi, limb + 4);
+      warp_limbs<8>(limb, S.part[warp]);
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      if (lane == 0) S.pmax[warp] = mx;
+    }
+    __syncthreads();
+    if (spare) {
+      unsigned long long word;
+      res_send<kAlphaWords>(a, S, words, S.ew);
+      const bool ok = res_receive<kAlphaWords>(a, words, word, ds);
+      if (ok) res_alpha(a, S, word, Sj, eu, e, j, leader, G, ds);
+      if (lane == 0) S.go = ok ? 1 : 0;
+    }
+    __syncthreads();
+    if (!S.go) return;
+    xs = S.xs;
+    if (!spare) {
+      // update: u_{j+1} = w' - (alpha_j / e) u_j
+      const double gr = S.gr, gi = S.gi;
+      unsigned long long lo = 0, hi = 0;
+      mx = 0;
+      int4* Xn = a.X + (int64_t)(j + 1) * a.n;
+      double2* un = a.u[j + 1 < m ? j + 1 : j];
+#pragma unroll 2
+      for (int i = warp; i < nc; i += W) {
+        const uint32_t r = ((uint32_t)blockIdx.x + (uint32_t)i * G) * 32u + lane;
+        if (r < n32) {
+          const double2 w = ws[i * 32 + lane], u = __ldca(uj + r);
+          double2 o;
+          o.x = fma(-gr, u.x, fma(gi, u.y, w.x));
+          o.y = fma(-gr, u.y, fma(-gi, u.x, w.y));
+          mx = max(mx, max(te_fix_hiword(o.x), te_fix_hiword(o.y)));
+          const int64_t er = te_fix_encode(o.x, xs), ei = te_fix_encode(o.y, xs);
+          if (j + 1 < m) {
+            const int2 p = te_fix_split(er), q = te_fix_split(ei);
+            Xn[r] = make_int4(p.x, p.y, q.x, q.y);
+            un[r] = o;
+          }
+          const unsigned long long sq = te_fix_sq(er) + te_fix_sq(ei);
+          lo += sq;
+          hi += lo < sq ? 1ull : 0ull;
+        }
+      }
+      int limb[kNormWords - 2];
+      limb[0] = (int)(lo & 0xffffffull);
+      limb[1] = (int)((lo >> 24) & 0xffffffull);
+      limb[2] = (int)(((lo >> 48) | (hi << 16)) & 0xffffffull);
+      limb[3] = (int)((hi >> 8) & 0xffffffull);
+      limb[4] = (int)((hi >> 32) & 0xffffffull);
+      warp_limbs<kNormWords - 2>(limb, S.part[warp]);
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      if (lane == 0) S.pmax[warp] = mx;
+    }
+    __syncthreads();
+    const bool last = j + 1 == m;
+    if (spare) {
+      fence_gpu();  // the rows this block stored, before its sums
+      res_send<kNormWords>(a, S, words + 16, S.eu);
+      unsigned long long word;
+      bool ok = true;
+      if (!last || leader) {
+        ok = res_receive<kNormWords>(a, words + 16, word, ds);
+        fence_gpu();  // the other blocks' rows, after their sums
+      }
+      if (ok && (!last || leader)) {
+        const int en = res_norm(S, word, G, norm2);
+        eup = eu;
+        eu = en;
+        if (last && lane == 0) {
+          S.cws[m] = Sj * norm2;
+          S.norm2[m] = norm2;
+        }
+      }
+      if (lane == 0) S.go = ok ? 1 : 0;
+    }
+    __syncthreads();
+    if (!S.go) return;
+  }
+  if (leader) res_coefficients(S, last_j, broke, bd2, e, ds);
 }
 
 namespace {
@@ -548,6 +822,14 @@ ResKernel res_kernel(int fmt, int cpw) {
 
 }  // namespace
 
+// w' of a block's rows and the value table fit its shared memory (2.0 million
+// rows on 152 SMs), fixed-point form built.
+bool te_stream_fits(const TeSell& A) {
+  if (A.n_long > 0 || A.fix_nblk > 0 || te_num_sms() > 255 || A.slots >= ((int64_t)1 << 31) - 256) return false;
+  const int64_t most = (A.n_chunks + te_num_sms() - 1) / te_num_sms();
+  return (size_t)most * 512 + sizeof(int2) * A.fix_nvals <= kStreamSmem;
+}
+
 // Rows that fit the registers of one block per SM: kResWarps warps of
 // kResMaxCpw chunks (369 664 rows on 152 SMs).
 bool te_resident_fits(const TeSell& A) {
@@ -557,19 +839,16 @@ bool te_resident_fits(const TeSell& A) {
 }
 
 bool te_launch_lanczos_resident(const TeSell& A, bool is_real, bool fixed, double norm1, double2* const* cols, int m,
-                                int4* X, TeDevState* ds, TeResidentSync* sync, unsigned int launch,
-                                cudaStream_t st, unsigned int spin_limit, unsigned int extra_arrivals) {
-  if (m < 1 || m > TE_MMAX || !te_resident_fits(A)) return false;
-  TeResidentArgs a{};
-  const int fmt = fixed ? (A.fix_val4 ? 2 : (A.fix_pk ? 1 : 0)) : (is_real ? 3 : 4);
-  const size_t smem = fmt == 1 ? sizeof(int2) * A.fix_nvals : 0;
-  const int G = (int)std::min<int64_t>(te_num_sms(), A.n_chunks);
+                                int4* X, TeDevState* ds, TeResidentSync* sync, unsigned int launch, cudaStream_t st,
+                                unsigned int spin_limit, unsigned int extra_arrivals) {
+  const bool stream = !te_resident_fits(A);
+  if (m < 1 || m > TE_MMAX || (stream && !(fixed && te_stream_fits(A)))) return false;
+  const int G = stream ? te_num_sms() : (int)std::min<int64_t>(te_num_sms(), A.n_chunks);
   const int per_block = (int)((A.n_chunks + G - 1) / G);
   const int cpw = (per_block + kResWarps - 1) / kResWarps;
-  const int workers = (per_block + cpw - 1) / cpw;
+  TeResidentArgs a{};
   a.n = A.n;
   a.n_chunks = (int)A.n_chunks;
-  a.n_workers = workers;
   a.m = m;
   a.chunk_off = A.chunk_off;
   a.col = A.col;
@@ -587,17 +866,31 @@ bool te_launch_lanczos_resident(const TeSell& A, bool is_real, bool fixed, doubl
   a.r_exp = ex;
   a.n_exp = 2;
   while (((int64_t)1 << (a.n_exp - 2)) < A.n) ++a.n_exp;
-  a.X = X;
+  a.X = fixed ? X : nullptr;
   a.sync = sync;
   a.parity = (int)(launch & 1u);
   a.epoch = launch + 1u;
   a.spin_limit = spin_limit;
   a.arrivals = (unsigned int)G + extra_arrivals;
   for (int j = 0; j < TE_MMAX; ++j) a.u[j] = j < m ? cols[j] : nullptr;
-  const ResKernel k = res_kernel(fmt, cpw);
+  const int fmt = fixed ? (A.fix_val4 ? 2 : (A.fix_pk ? 1 : 0)) : (is_real ? 3 : 4);
+  a.n_workers = stream ? (fmt == 1 ? kStreamWarps<1> : fmt == 2 ? kStreamWarps<2> : kStreamWarps<0>) : (per_block + cpw - 1) / cpw;
+  const ResKernel k = !stream    ? res_kernel(fmt, cpw)
+                      : fmt == 2 ? lanczos_stream_kernel<2>
+                      : fmt == 1 ? lanczos_stream_kernel<1>
+                                 : lanczos_stream_kernel<0>;
+  size_t smem = fmt == 1 ? sizeof(int2) * A.fix_nvals : 0;
+  if (stream) {
+    smem += (size_t)per_block * 512;
+    if (cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmem) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(G);
-  cfg.blockDim = dim3((workers + 1) * 32);
+  cfg.blockDim = dim3((a.n_workers + 1) * 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
