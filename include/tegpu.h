@@ -79,7 +79,9 @@ int te_set_device(int device);
  * cached device bytes (default 8 GiB; 0 disables the cache and frees what it
  * holds), te_release_buffers frees every cached block, te_buffer_cache_bytes
  * reports the cached device bytes.  A failed allocation releases the cache
- * and tries again. */
+ * and tries again.  The scratch of te_matrix_spmv comes from a stream-ordered
+ * pool that keeps at most 128 MB beside the cache, no more than the cap, and is
+ * emptied with it. */
 int te_set_buffer_cache_limit(int64_t device_bytes);
 int te_release_buffers(void);
 int64_t te_buffer_cache_bytes(void);
@@ -242,8 +244,8 @@ int te_matrix_destroy(te_matrix A);
 int te_matrix_info(te_matrix A, int64_t* n_rows, int64_t* n_cols, int64_t* nnz, int* flags, double* norm1);
 
 /* out = alpha * A * in on device buffers (complex n), on a CUDA stream
- * (NULL = the library's stream).  Replaces smatrix::spMV
- * (matrixDataTypes.cpp:169-190). */
+ * (NULL = the library's stream); in and out may be the same or overlap.
+ * Replaces smatrix::spMV (matrixDataTypes.cpp:169-190). */
 int te_matrix_spmv(te_matrix A, double alpha_re, double alpha_im, const double* in_dev, double* out_dev,
                    void* cuda_stream);
 
@@ -255,7 +257,7 @@ int te_matrix_spmv_host(te_matrix A, double alpha_re, double alpha_im, const dou
  * cudaMalloc (work recorded into CUDA graphs by stream capture, real-time
  * loops, hosts whose device memory is preallocated by another framework).
  * No counterpart in the reference.  Its scratch is a fixed array inside the
- * library (8 MiB on every GPU that loads it), so matrices are limited to
+ * library (4 MiB on every GPU that loads it), so matrices are limited to
  * 262144 rows (TE_ERR_UNSUPPORTED beyond); the first call on a device looks
  * the array up and should come before any stream capture; calls whose
  * executions overlap on the GPU share the array and race. */

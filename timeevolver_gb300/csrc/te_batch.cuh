@@ -318,7 +318,7 @@ __device__ __forceinline__ void batch_apply_warp(const BatchGeom& g, const Batch
     const int n_i = __ldg(g.inst_n + inst);
     double a0 = 0.0, a1 = 0.0;
     for (; c < c1; ++c) {
-      const double2 y = te_sell_row<REAL, XCG ? 2 : 0>(g.chunk_off, g.col, g.val, u_j, c, lane);
+      const double2 y = te_sell_row<REAL, XCG>(g.chunk_off, g.col, g.val, u_j, c, lane);
       const int64_t r = c * 32 + lane;
       double2 wr = make_double2(0.0, 0.0);
       if (r - row0 < n_i) {

@@ -1,6 +1,8 @@
 // te_common.cu -- error reporting, launch-shape helpers and the buffer cache
 // of libtegpu.
+#include <algorithm>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 
 #include <map>
@@ -117,6 +119,9 @@ namespace {
 constexpr size_t kCacheMinBytes = (size_t)1 << 20;
 constexpr size_t kHostCacheMaxBlock = (size_t)1 << 20;  // pinned blocks up to this size are cached
 
+constexpr int kScratchDevices = 64;
+constexpr size_t kScratchKeep = (size_t)128 << 20;
+
 struct BufferCache {
   std::mutex mu;
   // key (device, bytes); host blocks use device -1
@@ -124,6 +129,8 @@ struct BufferCache {
   std::unordered_map<void*, std::pair<int, size_t>> live;
   size_t cached_dev = 0, cached_host = 0;
   size_t limit_dev = (size_t)8 << 30, limit_host = (size_t)64 << 20;
+  cudaMemPool_t scratch[kScratchDevices] = {};  // per device, see te_scratch_malloc
+  uint64_t scratch_limit() const { return std::min(limit_dev, kScratchKeep); }
 };
 
 BufferCache& cache() {
@@ -136,6 +143,8 @@ BufferCache& cache() {
 void release_locked(BufferCache& c, int device) {
   int cur = 0;
   cudaGetDevice(&cur);
+  for (int d = 0; d < kScratchDevices; ++d)
+    if (c.scratch[d] && (device == -2 || d == device)) cudaMemPoolTrimTo(c.scratch[d], 0);
   for (auto it = c.free_blocks.begin(); it != c.free_blocks.end();) {
     const int d = it->first.first;
     if (device == -2 || d == device) {
@@ -200,6 +209,41 @@ cudaError_t te_free(void* p) {
   return cudaSuccess;
 }
 
+// Scratch of one call, ordered with the call's stream, from a pool of the
+// library's own: the device's default pool gives its memory back at every wait
+// for the GPU, so a caller that waits for each call paid ~170 us to map it
+// again.  The pool keeps at most 128 MB (less under a lower cache limit) and
+// is emptied with the buffer cache.  It is opened with the first matrix on a
+// device, so that no call under stream capture creates it; without it the
+// default pool serves.
+void te_scratch_open() {
+  int dev = 0;
+  BufferCache& c = cache();
+  std::lock_guard<std::mutex> lock(c.mu);
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kScratchDevices || c.scratch[dev]) return;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  uint64_t keep = c.scratch_limit();
+  if (cudaMemPoolCreate(&c.scratch[dev], &props) == cudaSuccess)
+    cudaMemPoolSetAttribute(c.scratch[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+  else
+    c.scratch[dev] = nullptr, cudaGetLastError();
+}
+
+cudaError_t te_scratch_malloc(void** p, size_t bytes, cudaStream_t st) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  cudaMemPool_t pool = nullptr;
+  if (dev < kScratchDevices) {
+    BufferCache& c = cache();
+    std::lock_guard<std::mutex> lock(c.mu);
+    pool = c.scratch[dev];
+  }
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
+}
+
 cudaError_t te_malloc_host_bytes(void** p, size_t bytes) {
   if (bytes > kHostCacheMaxBlock) return cudaMallocHost(p, bytes);
   BufferCache& c = cache();
@@ -248,6 +292,12 @@ extern "C" int te_set_buffer_cache_limit(int64_t device_bytes) {
   BufferCache& c = cache();
   std::lock_guard<std::mutex> lock(c.mu);
   c.limit_dev = (size_t)device_bytes;
+  for (cudaMemPool_t pool : c.scratch)
+    if (pool) {
+      uint64_t keep = c.scratch_limit();
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      cudaMemPoolTrimTo(pool, keep);
+    }
   if (c.cached_dev > c.limit_dev) {
     for (auto it = c.free_blocks.begin(); it != c.free_blocks.end();) {  // devices only
       if (it->first.first >= 0) {

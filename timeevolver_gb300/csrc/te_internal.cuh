@@ -136,6 +136,7 @@ struct TeSell {
   bool saturated = false;  // the grid is capped at every SM's resident blocks
   int warp_chunks = 0;     // most chunks of one warp of the schedule
   int64_t block_slots = 0; // most slots of one block of the schedule
+  int64_t longest = 0;     // slots per row of the longest chunk
   // lanes per row of the SpMV passes (1, 2 or 4), chosen by te_tune_sell_lanes
   // or set through te_matrix_set_spmv_lanes; lanes_fixed once chosen
   int lanes = 1;
@@ -307,6 +308,9 @@ int te_cuda_check(cudaError_t e, const char* what);
 // te_malloc_host / te_free_host cudaMallocHost / cudaFreeHost.
 cudaError_t te_malloc_bytes(void** p, size_t bytes);
 cudaError_t te_free(void* p);
+// stream-ordered scratch of one call (freed with cudaFreeAsync)
+void te_scratch_open();
+cudaError_t te_scratch_malloc(void** p, size_t bytes, cudaStream_t st);
 cudaError_t te_malloc_host_bytes(void** p, size_t bytes);
 cudaError_t te_free_host(void* p);
 template <class T>
@@ -341,8 +345,6 @@ int te_sell_blocks_per_sm(bool is_real);
 
 // ---------------------------------------------------------------- launches
 // te_matrix.cu
-void te_launch_sell_spmv(const TeSell& A, bool is_real, double2 alpha, const double2* x_perm, double2* y_perm,
-                         cudaStream_t st, const TeSegCarry* carry = nullptr);
 void te_launch_csr_spmv(const te_matrix_s& A, double2 alpha, const double2* x, double2* y, cudaStream_t st);
 void te_launch_permute(int64_t n, const int32_t* idx, const double2* in, double2* out, cudaStream_t st);
 void te_launch_permute_real(int64_t n, const int32_t* idx, const double* in, double* out, cudaStream_t st);

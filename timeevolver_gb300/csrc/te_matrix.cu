@@ -22,6 +22,7 @@
 #include <mutex>
 #include <numeric>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "te_internal.cuh"
@@ -30,16 +31,96 @@
 
 // ---------------------------------------------------------------- kernels
 
-// K lanes per row as in lanczos_apply_kernel: K = 1 follows the static chunk
-// schedule, K = 2, 4 stride over (chunk, part) units.
-template <bool REAL, int K>
+// te_sell_row with the next loads under way: entries go in groups of U, and
+// while group g's elements of x are on their way so are the addresses of group
+// g + 1 and the columns of group g + 2.  A group then costs one trip to the L2
+// (~1000 cycles) where te_sell_row's four entries cost three in a row (column,
+// permutation, x).  The same sums in the same order.  Past the end the loads
+// repeat the current group (its values are not used); the entries that are
+// left over run guarded, every branch the same in the whole warp.
+template <bool REAL, int U, typename X>
+__device__ __forceinline__ double2 te_sell_row_ahead(const int64_t* __restrict__ chunk_off,
+                                                     const int32_t* __restrict__ col, const double* __restrict__ val,
+                                                     const X& x, int64_t chunk, int lane) {
+  const double2* __restrict__ v2 = reinterpret_cast<const double2*>(val);
+  const int64_t e = __ldg(chunk_off + chunk + 1);
+  int64_t s = __ldg(chunk_off + chunk) + lane;
+  int groups = (int)((e - s + 31) / 32 / U);
+  double re = 0.0, im = 0.0;
+  if (groups > 0) {
+    int32_t at[U], c[U];
+    const int64_t second = groups > 1 ? 32 * U : 0;
+#pragma unroll
+    for (int k = 0; k < U; ++k) at[k] = __ldcs(col + s + 32 * k);
+#pragma unroll
+    for (int k = 0; k < U; ++k) c[k] = __ldcs(col + s + second + 32 * k);
+#pragma unroll
+    for (int k = 0; k < U; ++k) at[k] = te_place_x(x, at[k]);
+    for (; groups > 0; --groups, s += 32 * U) {
+      double2 a[U], xv[U];
+      int32_t next[U];
+      const int64_t third = groups > 2 ? 64 * U : 0;
+#pragma unroll
+      for (int k = 0; k < U; ++k) xv[k] = te_load_at(x, at[k]);
+#pragma unroll
+      for (int k = 0; k < U; ++k) a[k] = REAL ? make_double2(__ldcs(val + s + 32 * k), 0.0) : __ldcs(v2 + s + 32 * k);
+#pragma unroll
+      for (int k = 0; k < U; ++k) next[k] = te_place_x(x, c[k]);
+#pragma unroll
+      for (int k = 0; k < U; ++k) c[k] = __ldcs(col + s + third + 32 * k);
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        re = fma(a[k].x, xv[k].x, re);
+        if (!REAL) re = fma(-a[k].y, xv[k].y, re);
+        im = fma(a[k].x, xv[k].y, im);
+        if (!REAL) im = fma(a[k].y, xv[k].x, im);
+        at[k] = next[k];
+      }
+    }
+  }
+  double2 a[U - 1], xv[U - 1];
+#pragma unroll
+  for (int k = 0; k < U - 1; ++k)
+    if (s + 32 * k < e) {
+      xv[k] = te_load_x<false>(x, __ldcs(col + s + 32 * k));
+      a[k] = REAL ? make_double2(__ldcs(val + s + 32 * k), 0.0) : __ldcs(v2 + s + 32 * k);
+    }
+#pragma unroll
+  for (int k = 0; k < U - 1; ++k)
+    if (s + 32 * k < e) {
+      re = fma(a[k].x, xv[k].x, re);
+      if (!REAL) re = fma(-a[k].y, xv[k].y, re);
+      im = fma(a[k].x, xv[k].y, im);
+      if (!REAL) im = fma(a[k].y, xv[k].x, im);
+    }
+  return make_double2(re, im);
+}
+
+// y = alpha A x.  FORM: kSorted, x and y in the sorted row order; kScatter, x
+// in the sorted order, y in the caller's; kUnsorted, both in the caller's,
+// read and written through the permutation; kAhead, the same with
+// te_sell_row_ahead (product_form has the rule).  K lanes per row as in
+// lanczos_apply_kernel: K = 1 follows the static chunk schedule, K = 2, 4
+// stride over (chunk, part) units.
+enum { kSorted, kScatter, kUnsorted, kAhead };
+template <bool REAL, int K, int FORM>
 __global__ void __launch_bounds__(TE_THREADS) sell_spmv_kernel(int64_t n, int64_t n_chunks,
                                                                const int32_t* __restrict__ warp_chunk,
                                                                const int64_t* __restrict__ chunk_off,
                                                                const int32_t* __restrict__ col,
                                                                const double* __restrict__ val, TeLongRows L,
-                                                               double2 alpha, const double2* __restrict__ x,
+                                                               const int32_t* __restrict__ perm, double2 alpha,
+                                                               const double2* __restrict__ x_in,
                                                                double2* __restrict__ y) {
+  std::conditional_t<FORM <= kScatter, const double2*, TeUnsorted> x;
+  if constexpr (FORM <= kScatter)
+    x = x_in;
+  else
+    x = TeUnsorted{x_in, perm};
+  const auto put = [&](int64_t r, double2 acc) {
+    y[FORM == kSorted ? r : (int64_t)__ldg(perm + r)] =
+        make_double2(alpha.x * acc.x - alpha.y * acc.y, alpha.x * acc.y + alpha.y * acc.x);
+  };
   const int lane = threadIdx.x & 31;
   const int64_t wid = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (K == 1) {
@@ -47,15 +128,25 @@ __global__ void __launch_bounds__(TE_THREADS) sell_spmv_kernel(int64_t n, int64_
     for (int64_t sg = wid; sg < L.n_seg; sg += warps) {  // long rows by merge-path segments
       int64_t lr;
       double2 acc;
-      if (te_long_segment<REAL>(L, sg, x, lane, &lr, &acc) != 0 && lane == 0)
-        y[lr] = make_double2(alpha.x * acc.x - alpha.y * acc.y, alpha.x * acc.y + alpha.y * acc.x);
+      if (te_long_segment<REAL>(L, sg, x, lane, &lr, &acc) != 0 && lane == 0) put(lr, acc);
     }
     const int64_t c_end = warp_chunk[wid + 1];
     for (int64_t c = warp_chunk[wid]; c < c_end; ++c) {
-      double2 acc = te_sell_row<REAL>(chunk_off, col, val, x, c, lane);
-      int64_t r = c * 32 + lane;
-      if (r < n && r >= L.n)
-        y[r] = make_double2(alpha.x * acc.x - alpha.y * acc.y, alpha.x * acc.y + alpha.y * acc.x);
+      // The row's target is settled before the sum where y is the caller's, after
+      // it where y is sorted: complex values then take 48 and 47 registers.  At the
+      // 40 of the other way round, the loads of fewer entries overlap: 2 M
+      // sorted rows of up to 64 take 8% longer, 1 M unsorted ones of up to 256 13%.
+      if constexpr (FORM == kSorted) {
+        const double2 acc = te_sell_row<REAL>(chunk_off, col, val, x, c, lane);
+        const int64_t r = c * 32 + lane;
+        if (r < n && r >= L.n) put(r, acc);
+      } else {
+        const int64_t r = c * 32 + lane;
+        const bool mine = r < n && r >= L.n;
+        const double2 acc = FORM == kAhead ? te_sell_row_ahead<REAL, 8>(chunk_off, col, val, x, c, lane)
+                                           : te_sell_row<REAL>(chunk_off, col, val, x, c, lane);
+        if (mine) put(r, acc);
+      }
     }
   } else {
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -64,8 +155,7 @@ __global__ void __launch_bounds__(TE_THREADS) sell_spmv_kernel(int64_t n, int64_
       const int part = (int)(u - c * K);
       const double2 acc = te_sell_row_k<REAL, K>(chunk_off, col, val, x, c, part, lane);
       const int64_t r = c * 32 + part * (32 / K) + lane / K;
-      if (lane % K == 0 && r < n)
-        y[r] = make_double2(alpha.x * acc.x - alpha.y * acc.y, alpha.x * acc.y + alpha.y * acc.x);
+      if (lane % K == 0 && r < n) put(r, acc);
     }
   }
 }
@@ -95,21 +185,66 @@ __global__ void permute_real_kernel(int64_t n, const int32_t* __restrict__ idx, 
     out[i] = __ldg(in + __ldg(idx + i));
 }
 
-void te_launch_sell_spmv(const TeSell& A, bool is_real, double2 alpha, const double2* x_perm, double2* y_perm,
-                         cudaStream_t st, const TeSegCarry* carry) {
-  using K = void (*)(int64_t, int64_t, const int32_t*, const int64_t*, const int32_t*, const double*, TeLongRows,
-                     double2, const double2*, double2*);
-  static const K table[2][3] = {{sell_spmv_kernel<false, 1>, sell_spmv_kernel<false, 2>, sell_spmv_kernel<false, 4>},
-                                {sell_spmv_kernel<true, 1>, sell_spmv_kernel<true, 2>, sell_spmv_kernel<true, 4>}};
-  const int li = A.lanes == 4 ? 2 : A.lanes == 2 ? 1 : 0;
-  const K k = table[is_real ? 1 : 0][li];
+using ProductKernel = void (*)(int64_t, int64_t, const int32_t*, const int64_t*, const int32_t*, const double*,
+                               TeLongRows, const int32_t*, double2, const double2*, double2*);
+
+template <int FORM>
+ProductKernel product_kernel(bool is_real, int lanes) {
+  static const ProductKernel table[2][3] = {
+      {sell_spmv_kernel<false, 1, FORM>, sell_spmv_kernel<false, 2, FORM>, sell_spmv_kernel<false, 4, FORM>},
+      {sell_spmv_kernel<true, 1, FORM>, sell_spmv_kernel<true, 2, FORM>, sell_spmv_kernel<true, 4, FORM>}};
+  return table[is_real ? 1 : 0][lanes == 4 ? 2 : lanes == 2 ? 1 : 0];
+}
+
+// How a product reads x and writes y; all forms sum each row in the same order.
+// us per product among others, the copies both ways (kSorted: permute, product,
+// permute) against this rule's choice; ch: a chain's rows, sp: random columns, up
+// to 64 or 256 a row, c complex, r real values:
+//   kUnsorted  one launch, no scratch: 6435 ch 16.6 / 8.2, 184756 ch 20.9 / 12.3,
+//              1 M sp64c 194 / 169, sp256c 337 / 325.
+//   kAhead     where the longest row's chain of loads outlasts the rest, the
+//              slots of all rows shared by the chip: 30000 sp64c 29 / 18.5,
+//              100000 sp200c 79 / 56.  Against kUnsorted it breaks even at 50000
+//              rows of sp64c (50 thousand slots per lane) and at 400000 of
+//              sp256c (500 thousand), hence the square of the longest row;
+//              beyond, its registers cost occupancy (1 M sp64c 252).
+//   kScatter   a real matrix's two FMAs an entry don't hide the permutation's
+//              gathers: 300000 sp256r 99 / 94 (kUnsorted 121), 1.35 M ch 103 /
+//              89 (85: those gathers are local), 600000 sp64r 76 / 69 (98).  Also where x
+//              and y overlap: x is copied before y is written.
+//   kSorted    x, y and the permutation outgrow the L2: 4 M sp64c 737 (kUnsorted
+//              757), sp64r 407 (kScatter 436); 1.9 M sp64c 350 / 310, sp64r
+//              202 / 188.
+constexpr int64_t kProductScatterRows = 1 << 18, kProductSortedRows = 1 << 21;
+int product_form(const te_matrix_s& M, const double2* x, const double2* y) {
+  const TeSell& A = M.sell;
+  const char *x0 = (const char*)x, *y0 = (const char*)y;
+  const size_t bytes = sizeof(double2) * (size_t)A.n;
+  const bool overlap = x0 < y0 + bytes && y0 < x0 + bytes;
+  if (A.n > kProductSortedRows) return kSorted;
+  if (overlap || (M.is_real && A.n > kProductScatterRows)) return kScatter;
+  return A.lanes == 1 && A.longest >= 32 && A.slots / 32 < 7 * A.longest * A.longest ? kAhead : kUnsorted;
+}
+
+// y = alpha A x; xs, ys: n entries of scratch each for the sorted copies, ys
+// for kSorted only, xs for kSorted and kScatter.
+void launch_product(const te_matrix_s& M, int form, double2 alpha, const double2* x, double2* y, double2* xs,
+                    double2* ys, const TeSegCarry* carry, cudaStream_t st) {
+  const TeSell& A = M.sell;
+  const ProductKernel k = form == kSorted      ? product_kernel<kSorted>(M.is_real, A.lanes)
+                          : form == kScatter   ? product_kernel<kScatter>(M.is_real, A.lanes)
+                          : form == kUnsorted  ? product_kernel<kUnsorted>(M.is_real, A.lanes)
+                          : M.is_real          ? sell_spmv_kernel<true, 1, kAhead>
+                                               : sell_spmv_kernel<false, 1, kAhead>;
   int grid = A.grid;
   if (A.lanes > 1) {
     const int64_t cap = (int64_t)te_num_sms() * te_kernel_blocks_per_sm((const void*)k, TE_THREADS, 0);
     grid = (int)std::max<int64_t>(1, std::min<int64_t>((A.n_chunks * A.lanes + 7) / 8, cap));
   }
+  if (form <= kScatter) te_launch_permute(A.n, A.perm, x, xs, st);
   k<<<grid, TE_THREADS, 0, st>>>(A.n, A.n_chunks, A.warp_chunk, A.chunk_off, A.col, A.val, te_long_rows(A, carry),
-                                 alpha, x_perm, y_perm);
+                                 A.perm, alpha, form <= kScatter ? xs : x, form == kSorted ? ys : y);
+  if (form == kSorted) te_launch_permute(A.n, A.iperm, ys, y, st);
 }
 
 void te_launch_csr_spmv(const te_matrix_s& A, double2 alpha, const double2* x, double2* y, cudaStream_t st) {
@@ -635,14 +770,17 @@ int upload(T** dst, const T* src, size_t count) {
 // offsets; uploads warp_chunk.
 int sell_schedule(TeSell& S, const std::vector<int64_t>& off, bool real) {
   const int bps = std::min(te_sell_blocks_per_sm(real),
-                           te_kernel_blocks_per_sm(real ? (const void*)sell_spmv_kernel<true, 1>
-                                                        : (const void*)sell_spmv_kernel<false, 1>,
+                           te_kernel_blocks_per_sm(real ? (const void*)sell_spmv_kernel<true, 1, kSorted>
+                                                        : (const void*)sell_spmv_kernel<false, 1, kSorted>,
                                                    TE_THREADS, 0));
   std::vector<int32_t> wc;
   te_sell_schedule(off, S.n_chunks, bps, real, S.grid, S.saturated, wc);
   constexpr int kWarps = TE_THREADS / 32;
   S.warp_chunks = 0;
   S.block_slots = 0;
+  te_scratch_open();
+  S.longest = 0;
+  for (int64_t c = 0; c < S.n_chunks; ++c) S.longest = std::max(S.longest, (off[c + 1] - off[c]) >> 5);
   for (size_t w = 0; w + 1 < wc.size(); ++w) S.warp_chunks = std::max(S.warp_chunks, (int)(wc[w + 1] - wc[w]));
   for (int b = 0; b < S.grid; ++b)
     S.block_slots = std::max(S.block_slots, off[wc[(b + 1) * kWarps]] - off[wc[b * kWarps]]);
@@ -1521,27 +1659,29 @@ extern "C" int te_matrix_spmv(te_matrix A, double alpha_re, double alpha_im, con
   }
   cudaStream_t st = (cudaStream_t)cuda_stream;
   const int64_t n = A->n_rows;
-  // permute in, SELL product, permute out
-  double2 *xp = nullptr, *yp = nullptr;
+  const double2* x = reinterpret_cast<const double2*>(in_dev);
+  double2* y = reinterpret_cast<double2*>(out_dev);
+  double2 *xs = nullptr, *ys = nullptr;
   TeSegCarry carry;  // this call's carries of the split long rows (calls may overlap)
-  TE_CUDA(cudaMallocAsync(&xp, sizeof(double2) * n, st));
-  int rc = te_cuda_check(cudaMallocAsync(&yp, sizeof(double2) * n, st), "cudaMallocAsync");
+  int rc = TE_OK;
+  const int form = product_form(*A, x, y);
+  if (form <= kScatter) rc = te_cuda_check(te_scratch_malloc((void**)&xs, sizeof(double2) * n, st), "scratch");
+  if (rc == TE_OK && form == kSorted)
+    rc = te_cuda_check(te_scratch_malloc((void**)&ys, sizeof(double2) * n, st), "scratch");
   if (rc == TE_OK && A->sell.n_split > 0) {
-    rc = te_cuda_check(cudaMallocAsync(&carry.part, sizeof(double2) * A->sell.n_seg, st), "cudaMallocAsync");
+    rc = te_cuda_check(te_scratch_malloc((void**)&carry.part, sizeof(double2) * A->sell.n_seg, st), "scratch");
     if (rc == TE_OK)
-      rc = te_cuda_check(cudaMallocAsync(&carry.cnt, sizeof(unsigned int) * A->sell.n_long, st), "cudaMallocAsync");
+      rc = te_cuda_check(te_scratch_malloc((void**)&carry.cnt, sizeof(unsigned int) * A->sell.n_long, st), "scratch");
     if (rc == TE_OK)
       rc = te_cuda_check(cudaMemsetAsync(carry.cnt, 0, sizeof(unsigned int) * A->sell.n_long, st), "memset");
   }
   if (rc == TE_OK) {
-    te_launch_permute(n, A->sell.perm, reinterpret_cast<const double2*>(in_dev), xp, st);
-    te_launch_sell_spmv(A->sell, A->is_real, make_double2(alpha_re, alpha_im), xp, yp, st,
-                        A->sell.n_split > 0 ? &carry : nullptr);
-    te_launch_permute(n, A->sell.iperm, yp, reinterpret_cast<double2*>(out_dev), st);
+    launch_product(*A, form, make_double2(alpha_re, alpha_im), x, y, xs, ys, A->sell.n_split > 0 ? &carry : nullptr,
+                   st);
     rc = te_cuda_check(cudaGetLastError(), "spmv launch");
   }
-  cudaFreeAsync(xp, st);
-  cudaFreeAsync(yp, st);
+  if (xs) cudaFreeAsync(xs, st);
+  if (ys) cudaFreeAsync(ys, st);
   if (carry.part) cudaFreeAsync(carry.part, st);
   if (carry.cnt) cudaFreeAsync(carry.cnt, st);
   return rc;
@@ -1568,19 +1708,19 @@ extern "C" int te_matrix_spmv_host(te_matrix A, double alpha_re, double alpha_im
 
 // ------------------------------------------------- product without allocation
 //
-// te_matrix_spmv needs two vectors of scratch (the input and the output in the
-// matrix's sorted row order) and takes them from cudaMallocAsync on every call.
-// Callers that must not allocate -- code recorded into a CUDA graph by stream
-// capture, real-time loops whose memory is fixed up front, hosts whose device
-// memory budget is preallocated by another framework -- use
+// te_matrix_spmv takes its scratch (vectors in the matrix's sorted row order
+// where product_form wants them, the carries of split long rows) from a pool
+// on every call.  Callers that must not allocate -- code recorded into a CUDA
+// graph by stream capture, real-time loops whose memory is fixed up front,
+// hosts whose device memory budget is preallocated by another framework -- use
 // te_matrix_spmv_noalloc instead, which keeps that scratch in the fixed array
-// below.  The array is part of the library image, so every GPU that loads the
-// library holds it (TE_NOALLOC_MAX_ROWS * 2 * 16 bytes = 8 MiB) until the
-// process exits.
+// below (x only: product_form wants no sorted y up to its rows).  The array is
+// part of the library image, so every GPU that loads the library holds it
+// (TE_NOALLOC_MAX_ROWS * 16 bytes = 4 MiB) until the process exits.
 
 #define TE_NOALLOC_MAX_ROWS (1 << 18)
 
-static __device__ __align__(256) double2 g_noalloc_scratch[2 * TE_NOALLOC_MAX_ROWS];
+static __device__ __align__(256) double2 g_noalloc_scratch[TE_NOALLOC_MAX_ROWS];
 
 #define TE_NOALLOC_MAX_DEVICES 64
 
@@ -1619,15 +1759,12 @@ extern "C" int te_matrix_spmv_noalloc(te_matrix A, double alpha_re, double alpha
                  (long long)n, TE_NOALLOC_MAX_ROWS);
     return TE_ERR_UNSUPPORTED;
   }
-  double2* scratch = nullptr;
-  int rc = noalloc_scratch(&scratch);
+  const double2* x = reinterpret_cast<const double2*>(in_dev);
+  double2* y = reinterpret_cast<double2*>(out_dev);
+  double2* xs = nullptr;  // written in full before it is read: nothing to clear
+  int rc = noalloc_scratch(&xs);
   if (rc != TE_OK) return rc;
-  // both halves are written in full before they are read: nothing to clear
-  double2* xp = scratch;
-  double2* yp = scratch + TE_NOALLOC_MAX_ROWS;
   cudaStream_t st = (cudaStream_t)cuda_stream;
-  te_launch_permute(n, A->sell.perm, reinterpret_cast<const double2*>(in_dev), xp, st);
-  te_launch_sell_spmv(A->sell, A->is_real, make_double2(alpha_re, alpha_im), xp, yp, st);
-  te_launch_permute(n, A->sell.iperm, yp, reinterpret_cast<double2*>(out_dev), st);
+  launch_product(*A, product_form(*A, x, y), make_double2(alpha_re, alpha_im), x, y, xs, nullptr, nullptr, st);
   return te_cuda_check(cudaGetLastError(), "spmv_noalloc launch");
 }

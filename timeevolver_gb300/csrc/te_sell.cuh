@@ -8,22 +8,33 @@
 #pragma once
 #include "te_internal.cuh"
 
-// Loads of x (XCG): 0 through the read-only (non-coherent) cache; 1 ordinary
-// cached loads (ld.global.ca) for x written earlier in the same kernel by
-// other SMs and read after a grid barrier, with no copy of it in this SM's L1
-// from before the write (the persistent Lanczos kernel: each basis vector is
-// written once per launch, then read); 2 L2-only loads (ld.global.cg) for
-// vectors rewritten again and again within one launch (the persistent batched
-// kernel), where this SM's L1 could still hold an earlier copy.
-template <int XCG>
-__device__ __forceinline__ double2 te_load_x(const double2* __restrict__ x, int32_t c) {
-  return XCG == 2 ? __ldcg(x + c) : (XCG == 1 ? __ldca(x + c) : __ldg(x + c));
+// Loads of x.  XCG: false through the read-only (non-coherent) cache; true
+// L2-only loads (ld.global.cg) for vectors rewritten again and again within
+// one launch (the persistent batched kernel), where this SM's L1 could still
+// hold an earlier copy.  x is a vector in the sorted basis, or TeUnsorted: one
+// in the caller's order, read through the permutation.
+struct TeUnsorted {
+  const double2* v;
+  const int32_t* perm;  // sorted index -> the caller's
+};
+template <bool XCG>
+__device__ __forceinline__ double2 te_load_x(const double2* x, int32_t c) {
+  return XCG ? __ldcg(x + c) : __ldg(x + c);
 }
+template <bool XCG>
+__device__ __forceinline__ double2 te_load_x(const TeUnsorted& x, int32_t c) {
+  return __ldg(x.v + __ldg(x.perm + c));
+}
+// The same in two halves, for loops that fetch the place ahead.
+__device__ __forceinline__ int32_t te_place_x(const double2* x, int32_t c) { return c; }
+__device__ __forceinline__ int32_t te_place_x(const TeUnsorted& x, int32_t c) { return __ldg(x.perm + c); }
+__device__ __forceinline__ double2 te_load_at(const double2* x, int32_t place) { return __ldg(x + place); }
+__device__ __forceinline__ double2 te_load_at(const TeUnsorted& x, int32_t place) { return __ldg(x.v + place); }
 
-template <bool REAL, int XCG = 0>
+template <bool REAL, bool XCG = false, typename X>
 __device__ __forceinline__ double2 te_sell_row(const int64_t* __restrict__ chunk_off,
                                                const int32_t* __restrict__ col, const double* __restrict__ val,
-                                               const double2* __restrict__ x, int64_t chunk, int lane) {
+                                               const X& x, int64_t chunk, int lane) {
   const int64_t e = __ldg(chunk_off + chunk + 1);
   int64_t s = __ldg(chunk_off + chunk) + lane;
   double re = 0.0, im = 0.0;
@@ -82,10 +93,10 @@ __device__ __forceinline__ double2 te_sell_row(const int64_t* __restrict__ chunk
 // every lane of the row ends with the same value.  The entries are summed in
 // a different order than te_sell_row (interleaved by K): results differ from
 // the K = 1 kernel by rounding only.
-template <bool REAL, int K>
+template <bool REAL, int K, typename X>
 __device__ __forceinline__ double2 te_sell_row_k(const int64_t* __restrict__ chunk_off,
                                                  const int32_t* __restrict__ col, const double* __restrict__ val,
-                                                 const double2* __restrict__ x, int64_t chunk, int part, int lane) {
+                                                 const X& x, int64_t chunk, int part, int lane) {
   const int64_t off = __ldg(chunk_off + chunk);
   const int64_t len = (__ldg(chunk_off + chunk + 1) - off) >> 5;
   const int rloc = part * (32 / K) + lane / K;
@@ -96,7 +107,7 @@ __device__ __forceinline__ double2 te_sell_row_k(const int64_t* __restrict__ chu
       const int64_t s0 = off + 32 * k + rloc, s1 = s0 + 32 * K;
       const int32_t c0 = __ldcs(col + s0), c1 = __ldcs(col + s1);
       const double a0 = __ldcs(val + s0), a1 = __ldcs(val + s1);
-      const double2 x0 = __ldg(x + c0), x1 = __ldg(x + c1);
+      const double2 x0 = te_load_x<false>(x, c0), x1 = te_load_x<false>(x, c1);
       re = fma(a0, x0.x, re);
       im = fma(a0, x0.y, im);
       re = fma(a1, x1.x, re);
@@ -105,7 +116,7 @@ __device__ __forceinline__ double2 te_sell_row_k(const int64_t* __restrict__ chu
     for (; k < len; k += K) {
       const int64_t s = off + 32 * k + rloc;
       const double a = __ldcs(val + s);
-      const double2 xv = __ldg(x + __ldcs(col + s));
+      const double2 xv = te_load_x<false>(x, __ldcs(col + s));
       re = fma(a, xv.x, re);
       im = fma(a, xv.y, im);
     }
@@ -114,7 +125,7 @@ __device__ __forceinline__ double2 te_sell_row_k(const int64_t* __restrict__ chu
     for (; k < len; k += K) {
       const int64_t s = off + 32 * k + rloc;
       const double2 a = __ldcs(v2 + s);
-      const double2 xv = __ldg(x + __ldcs(col + s));
+      const double2 xv = te_load_x<false>(x, __ldcs(col + s));
       re = fma(a.x, xv.x, re);
       re = fma(-a.y, xv.y, re);
       im = fma(a.x, xv.y, im);
@@ -131,14 +142,13 @@ __device__ __forceinline__ double2 te_sell_row_k(const int64_t* __restrict__ chu
 
 // Entries [b, e) of the long-row CSR times x by a whole warp: lanes stride
 // over the entries, then a warp sum (lane 0's value is the one used).
-template <bool REAL, int XCG = 0>
-__device__ __forceinline__ double2 te_long_range(const TeLongRows& L, int64_t b, int64_t e,
-                                                 const double2* __restrict__ x, int lane) {
+template <bool REAL, typename X>
+__device__ __forceinline__ double2 te_long_range(const TeLongRows& L, int64_t b, int64_t e, const X& x, int lane) {
   double re = 0.0, im = 0.0;
   if (REAL) {
     for (int64_t p = b + lane; p < e; p += 32) {
       const double a = __ldcs(L.val + p);
-      const double2 xv = te_load_x<XCG>(x, __ldcs(L.col + p));
+      const double2 xv = te_load_x<false>(x, __ldcs(L.col + p));
       re = fma(a, xv.x, re);
       im = fma(a, xv.y, im);
     }
@@ -146,7 +156,7 @@ __device__ __forceinline__ double2 te_long_range(const TeLongRows& L, int64_t b,
     const double2* __restrict__ v2 = reinterpret_cast<const double2*>(L.val);
     for (int64_t p = b + lane; p < e; p += 32) {
       const double2 a = __ldcs(v2 + p);
-      const double2 xv = te_load_x<XCG>(x, __ldcs(L.col + p));
+      const double2 xv = te_load_x<false>(x, __ldcs(L.col + p));
       re = fma(a.x, xv.x, re);
       re = fma(-a.y, xv.y, re);
       im = fma(a.x, xv.y, im);
@@ -172,11 +182,11 @@ __device__ __forceinline__ double2 te_long_range(const TeLongRows& L, int64_t b,
 // to run, so a pass that reduces over rows must not fold a split row's terms
 // into that warp's sums: te_split_row_publish / te_split_rows_add move them
 // to a fixed place in the final reduction.
-template <bool REAL, int XCG = 0>
-__device__ __forceinline__ int te_long_segment(const TeLongRows& L, int64_t s, const double2* __restrict__ x,
-                                               int lane, int64_t* row, double2* y) {
+template <bool REAL, typename X>
+__device__ __forceinline__ int te_long_segment(const TeLongRows& L, int64_t s, const X& x, int lane, int64_t* row,
+                                               double2* y) {
   const int32_t i = __ldg(L.seg_row + s);
-  const double2 part = te_long_range<REAL, XCG>(L, __ldg(L.seg_begin + s), __ldg(L.seg_begin + s + 1), x, lane);
+  const double2 part = te_long_range<REAL>(L, __ldg(L.seg_begin + s), __ldg(L.seg_begin + s + 1), x, lane);
   *row = i;
   const int32_t s0 = __ldg(L.row_seg + i), s1 = __ldg(L.row_seg + i + 1);
   if (s1 - s0 == 1) {
