@@ -1414,8 +1414,19 @@ int create_coo_device(int64_t n_rows, int64_t n_cols, int64_t nnz, const uint64_
   return te_matrix_adopt_device_csr(n_rows, n_cols, nnz, d_rp, d_ci, d_v, out, 0.0);
 }
 
-// Below this many entries the host conversion is as fast as the device one.
+// From this many entries the device converts; an unsorted input costs it a
+// scan before the host takes over.
 const int64_t kDeviceCooMinEntries = (int64_t)1 << 18;
+// A smaller input goes there where it is known to be sorted (the host's check
+// stops at the first row out of order) and no gap between its rows is long.
+// us per matrix, host / device: 230229 entries 2700 / 1145 (complex 2895 /
+// 1441), 54482 1471 / 1170, 12803 1213 / 1105, 2981 1106 / 1082, 685 864 / 1078.
+const int64_t kDeviceCooSortedEntries = (int64_t)1 << 14;
+
+bool coo_on_device(int64_t n_rows, int64_t nnz, const uint64_t* row_index) {
+  if (nnz >= kDeviceCooMinEntries) return true;
+  return nnz >= kDeviceCooSortedEntries && n_rows <= nnz && std::is_sorted(row_index, row_index + nnz);
+}
 
 }  // namespace
 
@@ -1429,7 +1440,7 @@ extern "C" int te_matrix_create_coo(int64_t n_rows, int64_t n_cols, int64_t nnz,
     te_set_error("te_matrix_create_coo: sizes must stay below 2^31 (int32 indices)");
     return TE_ERR_UNSUPPORTED;
   }
-  if (nnz < kDeviceCooMinEntries)
+  if (!coo_on_device(n_rows, nnz, row_index))
     return create_coo_host(n_rows, n_cols, nnz, row_index, columns, values, coo_norm1(n_cols, nnz, columns, values),
                            out);
   // the 1-norm on host threads while the device builds the layout, started
