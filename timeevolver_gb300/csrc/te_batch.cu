@@ -33,18 +33,37 @@ __global__ void batch_active_kernel(int64_t n_chunks, const int32_t* __restrict_
                     (int64_t)gridDim.x * blockDim.x);
 }
 
-__global__ void __launch_bounds__(1024) batch_schedule_kernel(BatchGeom g, const TeDevState* states, int n_inst,
-                                                              int n_warps, double w_slot, double* inst_cost,
-                                                              int32_t* warp_begin, int32_t* inst_w0,
-                                                              int32_t* inst_nseg, int32_t* seg_base,
-                                                              int32_t* next_run, int32_t* inst_nwrite) {
-  __shared__ double total;
-  batch_schedule_body(g, states, n_inst, n_warps, w_slot, inst_cost, warp_begin, inst_w0, inst_nseg, seg_base,
-                      next_run, inst_nwrite, &total);
+// The instances' costs; clears the new-start flags, the copies being done.
+__global__ void __launch_bounds__(TE_BATCH_TILE) batch_cost_kernel(BatchGeom g, TeDevState* states, int n_inst,
+                                                                   double w_slot, double* inst_cost) {
+  __shared__ double tile[TE_BATCH_TILE];
+  for (int i = threadIdx.x; i < n_inst; i += blockDim.x) states[i].new_start = 0;
+  batch_cost_body(g, states, n_inst, w_slot, inst_cost, tile);
 }
 
+__global__ void __launch_bounds__(TE_THREADS) batch_boundaries_kernel(BatchGeom g, int n_inst, int n_warps,
+                                                                      double w_slot, const double* inst_cost,
+                                                                      int32_t* warp_begin) {
+  batch_boundaries_body(g, n_inst, n_warps, w_slot, inst_cost, warp_begin,
+                        (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+}
+
+constexpr int kSharedBoundaries = 12 << 10;  // more than a wave of 8 blocks on each of 152 SMs has warps
+__global__ void __launch_bounds__(1024) batch_segments_kernel(BatchGeom g, const TeDevState* states, int n_inst,
+                                                              int n_warps, const int32_t* warp_begin,
+                                                              int32_t* inst_w0, int32_t* inst_nseg,
+                                                              int32_t* seg_base, int32_t* next_run,
+                                                              int32_t* inst_nwrite) {
+  __shared__ int32_t boundaries[kSharedBoundaries];
+  batch_segments_body(g, states, n_inst, n_warps, warp_begin, inst_w0, inst_nseg, seg_base, next_run, inst_nwrite,
+                      n_warps < kSharedBoundaries ? boundaries : nullptr);
+}
+
+// The schedule's wave has 5 blocks per SM (what the complex kernels' registers
+// allow), so the real kernels get the same registers: at 40 they spilled, and
+// 48 chains took 118.9 ms instead of 116.5.
 template <bool REAL, bool HAS_PREV>
-__global__ void __launch_bounds__(TE_THREADS, REAL ? 6 : 5) batch_apply_kernel(BatchGeom g, BatchSched sc,
+__global__ void __launch_bounds__(TE_THREADS, 5) batch_apply_kernel(BatchGeom g, BatchSched sc,
                                                                  const double2* __restrict__ V,
                                                                  double2* __restrict__ w, TeDevState* states,
                                                                  double* seg_partials, int j) {
@@ -64,12 +83,6 @@ __global__ void __launch_bounds__(TE_THREADS) batch_new_start_kernel(BatchGeom g
                                                                      const TeDevState* states) {
   batch_new_start_body<false>(g, V, spare, states, (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5),
                        (int64_t)gridDim.x * (blockDim.x >> 5));
-}
-
-// Clear the new-start flags once the copies are done (one thread per instance).
-__global__ void batch_clear_start_kernel(TeDevState* states, int n_inst) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_inst; i += gridDim.x * blockDim.x)
-    states[i].new_start = 0;
 }
 
 __global__ void __launch_bounds__(TE_THREADS) batch_combine_kernel(BatchGeom g, const double2* __restrict__ V,
@@ -302,14 +315,15 @@ int enqueue_step(te_batch b, bool full_step) {
     batch_active_kernel<<<te_grid_fit((const void*)batch_active_kernel, b->n_chunks, 256), 256, 0, st>>>(
         b->n_chunks, b->d_chunk_inst, b->ds, b->d_active, b->d_active_count);
     batch_new_start_kernel<<<gc, TE_THREADS, 0, st>>>(g, b->V, b->spare, b->ds);
-    batch_clear_start_kernel<<<(b->B + 255) / 256, 256, 0, st>>>(b->ds, b->B);
-    k += 2;
     const BatchSched sc = sched(b);
     const int gl = b->n_warps / (TE_THREADS / 32);
-    batch_schedule_kernel<<<1, 1024, 0, st>>>(g, b->ds, b->B, b->n_warps, b->is_real ? 2.0 : 4.0, b->d_inst_cost,
-                                              b->d_warp_begin, b->d_inst_w0, b->d_inst_nseg, b->d_seg_base,
-                                              b->d_next_run, b->d_inst_nwrite);
-    k += 1;
+    const double w_slot = b->is_real ? 2.0 : 4.0;
+    batch_cost_kernel<<<1, TE_BATCH_TILE, 0, st>>>(g, b->ds, b->B, w_slot, b->d_inst_cost);
+    batch_boundaries_kernel<<<b->n_warps / TE_THREADS + 1, TE_THREADS, 0, st>>>(g, b->B, b->n_warps, w_slot,
+                                                                               b->d_inst_cost, b->d_warp_begin);
+    batch_segments_kernel<<<1, 1024, 0, st>>>(g, b->ds, b->B, b->n_warps, b->d_warp_begin, b->d_inst_w0,
+                                              b->d_inst_nseg, b->d_seg_base, b->d_next_run, b->d_inst_nwrite);
+    k += 5;
     for (int j = 0; j < b->m_max; ++j) {
       if (b->is_real) {
         if (j > 0)
@@ -339,7 +353,7 @@ int enqueue_step(te_batch b, bool full_step) {
 }
 
 int64_t kernels_per_replay(const te_batch_s* b, bool full_step) {
-  return (full_step ? 4 + 2 * (int64_t)b->m_max : 0) + 4;
+  return (full_step ? 5 + 2 * (int64_t)b->m_max : 0) + 4;
 }
 
 int capture(te_batch b, bool full_step, cudaGraphExec_t* exec) {

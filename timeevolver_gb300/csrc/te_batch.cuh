@@ -40,7 +40,7 @@ struct BatchGeom {
   const int* active_count;
 };
 
-// The Lanczos schedule of one global step (batch_schedule_body).
+// The Lanczos schedule of one global step (batch_segments_body).
 struct BatchSched {
   const int32_t* warp_begin;  // W + 1 global chunk indices
   const int32_t* inst_w0;     // first warp covering each instance
@@ -158,30 +158,50 @@ __device__ __forceinline__ int64_t batch_skip_to(const BatchGeom& g, const Batch
   return min(nxt, cend);
 }
 
-// Per-instance costs, warp boundaries by binary search, segment bases (one
-// block; *total is a shared-memory double).
-__device__ __forceinline__ void batch_schedule_body(const BatchGeom& g, const TeDevState* states, int n_inst,
-                                                    int n_warps, double w_slot, double* inst_cost,
-                                                    int32_t* warp_begin, int32_t* inst_w0, int32_t* inst_nseg,
-                                                    int32_t* seg_base, int32_t* next_run, int32_t* inst_nwrite,
-                                                    double* total) {
+// The schedule of a global step, in three passes: the instances' costs and
+// their prefix sums (one block), the warps' boundaries (any number of
+// threads), the instances' segments (one block).  One block alone took 160 us
+// for all of it, its SM's FP64 pipe busy with the ~7300 boundaries and its
+// threads with chains of loads; this takes ~20.  Costs are whole
+// numbers of FP64 instructions, exact as double, so the searches below
+// compare integers.
+
+// inst_cost[i + 1] = cost of instances 0 .. i; tile: TE_BATCH_TILE doubles of
+// shared memory.
+#define TE_BATCH_TILE 1024
+__device__ __forceinline__ void batch_cost_body(const BatchGeom& g, const TeDevState* states, int n_inst,
+                                                double w_slot, double* inst_cost, double* tile) {
   const double w_chunk = 8.0 * 32.0;
-  for (int i = threadIdx.x; i < n_inst; i += blockDim.x) {
-    const TeDevState& d = states[i];
-    const int64_t c0 = g.inst_chunk[i], c1 = g.inst_chunk[i + 1];
-    const bool run = !d.done && !d.fatal;
-    inst_cost[i + 1] =
-        run ? fma(w_slot, (double)(g.chunk_off[c1] - g.chunk_off[c0]), w_chunk * (double)(c1 - c0)) : 0.0;
+  double sum = 0.0;
+  if (threadIdx.x == 0) inst_cost[0] = 0.0;
+  for (int base = 0; base < n_inst; base += TE_BATCH_TILE) {
+    const int count = min(TE_BATCH_TILE, n_inst - base);
+    for (int k = threadIdx.x; k < count; k += blockDim.x) {
+      const TeDevState& d = states[base + k];
+      const int64_t c0 = g.inst_chunk[base + k], c1 = g.inst_chunk[base + k + 1];
+      const bool run = !d.done && !d.fatal;
+      tile[k] = run ? fma(w_slot, (double)(g.chunk_off[c1] - g.chunk_off[c0]), w_chunk * (double)(c1 - c0)) : 0.0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 4
+      for (int k = 0; k < count; ++k) {
+        sum += tile[k];
+        inst_cost[base + k + 1] = sum;
+      }
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {  // exclusive prefix over instances (n_inst is small)
-    inst_cost[0] = 0.0;
-    for (int i = 0; i < n_inst; ++i) inst_cost[i + 1] += inst_cost[i];
-    *total = inst_cost[n_inst];
-  }
-  __syncthreads();
-  const double tot = *total;
-  for (int w = threadIdx.x; w <= n_warps; w += blockDim.x) {
+}
+
+// warp_begin[w] of thread t0 of T: the first chunk at or beyond w's share of
+// the cost.
+__device__ __forceinline__ void batch_boundaries_body(const BatchGeom& g, int n_inst, int n_warps, double w_slot,
+                                                      const double* inst_cost, int32_t* warp_begin, int64_t t0,
+                                                      int64_t T) {
+  const double tot = inst_cost[n_inst];
+  const int64_t slot_cost = (int64_t)w_slot, chunk_cost = 8 * 32;
+  for (int64_t w = t0; w <= n_warps; w += T) {
     int32_t c;
     const double target = tot * (double)w / (double)n_warps;
     if (w == n_warps || !(tot > 0.0)) {
@@ -197,22 +217,44 @@ __device__ __forceinline__ void batch_schedule_body(const BatchGeom& g, const Te
       }
       int k = lo;
       while (k < n_inst - 1 && !(inst_cost[k + 1] > target)) ++k;  // step over empty (finished) instances
-      const double rem = target - inst_cost[k];
-      const int64_t c0 = g.inst_chunk[k], c1 = g.inst_chunk[k + 1];
-      int64_t a = c0, b = c1;  // first chunk whose cost prefix within the instance reaches rem
-      while (a < b) {
-        const int64_t mid = (a + b) >> 1;
-        const double cm = fma(w_slot, (double)(g.chunk_off[mid] - g.chunk_off[c0]), w_chunk * (double)(mid - c0));
-        if (cm < rem)
-          a = mid + 1;
-        else
-          b = mid;
+      const int64_t rem = (int64_t)ceil(target - inst_cost[k]);
+      const int64_t c0 = g.inst_chunk[k], off0 = g.chunk_off[c0];
+      int64_t a = c0, b = g.inst_chunk[k + 1];  // first chunk whose cost prefix within the instance reaches rem
+      while (a < b) {  // seven pivots at a time: their loads overlap
+        const int64_t len = b - a, from = a;
+        int64_t cost[7];
+#pragma unroll
+        for (int q = 0; q < 7; ++q) cost[q] = g.chunk_off[from + len * (q + 1) / 8];
+#pragma unroll
+        for (int q = 6; q >= 0; --q) {  // the first pivot that reaches rem ends the range
+          const int64_t p = from + len * (q + 1) / 8;
+          if (slot_cost * (cost[q] - off0) + chunk_cost * (p - c0) >= rem) b = p;
+        }
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+          const int64_t p = from + len * (q + 1) / 8;
+          if (p < b) a = p + 1;
+        }
       }
       c = (int32_t)a;
     }
     warp_begin[w] = c;
   }
-  __syncthreads();
+}
+
+// The instances' segments from the boundaries (one block of whole warps);
+// shared: a copy of the boundaries, or null where they don't fit.
+__device__ __forceinline__ void batch_segments_body(const BatchGeom& g, const TeDevState* states, int n_inst,
+                                                    int n_warps, const int32_t* warp_begin, int32_t* inst_w0,
+                                                    int32_t* inst_nseg, int32_t* seg_base, int32_t* next_run,
+                                                    int32_t* inst_nwrite, int32_t* shared) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int32_t* begin = warp_begin;
+  if (shared) {
+    for (int w = threadIdx.x; w <= n_warps; w += blockDim.x) shared[w] = warp_begin[w];
+    begin = shared;
+    __syncthreads();
+  }
   for (int i = threadIdx.x; i < n_inst; i += blockDim.x) {
     const TeDevState& d = states[i];
     const int64_t c0 = g.inst_chunk[i], c1 = g.inst_chunk[i + 1];
@@ -222,7 +264,7 @@ __device__ __forceinline__ void batch_schedule_body(const BatchGeom& g, const Te
         int lo = 0, hi = n_warps;
         while (lo < hi) {
           const int mid = (lo + hi + 1) >> 1;
-          if (warp_begin[mid] <= c)
+          if (begin[mid] <= c)
             lo = mid;
           else
             hi = mid - 1;
@@ -234,22 +276,37 @@ __device__ __forceinline__ void batch_schedule_body(const BatchGeom& g, const Te
     }
     inst_w0[i] = w0;
     inst_nseg[i] = nseg;
-    int nw = 0;
-    for (int s = 0; s < nseg; ++s) nw += warp_begin[w0 + s] < warp_begin[w0 + s + 1];
-    inst_nwrite[i] = nw;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  for (int i = warp; i < n_inst; i += blockDim.x >> 5) {  // segments that are written: non-empty warps
+    const int w0 = inst_w0[i], nseg = inst_nseg[i];
+    int nw = 0;
+    for (int s = lane; s < nseg; s += 32) nw += begin[w0 + s] < begin[w0 + s + 1];
+    nw = __reduce_add_sync(0xffffffffu, nw);
+    if (lane == 0) inst_nwrite[i] = nw;
+  }
+  if (warp == 0) {
     int32_t base = 0;
-    for (int i = 0; i < n_inst; ++i) {
-      seg_base[i] = base;
-      base += inst_nseg[i];
+    for (int b = 0; b < n_inst; b += 32) {
+      const int32_t nseg = b + lane < n_inst ? inst_nseg[b + lane] : 0;
+      int32_t upto = nseg;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int32_t x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += x;
+      }
+      if (b + lane < n_inst) seg_base[b + lane] = base + upto - nseg;
+      base += __shfl_sync(0xffffffffu, upto, 31);
     }
-  } else if (threadIdx.x == 32) {
+  } else if (warp == 1) {
     int32_t nxt = n_inst;  // next running instance after i
-    for (int i = n_inst - 1; i >= 0; --i) {
-      next_run[i] = nxt;
-      if (!states[i].done && !states[i].fatal) nxt = i;
+    for (int b = (n_inst - 1) / 32 * 32; b >= 0; b -= 32) {
+      const int i = b + lane;
+      const bool run = i < n_inst && !states[i].done && !states[i].fatal;
+      const unsigned running = __ballot_sync(0xffffffffu, run);
+      const unsigned after = lane == 31 ? 0u : running & (0xffffffffu << (lane + 1));
+      if (i < n_inst) next_run[i] = after ? b + __ffs(after) - 1 : nxt;
+      if (running) nxt = b + __ffs(running) - 1;
     }
   }
 }
@@ -274,10 +331,19 @@ __device__ __forceinline__ bool batch_segment_done(const BatchSched& sc, int ins
   const int w0 = sc.inst_w0[inst], ns = sc.inst_nseg[inst];
 #pragma unroll
   for (int k = 0; k < NV; ++k) tot[k] = 0.0;
+  // The partials are loaded whether they were written or not, so that the loads
+  // of several rounds overlap: a 92378-row instance has ~700 segments, and its
+  // last warp holds up the pass (48 chains: 125 -> 116.5 ms).  Spelled out for 2,
+  // 4 or 8 rounds, inline or not, it took 118.5 to 130 ms: registers.
   for (int s = lane; s < ns; s += 32) {
-    if (!(sc.warp_begin[w0 + s] < sc.warp_begin[w0 + s + 1])) continue;  // an empty warp wrote nothing
+    double part[NV];
+    const bool wrote = sc.warp_begin[w0 + s] < sc.warp_begin[w0 + s + 1];  // an empty warp wrote nothing
 #pragma unroll
-    for (int k = 0; k < NV; ++k) tot[k] += __ldcg(seg_partials + NV * (s0 + s) + k);
+    for (int k = 0; k < NV; ++k) part[k] = __ldcg(seg_partials + NV * (s0 + s) + k);
+    if (wrote) {
+#pragma unroll
+      for (int k = 0; k < NV; ++k) tot[k] += part[k];
+    }
   }
 #pragma unroll
   for (int k = 0; k < NV; ++k) {

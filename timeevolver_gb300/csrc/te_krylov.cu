@@ -1193,11 +1193,11 @@ template <bool REAL>
 __global__ void __launch_bounds__(TE_BATCH_PTHREADS, 1) batch_persistent_kernel(TeBatchPersist a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   KSmem* S = reinterpret_cast<KSmem*>(smem_raw);
-  // outside the Krylov phase the start of the shared memory serves the group
-  // reductions and the schedule's total
+  // outside the Krylov phase the shared memory serves the group reductions and
+  // the schedule
+  static_assert(sizeof(KSmem) >= TE_BATCH_TILE * sizeof(double), "the schedule's tile");
   const int ngrp = blockDim.x / TE_THREADS, grp = threadIdx.x / TE_THREADS, gtid = threadIdx.x % TE_THREADS;
   double* gscratch = reinterpret_cast<double*>(smem_raw) + grp * (TE_BATCH_MAX_OBS * 32);
-  double* total = reinterpret_cast<double*>(smem_raw) + ngrp * (TE_BATCH_MAX_OBS * 32);
   auto gsync = [grp]() { asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "r"(TE_THREADS) : "memory"); };
   const int G = gridDim.x;
   auto bar = [&]() { return te_grid_barrier(a.bar_count, a.bar_gen, a.err, a.spin_limit, a.arrivals); };
@@ -1214,8 +1214,15 @@ __global__ void __launch_bounds__(TE_BATCH_PTHREADS, 1) batch_persistent_kernel(
     if (!bar()) return;
     for (int64_t i = tg; i < n_inst; i += TG) a.states[i].new_start = 0;
     if (blockIdx.x == 0)
-      batch_schedule_body(a.g, a.states, n_inst, a.n_warps, a.w_slot, a.inst_cost, a.warp_begin, a.inst_w0,
-                          a.inst_nseg, a.seg_base, a.next_run, a.inst_nwrite, total);
+      batch_cost_body(a.g, a.states, n_inst, a.w_slot, a.inst_cost, reinterpret_cast<double*>(smem_raw));
+    if (!bar()) return;
+    batch_boundaries_body(a.g, n_inst, a.n_warps, a.w_slot, a.inst_cost, a.warp_begin, tg, TG);
+    if (!bar()) return;
+    if (blockIdx.x == 0)
+      batch_segments_body(a.g, a.states, n_inst, a.n_warps, a.warp_begin, a.inst_w0, a.inst_nseg, a.seg_base,
+                          a.next_run, a.inst_nwrite,
+                          (a.n_warps + 1) * sizeof(int32_t) <= sizeof(KSmem) ? reinterpret_cast<int32_t*>(smem_raw)
+                                                                             : nullptr);
     if (!bar()) return;
     for (int j = 0; j < a.m_max; ++j) {
       for (int64_t vw = pw; vw < a.n_warps; vw += PW) {
