@@ -102,10 +102,10 @@ def load_peaks(te):
     return peaks
 
 
-def ncu_traffic(fixed=False):
-    """Per-launch DRAM traffic of the Lanczos apply kernel in use (fixed-point
-    or FP64 SpMV) from the committed ncu summary, if one exists."""
-    p = os.path.join(ROOT, "profiles", "lanczos_apply_fix_bh12.json" if fixed else "lanczos_apply_bh12.json")
+def ncu_traffic(kernel):
+    """Per-launch DRAM traffic of the Lanczos kernel in use from its committed
+    ncu summary, if one exists."""
+    p = os.path.join(ROOT, "profiles", kernel + ".json")
     if os.path.exists(p):
         with open(p) as f:
             return json.load(f).get("dram_bytes_per_launch")
@@ -309,10 +309,17 @@ def run_gb300(args):
     b_format = apply_kernel_bytes(n, nnz, info["real"], fixed, fixed_layout["state"] == 2)
     b_apply = spmv_bytes(n, nnz)
     f_apply = apply_kernel_flops(n, nnz, info["real"], fixed)
+    one_launch = kernel_ms["lanczos_update"][1] == 0  # all iterations of a Krylov step in one launch
+    if one_launch:  # the recurrence's vectors too: u_j, u_{j-1} and w' read, u_{j+1} written
+        b_apply = M_KRYLOV * (b_apply + 64 * n)
+        # stored form: slots, offsets, X_j gathered, u_j and u_{j-1} read, u_{j+1} and X_{j+1} written
+        b_format = M_KRYLOV * (b_format + (2 if fixed else 1) * 16 * n - 16 * n)
+        f_apply = M_KRYLOV * (f_apply + 8 * n)
     avg_apply_s = apply_ms / 1000.0 / max(1, apply_n)
     achieved = b_apply / avg_apply_s / 1e9
-    traffic = ncu_traffic(fixed)
-    iters = kernel_ms["lanczos_update"][1]  # one update pass per Lanczos iteration
+    traffic = ncu_traffic("lanczos_stream_bh12" if one_launch else
+                          "lanczos_apply_fix_bh12" if fixed else "lanczos_apply_bh12")
+    iters = apply_n * M_KRYLOV if one_launch else kernel_ms["lanczos_update"][1]
     vw = steps_per_solve + int(T_FINAL / SAMPLING)  # V.w per step and per sample after t=0
     b_whole = whole_solve_bytes(n, nnz, iters, vw, M_KRYLOV)
     line = {
@@ -329,17 +336,21 @@ def run_gb300(args):
         "e2e": {"value": e2e_s, "unit": "s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "gpu_launches": int(launches),
         "roofline": {"bound": "hbm",
-                     "kernel": ("lanczos_apply_fix_kernel (fixed-point SELL-32 SpMV%s + FP64 recurrence epilogue)"
-                                % (", value dictionary of %d values" % fixed_layout["n_values"]
-                                   if fixed_layout["state"] == 2 else "")
+                     "kernel": ("%s (fixed-point SELL-32 SpMV%s + FP64 recurrence%s)"
+                                % ("lanczos_stream_kernel" if one_launch else "lanczos_apply_fix_kernel",
+                                   ", value dictionary of %d values" % fixed_layout["n_values"]
+                                   if fixed_layout["state"] == 2 else "",
+                                   ", %d iterations per launch" % M_KRYLOV if one_launch else " epilogue")
                                 if fixed else "lanczos_apply_kernel (SELL-32 SpMV + recurrence epilogue)"),
                      "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"],
                      "traffic": traffic, "algorithmic_bytes_per_launch": b_apply,
-                     "algorithmic_bytes": "complex128 CSR SpMV, 20 nnz + 4 (n + 1) + 32 n",
+                     "algorithmic_bytes": "complex128 CSR SpMV, 20 nnz + 4 (n + 1) + 32 n"
+                                          + (", and 64 n of the recurrence, per iteration" if one_launch else ""),
                      "format_bytes_per_launch": b_format,
                      "format_frac": b_format / avg_apply_s / 1e9 / peaks["hbm_gbs"],
                      "avg_launch_us": avg_apply_s * 1e6, "launches": apply_n,
+                     "us_per_iteration": avg_apply_s * 1e6 / (M_KRYLOV if one_launch else 1),
                      "fp64": {"achieved_tflops": f_apply / avg_apply_s / 1e12, "peak_tflops": peaks["fp64_tflops"],
                               "peak_source": "measured (te_probe_fp64_tflops)",
                               "frac": f_apply / avg_apply_s / 1e12 / peaks["fp64_tflops"],

@@ -372,9 +372,11 @@ int te_evolver_krylov_matrix(te_evolver ev, double* diag, double* offdiag, doubl
  * as one persistent cooperative kernel that exchanges its sums between all
  * blocks, instead of two launches per iteration (same step sequence; the sums
  * round differently).  0: never; 1 (default): for every matrix without long
- * rows whose rows fit the kernels' registers (369 664 rows on 152 SMs;
- * measured on GB300, per iteration: 31 against 11.5 us at dim 92378); 2: the
- * same with the FP64 SpMV, whatever TE_OPT_FIXED_SPMV says. */
+ * rows whose rows fit the kernels' registers (369 664 rows on 152 SMs) and,
+ * with the fixed-point SpMV, whose rows stream through them (about 2 million;
+ * measured on GB300, per iteration: 31 against 11.5 us at dim 92378, 85.6
+ * against 61.4 at 1.35 million); 2: the first with the FP64 SpMV, whatever
+ * TE_OPT_FIXED_SPMV says. */
 #define TE_OPT_FUSED_LANCZOS 1
 /* TE_OPT_FIXED_SPMV: the SpMV of the three-term Lanczos passes in integer
  * arithmetic instead of FP64 FMAs (GB300 issues FP64 at 1/58 of its FP32
@@ -386,14 +388,13 @@ int te_evolver_krylov_matrix(te_evolver ev, double* diag, double* offdiag, doubl
  * real H, (5 k 2^-56 + (2 k + 1) 2^-61) R U + 2^-53 |y| for complex H, against
  * FP64's k 2^-53 sum|h||u|.  The recurrence and all reductions stay FP64.
  * Applies to matrices of at least 2048 32-row chunks (smaller ones run the
- * persistent FP64 kernel); see
- * te_matrix_fixed_layout for the forms (value dictionary, column blocks).
- * 0: FP64 SpMV; 1 (default): fixed point. */
+ * one-launch FP64 kernel); see te_matrix_fixed_layout for the forms (value
+ * dictionary, column blocks).  0: FP64 SpMV; 1 (default): fixed point. */
 #define TE_OPT_FIXED_SPMV 2
 /* Options that bound or exercise the failure paths (no counterpart in the
  * reference, which exits or keeps going where these return an error):
  * TE_OPT_BARRIER_SPIN_LIMIT: polls (each a load) before a grid-barrier wait of
- * the persistent Lanczos kernels gives up; the run then
+ * the one-launch Lanczos kernels gives up; the run then
  * returns TE_ERR_DEVICE_TIMEOUT and the evolver can be reset and run again.
  * Default 2^22 (seconds; a co-resident grid arrives in microseconds).
  * TE_OPT_BARRIER_EXTRA_ARRIVALS: 1 makes every barrier of that kernel wait

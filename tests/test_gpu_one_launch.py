@@ -1,5 +1,6 @@
 """The one-launch Lanczos kernels (te_step.cu below 2048 chunks of 32 rows,
-te_resident.cu from there on) against the per-iteration (TE_OPT_FUSED_LANCZOS 0), needs a GB300.
+te_resident.cu from there on) against the per-iteration passes
+(TE_OPT_FUSED_LANCZOS 0); needs a GB300.
 
 Sizes sit at the edges of the kernels' layouts: one row, one chunk, chunks per
 warp 1 / 2 / more than 4 (rows re-read), one and several groups of 32 blocks,

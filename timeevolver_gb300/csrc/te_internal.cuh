@@ -87,8 +87,6 @@ struct TeDevState {
   // 1 / expFactor (0 when expFactor is 0): the folded three-term passes use
   // beta_j^2 / expFactor^2 and alpha_j / expFactor without a division per thread
   double inv_exp_factor;
-  // grid barrier of the persistent Lanczos kernel (arrivals, generation)
-  unsigned int bar_count, bar_gen;
   // fixed-point SpMV (te_fixed.cuh): u_j is encoded as round(u_j 2^fx_xs[j]);
   // fx_umax[j] is the high word of max |u_j| (a bound), fx_wmax the running
   // high word of max |w'| of the current apply pass

@@ -32,7 +32,7 @@ __device__ __forceinline__ bool te_step_inactive(const TeDevState* ds) {
 
 // The recurrence epilogue of one row r (A u_j row sum y): writes w (or the
 // folded w') and accumulates conj(u_j) w.
-template <bool HAS_PREV, bool FOLD, bool CG = false>
+template <bool HAS_PREV, bool FOLD>
 __device__ __forceinline__ double2 apply_row_epilogue(int64_t r, double2 y, double g, double cw,
                                                    const double2* __restrict__ u_j,
                                                    const double2* __restrict__ u_jm1, double2* __restrict__ w,
@@ -40,7 +40,7 @@ __device__ __forceinline__ double2 apply_row_epilogue(int64_t r, double2 y, doub
   double2 wr;
   if (FOLD) {
     if (HAS_PREV) {
-      double2 up = CG ? __ldca(u_jm1 + r) : u_jm1[r];
+      double2 up = u_jm1[r];
       wr.x = fma(cw, up.x, y.y);
       wr.y = fma(cw, up.y, -y.x);
     } else {
@@ -56,7 +56,7 @@ __device__ __forceinline__ double2 apply_row_epilogue(int64_t r, double2 y, doub
     wr.y = -g * y.x;
   }
   w[r] = wr;
-  double2 uj = CG ? __ldca(u_j + r) : u_j[r];
+  double2 uj = u_j[r];
   // conj(u_j) * w
   acc[0] = fma(uj.x, wr.x, fma(uj.y, wr.y, acc[0]));
   acc[1] = fma(uj.x, wr.y, fma(-uj.y, wr.x, acc[1]));
@@ -1022,7 +1022,7 @@ void te_launch_lanczos_apply(const TeSell& A, bool is_real, const double2* u_j, 
 // launch, K = 1 / 2 / 4): L=10 (2 887 chunks, 7 296 resident warps) 24.1 /
 // 22.1 / 26.8 us; L=11 (11 011 chunks) 38 / 41 / 61 us; L=12 97 / 122 / 197
 // us; four lanes never won where this choice applies.  Matrices of fewer than
-// 2048 chunks run their Lanczos iterations in the persistent kernel (K = 1);
+// 2048 chunks run their Lanczos iterations in one launch (te_step.cu, K = 1);
 // matrices with long rows keep K = 1.  te_matrix_set_spmv_lanes overrides.
 //
 // The autotuner proper (te_matrix_set_spmv_lanes(A, -1)): time the
