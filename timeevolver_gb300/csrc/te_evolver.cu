@@ -531,7 +531,7 @@ int run(te_evolver ev, te_result* out) {
     te_set_error("device-side failure %d during the evolution (%s)", S->fatal,
                  S->fatal == TE_ERR_NO_STEP              ? "no small enough time step found to meet the tolerance"
                  : S->fatal == TE_ERR_EIGEN              ? "Krylov eigensolver did not converge"
-                 : S->fatal == TE_ERR_DEVICE_TIMEOUT     ? "a wait of a one-launch Lanczos kernel gave up"
+                 : S->fatal == TE_ERR_DEVICE_TIMEOUT     ? "a grid-barrier wait of the persistent Lanczos kernel gave up"
                                                          : "step search limit");
     return S->fatal;
   }
