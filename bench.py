@@ -310,8 +310,8 @@ def run_gb300(args):
     b_apply = spmv_bytes(n, nnz)
     f_apply = apply_kernel_flops(n, nnz, info["real"], fixed)
     one_launch = kernel_ms["lanczos_update"][1] == 0  # all iterations of a Krylov step in one launch
-    if one_launch:  # the recurrence's vectors too: u_j, u_{j-1} and w' read, u_{j+1} written
-        b_apply = M_KRYLOV * (b_apply + 64 * n)
+    if one_launch:  # the SpMVs' bytes alone over the whole launch, recurrence included
+        b_apply *= M_KRYLOV
         # stored form: slots, offsets, X_j gathered, u_j and u_{j-1} read, u_{j+1} and X_{j+1} written
         b_format = M_KRYLOV * (b_format + (2 if fixed else 1) * 16 * n - 16 * n)
         f_apply = M_KRYLOV * (f_apply + 8 * n)
@@ -346,7 +346,7 @@ def run_gb300(args):
                      "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"],
                      "traffic": traffic, "algorithmic_bytes_per_launch": b_apply,
                      "algorithmic_bytes": "complex128 CSR SpMV, 20 nnz + 4 (n + 1) + 32 n"
-                                          + (", and 64 n of the recurrence, per iteration" if one_launch else ""),
+                                          + (", per iteration" if one_launch else ""),
                      "format_bytes_per_launch": b_format,
                      "format_frac": b_format / avg_apply_s / 1e9 / peaks["hbm_gbs"],
                      "avg_launch_us": avg_apply_s * 1e6, "launches": apply_n,

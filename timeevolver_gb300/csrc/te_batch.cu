@@ -59,11 +59,8 @@ __global__ void __launch_bounds__(1024) batch_segments_kernel(BatchGeom g, const
                       n_warps < kSharedBoundaries ? boundaries : nullptr);
 }
 
-// The schedule's wave has 5 blocks per SM (what the complex kernels' registers
-// allow), so the real kernels get the same registers: at 40 they spilled, and
-// 48 chains took 118.9 ms instead of 116.5.
 template <bool REAL, bool HAS_PREV>
-__global__ void __launch_bounds__(TE_THREADS, 5) batch_apply_kernel(BatchGeom g, BatchSched sc,
+__global__ void __launch_bounds__(TE_THREADS, REAL ? 6 : 5) batch_apply_kernel(BatchGeom g, BatchSched sc,
                                                                  const double2* __restrict__ V,
                                                                  double2* __restrict__ w, TeDevState* states,
                                                                  double* seg_partials, int j) {
@@ -277,19 +274,24 @@ int grid_chunks(const te_batch_s* b) {
   return (int)std::min<int64_t>((b->n_chunks * 32 + TE_THREADS - 1) / TE_THREADS, (int64_t)te_num_sms() * bps);
 }
 
-// Logical warps of the Lanczos schedule: one resident wave of the apply/update
-// kernels.  The graph path launches one hardware warp for each; the persistent
-// kernel's warps loop over them, so both sum the same segments in the same
-// order.
+// Logical warps of the Lanczos schedule: at least 4 chunks each, within 4
+// blocks of the apply and update kernels per SM.  More warps hide more latency but
+// leave more segments for an instance's last warp to sum while the pass waits.
+// ms per run at 1 / 2 / 3 / 4 / 5 blocks per SM (5 are resident): 12 chains (7
+// thousand chunks) 51 / 50 / 50 / 56 / 63, 24 (16) 92 / 72 / 69 / 72 / 75, 48
+// (35) 154 / 106 / 95 / 93 / 98, 96 (74) 292 / 188 / 157 / 147 / 151, 128 (98)
+// 377 / 246 / 209 / 195 / 204; 256 chains (241) take 1% longer at 4 than at 5.
+// The graph path launches one hardware warp for each; the persistent kernel's
+// warps loop over them, so both sum the same segments in the same order.
 int lanczos_warps(const te_batch_s* b) {
   const void* k[] = {(const void*)batch_apply_kernel<true, true>,  (const void*)batch_apply_kernel<true, false>,
                      (const void*)batch_apply_kernel<false, true>, (const void*)batch_apply_kernel<false, false>,
                      (const void*)batch_update_kernel};
-  int bps = 8;
+  int bps = 4;
   for (const void* f : k) bps = std::min(bps, te_kernel_blocks_per_sm(f, TE_THREADS, 0));
-  const int64_t blocks = std::min<int64_t>((b->n_chunks * 32 + TE_THREADS - 1) / TE_THREADS,
-                                           (int64_t)te_num_sms() * bps);
-  return (int)std::max<int64_t>(blocks, 1) * (TE_THREADS / 32);
+  constexpr int kWarps = TE_THREADS / 32, kChunks = 4;
+  const int64_t blocks = std::min<int64_t>(b->n_chunks / (kChunks * kWarps), (int64_t)te_num_sms() * bps);
+  return (int)std::max<int64_t>(blocks, 1) * kWarps;
 }
 
 BatchSched sched(const te_batch_s* b) {

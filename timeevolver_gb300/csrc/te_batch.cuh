@@ -331,19 +331,10 @@ __device__ __forceinline__ bool batch_segment_done(const BatchSched& sc, int ins
   const int w0 = sc.inst_w0[inst], ns = sc.inst_nseg[inst];
 #pragma unroll
   for (int k = 0; k < NV; ++k) tot[k] = 0.0;
-  // The partials are loaded whether they were written or not, so that the loads
-  // of several rounds overlap: a 92378-row instance has ~700 segments, and its
-  // last warp holds up the pass (48 chains: 125 -> 116.5 ms).  Spelled out for 2,
-  // 4 or 8 rounds, inline or not, it took 118.5 to 130 ms: registers.
   for (int s = lane; s < ns; s += 32) {
-    double part[NV];
-    const bool wrote = sc.warp_begin[w0 + s] < sc.warp_begin[w0 + s + 1];  // an empty warp wrote nothing
+    if (!(sc.warp_begin[w0 + s] < sc.warp_begin[w0 + s + 1])) continue;  // an empty warp wrote nothing
 #pragma unroll
-    for (int k = 0; k < NV; ++k) part[k] = __ldcg(seg_partials + NV * (s0 + s) + k);
-    if (wrote) {
-#pragma unroll
-      for (int k = 0; k < NV; ++k) tot[k] += part[k];
-    }
+    for (int k = 0; k < NV; ++k) tot[k] += __ldcg(seg_partials + NV * (s0 + s) + k);
   }
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
