@@ -200,7 +200,7 @@ ProductKernel product_kernel(bool is_real, int lanes) {
 // us per product among others, the copies both ways (kSorted: permute, product,
 // permute) against this rule's choice; ch: a chain's rows, sp: random columns, up
 // to 64 or 256 a row, c complex, r real values:
-//   kUnsorted  one launch, no scratch: 6435 ch 16.6 / 8.2, 184756 ch 20.9 / 12.3,
+//   kUnsorted  one launch, no scratch: 6435 ch 16.6 / 8.2, 92378 ch 20.9 / 12.3,
 //              1 M sp64c 194 / 169, sp256c 337 / 325.
 //   kAhead     where the longest row's chain of loads outlasts the rest, the
 //              slots of all rows shared by the chip: 30000 sp64c 29 / 18.5,
@@ -210,8 +210,8 @@ ProductKernel product_kernel(bool is_real, int lanes) {
 //              beyond, its registers cost occupancy (1 M sp64c 252).
 //   kScatter   a real matrix's two FMAs an entry don't hide the permutation's
 //              gathers: 300000 sp256r 99 / 94 (kUnsorted 121), 1.35 M ch 103 /
-//              89 (85: those gathers are local), 600000 sp64r 76 / 69 (98).  Also where x
-//              and y overlap: x is copied before y is written.
+//              89 (85: those gathers are local), 600000 sp64r 76 / 69 (98).
+//              Also where x and y overlap: x is copied before y is written.
 //   kSorted    x, y and the permutation outgrow the L2: 4 M sp64c 737 (kUnsorted
 //              757), sp64r 407 (kScatter 436); 1.9 M sp64c 350 / 310, sp64r
 //              202 / 188.

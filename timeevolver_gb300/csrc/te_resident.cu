@@ -874,7 +874,10 @@ bool te_launch_lanczos_resident(const TeSell& A, bool is_real, bool fixed, doubl
   a.arrivals = (unsigned int)G + extra_arrivals;
   for (int j = 0; j < TE_MMAX; ++j) a.u[j] = j < m ? cols[j] : nullptr;
   const int fmt = fixed ? (A.fix_val4 ? 2 : (A.fix_pk ? 1 : 0)) : (is_real ? 3 : 4);
-  a.n_workers = stream ? (fmt == 1 ? kStreamWarps<1> : fmt == 2 ? kStreamWarps<2> : kStreamWarps<0>) : (per_block + cpw - 1) / cpw;
+  a.n_workers = !stream    ? (per_block + cpw - 1) / cpw
+                : fmt == 1 ? kStreamWarps<1>
+                : fmt == 2 ? kStreamWarps<2>
+                           : kStreamWarps<0>;
   const ResKernel k = !stream    ? res_kernel(fmt, cpw)
                       : fmt == 2 ? lanczos_stream_kernel<2>
                       : fmt == 1 ? lanczos_stream_kernel<1>
