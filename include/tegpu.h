@@ -373,7 +373,7 @@ int te_evolver_krylov_matrix(te_evolver ev, double* diag, double* offdiag, doubl
  * blocks, instead of two launches per iteration (same step sequence; the sums
  * round differently).  0: never; 1 (default): for every matrix without long
  * rows whose rows fit the kernels' registers (369 664 rows on 152 SMs) and,
- * with the fixed-point SpMV, whose rows stream through them (about 2 million;
+ * with the fixed-point SpMV, whose rows stream through them (about 1.5 million;
  * measured on GB300, per iteration: 31 against 11.5 us at dim 92378, 85.6
  * against 61.4 at 1.35 million), both from 2048 chunks of 32 rows on up to 40
  * Krylov dimensions; 2: the first with the FP64 SpMV, whatever

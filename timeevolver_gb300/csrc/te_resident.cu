@@ -44,7 +44,11 @@ namespace {
 constexpr int kResWarps = 19;     // worker warps per block at most
 constexpr int kResMaxCpw = 4;     // chunks per worker warp at most
 constexpr int kStreamMaxWarps = 31;        // worker warps per block of the streaming kernel at most
-constexpr size_t kStreamSmem = 216 << 10;  // its dynamic shared memory at most
+// Its dynamic shared memory at most.  The L1 has the rest of the SM's 256 KB, and
+// the gathers in flight need it: us per iteration, passes / streamed, random
+// rows of up to 64 and 256 (complex): 1.2 M 167 / 137 and 350 / 253, 1.5 M (158
+// KB) 202 / 189 and 421 / 350, 1.9 M (196 KB) 245 / 517 and 481 / 966.
+constexpr size_t kStreamSmem = 160 << 10;
 // Worker warps and slots in flight per lane by format (0 real limbs, 1 value
 // dictionary, 2 complex limbs): more warps leave fewer registers for slots in
 // flight.  Measured per iteration on GB300, dictionary (Bose-Hubbard L=12): 31
@@ -822,7 +826,7 @@ ResKernel res_kernel(int fmt, int cpw) {
 
 }  // namespace
 
-// w' of a block's rows and the value table fit its shared memory (2.0 million
+// w' of a block's rows and the value table fit its shared memory (1.55 million
 // rows on 152 SMs), fixed-point form built.
 bool te_stream_fits(const TeSell& A) {
   if (A.n_long > 0 || A.fix_nblk > 0 || te_num_sms() > 255 || A.slots >= ((int64_t)1 << 31) - 256) return false;
