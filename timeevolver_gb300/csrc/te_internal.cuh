@@ -405,8 +405,8 @@ bool te_launch_lanczos_step(const TeSell& A, bool is_real, double2* const* cols,
 // (te_launch_fix_start done, X the copies of the basis; u_1.. are then not
 // stored), else the FP64 SpMV.  launch counts the launches on this sync block.
 struct TeResidentSync {
-  unsigned long long words[2][TE_MMAX][32];  // sums, by launch parity and iteration
-  unsigned long long umax[256];              // tagged max|u_0|, one per block
+  unsigned long long words[2][TE_MMAX][32];     // sums, by launch parity and iteration
+  unsigned long long wmax[2][160], umax[2][160];  // tagged max|w'|, max|u_j| of the blocks, by parity of j
 };
 bool te_resident_fits(const TeSell& A);
 // Larger matrices, fixed point: rows streamed, w' in shared memory

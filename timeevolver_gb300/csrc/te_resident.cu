@@ -20,8 +20,14 @@
 //    reader knows from the word itself that its sum is complete, so the sum
 //    is its own barrier: no separate arrival counter, and no FP64 reduction
 //    tree (a warp-wide FP64 instruction costs 64 cycles here);
-//  * maxima (the fixed-point scale, and the units of the sums) travel in the
-//    same line as counts of exponents: a sum can carry them, a maximum could not;
+//  * maxima (the fixed-point scale, as tight as the passes': the scale costs
+//    u_{j+1} a bit per factor of two) go out as one tagged word per block and
+//    are read once a sum is complete, when they have nearly always arrived:
+//    max|w'| while alpha_j / e is formed, max|u_{j+1}| while the others gather.
+//    (Polled together with the sums they took the L2 slices' time, see below;
+//    counted by exponent inside a sum's line, below a bound known beforehand,
+//    they cost ten and more bits where ||H|| is far above what the state
+//    reaches: energies of 1e4 and more in rows that no other row couples to.)
 //  * every scalar of the recurrence is a product of ||u_j||^2 and its
 //    reciprocal: c_w = (beta_j / e)^2 = S_{j-1} ||u_j||^2, alpha_j / e =
 //    S_j <u_j, w'> with S_j = s_j^2 = 1 / ||u_j||^2, so the chain holds no
@@ -29,7 +35,7 @@
 //    while the others gather.
 //
 // Times on GB300, per iteration: Bose-Hubbard L=10 (dim 92 378) 31 us as two
-// passes, 11.5 us here; an exchange takes 2 to 4 thousand cycles, the gathers
+// passes, 11.4 us here; an exchange takes 2 to 4 thousand cycles, the gathers
 // 6 700, the rows' FP64 recurrence 4 100 of an iteration's 23 000.  With the
 // rows' sums of all 152 blocks in tagged words instead (one line per 16
 // blocks) the polls themselves took the L2 slices' time: 16 us.
@@ -43,6 +49,8 @@ namespace {
 
 constexpr int kResWarps = 19;     // worker warps per block at most
 constexpr int kResMaxCpw = 4;     // chunks per worker warp at most
+constexpr int kMaxPerLane = 5;    // blocks whose maximum a lane reads
+constexpr int kResMaxBlocks = 32 * kMaxPerLane;
 constexpr int kStreamMaxWarps = 31;        // worker warps per block of the streaming kernel at most
 // Its dynamic shared memory at most.  The L1 has the rest of the SM's 256 KB, and
 // the gathers in flight need it: us per iteration, passes / streamed, random
@@ -58,24 +66,24 @@ template <int FMT>
 constexpr int kStreamWarps = FMT == 1 ? 31 : FMT == 2 ? 23 : 27;
 template <int FMT>
 constexpr int kStreamSlots = FMT == 2 ? 8 : 6;
-constexpr int kAlphaWords = 10;   // <u_j, w'>: re, im (4 limbs of 24 bits each), 2 words of exponent counts
-constexpr int kNormWords = 7;     // ||u_{j+1}||^2: 5 limbs, 2 words of exponent counts
+constexpr int kLimbs = 5;                // of 24 bits each
+constexpr int kAlphaWords = 2 * kLimbs;  // <u_j, w'>: re, im
+constexpr int kNormWords = kLimbs;       // ||u_{j+1}||^2
+constexpr unsigned int kNonFinite = 0x7ff00000u;  // high word of an infinity, the least of a non-finite value
 constexpr int kCountShift = 48;   // blocks counted in bits 48..63 of a word
 constexpr unsigned long long kTopBias = 1ull << 34;  // per block, keeps a signed top limb's sum positive
 
 // exponent x with |v| < 2^x (from the high word; zero and subnormals give -1022)
 __device__ __forceinline__ int exp_above(unsigned int hiword) { return (int)((hiword >> 20) & 0x7ffu) - 1022; }
 __device__ __forceinline__ int exp_above(double v) { return exp_above(te_fix_hiword(v)); }
-// 2^x, at least the smallest normal number
-__device__ __forceinline__ double pow2(int x) { return __hiloint2double((min(max(x, -1022), 1023) + 1023) << 20, 0); }
 
 struct ResShared {
-  unsigned long long part[kStreamMaxWarps][8];  // per-warp limb sums
+  unsigned long long part[kStreamMaxWarps][kAlphaWords];  // per-warp limb sums
   unsigned int pmax[kStreamMaxWarps];
   double cw, gr, gi;
-  int k1, k2, xs;    // units of the two sums, fixed-point scale of u_{j+1}
-  int ew, eu;        // exponents that the maxima of w' and u_{j+1} are counted from
-  int go, go_start;  // 1 continue, 0 leave (timeout; lucky breakdown)
+  int k1, k2, xs;  // units of the two sums, fixed-point scale of u_{j+1}
+  int go;          // 1 continue, 0 leave (a wait gave up)
+  int go_start;    // 1 continue, 0 lucky breakdown, -1 a wait gave up
   double norm2[TE_MMAX + 1], cws[TE_MMAX + 1];  // ||u_j||^2 and (beta_j / e)^2 of the step
 };
 
@@ -92,29 +100,21 @@ __device__ __forceinline__ void warp_limbs(const int (&limb)[N], unsigned long l
   if (lane < N) out[lane] = (unsigned long long)mine;
 }
 
-__device__ __forceinline__ void limbs4(unsigned long long lo, unsigned long long hi, int* l) {
-  l[0] = (int)(lo & 0xffffffull);
-  l[1] = (int)((lo >> 24) & 0xffffffull);
-  l[2] = (int)(((lo >> 48) | (hi << 16)) & 0xffffffull);
-  l[3] = (int)((long long)hi >> 8);  // signed; the caller's units keep it below 2^23
-}
-
-// Counts of exponents: a maximum below 2^e0 is counted in one of 11 bins (bin
-// b: below 2^(e0 - b), the last one open below), 6 bins of 8 bits in the
-// first word, 5 in the second, whose sixth counts non-finite values.
-__device__ __forceinline__ unsigned long long exp_count(unsigned int hiword, int e0, int word) {
-  if (hiword >= 0x7ff00000u) return word == 1 ? 1ull << 40 : 0ull;
-  const int bin = min(max(e0 - exp_above(hiword), 0), 10);
-  return bin / 6 == word ? 1ull << (8 * (bin % 6)) : 0ull;
-}
-// The exponent of the largest counted value, or INT_MAX for a non-finite one.
-__device__ __forceinline__ int exp_of_counts(unsigned long long w0, unsigned long long w1, int e0) {
-  const unsigned long long mask = (1ull << kCountShift) - 1;
-  w0 &= mask;
-  w1 &= mask;
-  if (w1 >> 40) return 0x7fffffff;
-  if (w0) return e0 - (__ffsll((long long)w0) - 1) / 8;
-  return e0 - 6 - (w1 ? (__ffsll((long long)w1) - 1) / 8 : 4);
+// A warp's sum of the lanes' x in units of 2^-k, as limbs (the top one signed).
+// The caller's units keep a top limb below 2^23; an x beyond (not finite, or a
+// matrix whose norm is beyond the units' range) counts as zero here and as
+// non-finite in mx, so that no limb runs into the count of blocks.
+__device__ __forceinline__ void warp_limbs_signed(double x, int k, unsigned long long* out, unsigned int& mx) {
+  unsigned long long lo = 0ull, hi = 0ull;
+  const unsigned int h = te_fix_hiword(x);
+  if (h < kNonFinite && exp_above(h) + k < 24 * kLimbs)
+    te_fix_encode128(x, k, lo, hi);
+  else
+    mx = kNonFinite;
+  const int limb[kLimbs] = {(int)(lo & 0xffffffull), (int)((lo >> 24) & 0xffffffull),
+                            (int)(((lo >> 48) | (hi << 16)) & 0xffffffull), (int)((hi >> 8) & 0xffffffull),
+                            (int)(hi >> 32)};
+  warp_limbs<kLimbs>(limb, out);
 }
 
 // Sum over limb words (weights 2^24i, the top one biased) as a 128-bit integer.
@@ -165,8 +165,8 @@ struct TeResidentArgs {
   int n_exp;           // 2 n < 2^n_exp
   int4* X;             // fixed point: copies of the basis (m x n)
   TeResidentSync* sync;
-  int parity;          // which half of sync this launch uses
-  unsigned int epoch;  // tags of this launch's maxima
+  int parity;         // which half of sync this launch uses
+  unsigned int tag0;  // tags of this launch's maxima: tag0 + j
   unsigned int spin_limit, arrivals;
   double2* u[TE_MMAX];
 };
@@ -222,19 +222,20 @@ __device__ __forceinline__ double2 res_row(const TeResidentArgs& a, const int2* 
   return make_double2(te_i64_to_double(sr, 62 - shift), te_i64_to_double(si, 62 - shift));
 }
 
-// The spare warp sends this block's words: its warps' limb sums (N - 2 words;
-// the signed top limbs biased) and its maximum's exponent counts.
+// The spare warp sends this block's words: its warps' limb sums (the signed top
+// limbs biased), and its maximum, tagged.
 template <int N>
-__device__ __forceinline__ void res_send(const TeResidentArgs& a, ResShared& S, unsigned long long* words, int e0) {
+__device__ __forceinline__ void res_send(const TeResidentArgs& a, const ResShared& S, unsigned long long* words,
+                                         unsigned long long* maxima, unsigned int tag) {
   const int lane = threadIdx.x & 31, l = lane & 15;
   unsigned long long v = 0;
   unsigned int mx = 0;
   for (int w = 0; w < a.n_workers; ++w) {
-    if (l < N - 2) v += S.part[w][l];
+    if (l < N) v += S.part[w][l];
     mx = max(mx, S.pmax[w]);
   }
-  if (l >= N - 2) v = exp_count(mx, e0, l - (N - 2));
-  if (l == N - 3 || (N == kAlphaWords && l == 3)) v += kTopBias;
+  if (lane == 31) st_relaxed(maxima + blockIdx.x, ((unsigned long long)tag << 32) | mx);
+  if (l % kLimbs == kLimbs - 1) v += kTopBias;
   v += 1ull << kCountShift;
   if (lane < N) red_add(words + lane, v);
 }
@@ -260,75 +261,127 @@ __device__ __forceinline__ bool res_receive(const TeResidentArgs& a, const unsig
   }
 }
 
-// max|u_0| over the grid (FP64 rows, whose start has no encoding pass).
-__device__ __forceinline__ bool res_start_max(const TeResidentArgs& a, const ResShared& S, unsigned int tag,
-                                              unsigned int& gmax, TeDevState* ds) {
+// The blocks' tagged maxima, kMaxPerLane per lane: fetched first, then waited
+// for until every tag has arrived (false: gave up).
+struct ResMaxima {
+  unsigned long long t[kMaxPerLane];
+};
+__device__ __forceinline__ ResMaxima res_fetch(const unsigned long long* maxima) {
+  ResMaxima r;
+#pragma unroll
+  for (int k = 0; k < kMaxPerLane; ++k) {
+    const int b = (threadIdx.x & 31) + 32 * k;
+    r.t[k] = b < (int)gridDim.x ? ld_relaxed(maxima + b) : 0ull;
+  }
+  return r;
+}
+__device__ __forceinline__ bool res_max(const TeResidentArgs& a, const unsigned long long* maxima, unsigned int tag,
+                                        ResMaxima r, unsigned int& hiword, TeDevState* ds) {
   const int lane = threadIdx.x & 31;
-  unsigned int mx = 0;
-  for (int w = 0; w < a.n_workers; ++w) mx = max(mx, S.pmax[w]);
-  if (lane == 0) st_relaxed(a.sync->umax + blockIdx.x, ((unsigned long long)tag << 32) | mx);
   unsigned int spins = 0;
   while (true) {
     bool ok = (unsigned int)gridDim.x == a.arrivals;
     unsigned int m = 0;
-    for (int b = lane; b < (int)gridDim.x; b += 32) {
-      const unsigned long long t = ld_relaxed(a.sync->umax + b);
-      ok = ok && (unsigned int)(t >> 32) == tag;
-      m = max(m, (unsigned int)t);
+#pragma unroll
+    for (int k = 0; k < kMaxPerLane; ++k) {
+      if (lane + 32 * k < (int)gridDim.x) ok = ok && (unsigned int)(r.t[k] >> 32) == tag;
+      m = max(m, (unsigned int)r.t[k]);
     }
     if (__all_sync(0xffffffffu, ok)) {
-      gmax = __reduce_max_sync(0xffffffffu, m);
+      hiword = __reduce_max_sync(0xffffffffu, m);
       return true;
     }
     if (++spins > a.spin_limit) {
       if (lane == 0) atomicExch(&ds->fatal, TE_ERR_DEVICE_TIMEOUT);
       return false;
     }
+    r = res_fetch(maxima);
   }
 }
 
-// Spare warp, from the grid's words of <u_j, w'> and max|w'|: alpha_j / e =
-// S_j <u_j, w'>, the fixed-point scale of u_{j+1} and the units of its norm.
-__device__ __forceinline__ void res_alpha(const TeResidentArgs& a, ResShared& S, unsigned long long word, double Sj,
-                                          int eu, double e, int j, bool leader, int G, TeDevState* ds) {
+// Spare warp, from the grid's words of <u_j, w'> and its maxima: alpha_j / e =
+// S_j <u_j, w'>, the fixed-point scale of u_{j+1} from B = (W + (|Re| + |Im|)
+// (alpha_j / e) U)(1 + 1e-12) (W >= max|w'|, U >= max|u_j|, as in
+// lanczos_update_kernel), and the units of its norm.  False: the wait for the
+// maxima gave up.
+__device__ __forceinline__ bool res_alpha(const TeResidentArgs& a, ResShared& S, unsigned long long word, double Sj,
+                                          unsigned int umax, const unsigned long long* maxima, unsigned int tag,
+                                          double e, int j, bool leader, int G, TeDevState* ds) {
+  const ResMaxima r = res_fetch(maxima);
   // the even lanes join re, the odd lanes im
   const int lane = threadIdx.x & 31, im = lane & 1;
-  unsigned long long t[4], lo, hi;
+  unsigned long long t[kLimbs], lo, hi;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) t[i] = __shfl_sync(0xffffffffu, word, i + 4 * im);
-  const int ew = exp_of_counts(__shfl_sync(0xffffffffu, word, 8), __shfl_sync(0xffffffffu, word, 9), S.ew);
-  limbs_join<4>(t, (unsigned long long)G * kTopBias, lo, hi);
+  for (int i = 0; i < kLimbs; ++i) t[i] = __shfl_sync(0xffffffffu, word, i + kLimbs * im);
+  limbs_join<kLimbs>(t, (unsigned long long)G * kTopBias, lo, hi);
   double g = Sj * te_i128_to_double(lo, hi, -S.k1);
-  if (ew == 0x7fffffff || eu > 1024) g = __longlong_as_double(0x7ff8000000000000ll);
+  unsigned int wmax = 0;
+  if (!res_max(a, maxima, tag, r, wmax, ds)) return false;
   const double go = __shfl_xor_sync(0xffffffffu, g, 1);
-  // |u_{j+1}| < B
-  const double B = fma(fabs(g) + fabs(go), pow2(eu), pow2(ew)) * (1.0 + 1e-12);
-  const int eb = exp_above(B), xs = te_fix_scale(B);
+  const double B = fma(fabs(g) + fabs(go), te_fix_upper(umax), te_fix_upper(wmax)) * (1.0 + 1e-12);
+  const int xs = te_fix_scale(B);
+  // beyond the scale's range (or not finite): no coefficients rather than wrong ones
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  const bool fits = max(wmax, umax) < kNonFinite && B < 1e300;
+  g = fits ? g : nan;
   if (lane == 0) {
     S.gr = g;
-    S.gi = go;
+    S.gi = fits ? go : nan;
     S.xs = xs;
-    S.k2 = a.X ? 2 * xs - 62 : 117 - (2 * eb + a.n_exp);
-    S.eu = eb;
+    S.k2 = a.X ? 2 * xs - 62 : 117 - (2 * exp_above(B) + a.n_exp);
     if (leader) {
-      ds->alpha[j] = make_double2(g * e, go * e);
+      ds->alpha[j] = make_double2(S.gr * e, S.gi * e);
       if (a.X) ds->fx_xs[j + 1] = xs;
     }
   }
   __syncwarp();
+  return true;
 }
 
-// ||u_{j+1}||^2 from the grid's words; returns the exponent above max|u_{j+1}|.
-__device__ __forceinline__ int res_norm(const ResShared& S, unsigned long long word, int G, double& norm2) {
-  unsigned long long t[kNormWords - 2], lo, hi;
+// ||u_{j+1}||^2 from the grid's words.
+__device__ __forceinline__ double res_norm(const ResShared& S, unsigned long long word, int G) {
+  unsigned long long t[kLimbs], lo, hi;
 #pragma unroll
-  for (int i = 0; i < kNormWords - 2; ++i) t[i] = __shfl_sync(0xffffffffu, word, i);
-  const int en = exp_of_counts(__shfl_sync(0xffffffffu, word, kNormWords - 2),
-                               __shfl_sync(0xffffffffu, word, kNormWords - 1), S.eu);
-  limbs_join<kNormWords - 2>(t, (unsigned long long)G * kTopBias, lo, hi);
-  norm2 = te_u128_to_double(hi, lo, -S.k2);
-  if (en == 0x7fffffff) norm2 = __longlong_as_double(0x7ff8000000000000ll);
-  return en;
+  for (int i = 0; i < kLimbs; ++i) t[i] = __shfl_sync(0xffffffffu, word, i);
+  limbs_join<kLimbs>(t, (unsigned long long)G * kTopBias, lo, hi);
+  return te_u128_to_double(hi, lo, -S.k2);
+}
+
+// Start of iteration j on the spare warp, while the others gather: max|u_j|,
+// then the scalars that the rows and the sum of <u_j, w'> need.  umax: the
+// high word of max|u_j|, known at j = 0 on the fixed-point path.
+__device__ __forceinline__ void res_start(const TeResidentArgs& a, ResShared& S, int j, bool leader, double bd2,
+                                          unsigned int& umax, double& Sj, double& norm2, TeDevState* ds) {
+  const int lane = threadIdx.x & 31;
+  bool ok = true;
+  if (j > 0 || !a.X) {
+    const unsigned long long* maxima = a.sync->umax[j & 1];
+    ok = res_max(a, maxima, a.tag0 + j, res_fetch(maxima), umax, ds);
+    if (umax >= kNonFinite) norm2 = __longlong_as_double(0x7ff8000000000000ll);
+  }
+  const double cw = j > 0 ? Sj * norm2 : 0.0;  // (beta_j / e)^2
+  const bool go = !(cw < bd2) || j == 0;       // else the lucky breakdown (:551-555)
+  if (lane == 0) {
+    S.cw = cw;
+    S.go_start = !ok ? -1 : go ? 1 : 0;
+    // units 2^-k1 of <u_j, w'>: |<u_j, w'>| <= ||u_j||^2 (||H|| + beta_j / e),
+    // 12 bits to spare (||H|| in the 2-norm is below the 1-norm, sqrt(n) of it
+    // for an H that is not Hermitian).  ||u_0|| is only bounded through max|u_0|
+    const int ex = j == 0 ? 2 * exp_above(umax) + a.n_exp : exp_above(norm2);
+    S.k1 = 24 * kLimbs - 14 - ex - max(a.r_exp, j > 0 ? (exp_above(cw) + 2) / 2 : -2000);
+    if (leader && j > 0) {
+      S.norm2[j] = norm2;
+      S.cws[j] = cw;
+    }
+  }
+  if (j > 0) Sj = 1.0 / norm2;
+}
+// The same as a call, for the streaming kernel: inlined, its registers come out
+// of the others' slots in flight there (complex, dim 1 000 003: 225 us an iteration
+// against 214; the resident kernel loses by the call: L=10 11.7 us against 11.4).
+__device__ __noinline__ void res_start_call(const TeResidentArgs& a, ResShared& S, int j, bool leader, double bd2,
+                                            unsigned int& umax, double& Sj, double& norm2, TeDevState* ds) {
+  res_start(a, S, j, leader, bd2, umax, Sj, norm2, ds);
 }
 
 // End of a launch, first block: the step's coefficients beta_j = |e| sqrt((beta_j
@@ -384,28 +437,22 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
     if (!FIX) mx = max(mx, max(te_fix_hiword(u[i].x), te_fix_hiword(u[i].y)));
   }
   // scalars of the spare warp (the same in every block): S_j = s_j^2 and
-  // ||u_j||^2, exponents above max|u_j| and max|u_{j-1}|
+  // ||u_j||^2, the high word of max|u_j|
   double Sj = 1.0, norm2 = 1.0;
-  int eu = 0, eup = -4000;
+  unsigned int umax = FIX ? ds->fx_umax[0] : 0u;
   int xs = FIX ? ds->fx_xs[0] : 0;
   const double bd2 = (ds->tol_rate / e) * (ds->tol_rate / e);
   int last_j = m;
   bool broke = false;
-  if (FIX) {
-    eu = exp_above(ds->fx_umax[0]);
-    __syncthreads();  // the value table
-  } else {
+  if (!FIX) {
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (!spare && lane == 0) S.pmax[warp] = mx;
-    __syncthreads();
-    if (spare) {
-      unsigned int um = 0;
-      const bool ok = res_start_max(a, S, a.epoch, um, ds);
-      eu = exp_above(um);
-      if (lane == 0) S.go = ok ? 1 : 0;
-    }
-    __syncthreads();
-    if (!S.go) return;
+  }
+  __syncthreads();  // the value table, or the maxima of u_0
+  if (!FIX && spare) {
+    mx = 0;
+    for (int w = 0; w < a.n_workers; ++w) mx = max(mx, S.pmax[w]);
+    if (lane == 0) st_relaxed(sy.umax[0] + blockIdx.x, ((unsigned long long)a.tag0 << 32) | mx);
   }
   for (int j = 0; j < m; ++j) {
     unsigned long long* words = sy.words[a.parity][j];
@@ -416,28 +463,11 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
 #pragma unroll
       for (int i = 0; i < CPW; ++i) w[i] = res_row<FMT, CPW == 1 ? 8 : 4>(a, tab, s0[i], s1[i], x, a.sh + xs);
     } else {
-      const double cw = j > 0 ? Sj * norm2 : 0.0;  // (beta_j / e)^2
-      const bool go = !(cw < bd2) || j == 0;       // else the lucky breakdown (:551-555)
-      const int ecw = j > 0 ? exp_above(cw) : -4000;
-      if (lane == 0) {
-        S.cw = cw;
-        S.go_start = go ? 1 : 0;
-        // units 2^-k1 of <u_j, w'>: |<u_j, w'>| <= ||u_j||^2 (||H|| + beta_j / e),
-        // beta_j / e <= ||H|| for the Hermitian H of an evolution; 12 bits to spare.
-        // ||u_0|| is only bounded through max|u_0|
-        const int ex = j == 0 ? 2 * eu + a.n_exp : exp_above(norm2);
-        S.k1 = 82 - ex - max(a.r_exp, (ecw + 2) / 2);
-        // |w'| <= ||H||_inf max|u_j| + c_w max|u_{j-1}|
-        S.ew = max(a.r_exp + eu, ecw + eup) + 1;
-        if (leader && j > 0) {
-          S.norm2[j] = norm2;
-          S.cws[j] = cw;
-        }
-      }
-      if (j > 0) Sj = 1.0 / norm2;
+      res_start(a, S, j, leader, bd2, umax, Sj, norm2, ds);
     }
     __syncthreads();
-    if (!S.go_start) {
+    if (S.go_start < 0) return;
+    if (S.go_start == 0) {
       last_j = j;
       broke = true;
       break;
@@ -462,22 +492,17 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
           mx = max(mx, max(te_fix_hiword(w[i].x), te_fix_hiword(w[i].y)));
         }
       }
-      int limb[8];
-      unsigned long long lo, hi;
-      te_fix_encode128(dr, S.k1, lo, hi);
-      limbs4(lo, hi, limb);
-      te_fix_encode128(di, S.k1, lo, hi);
-      limbs4(lo, hi, limb + 4);
-      warp_limbs<8>(limb, S.part[warp]);
+      warp_limbs_signed(dr, S.k1, S.part[warp], mx);
+      warp_limbs_signed(di, S.k1, S.part[warp] + kLimbs, mx);
       mx = __reduce_max_sync(0xffffffffu, mx);
       if (lane == 0) S.pmax[warp] = mx;
     }
     __syncthreads();
     if (spare) {
-      res_send<kAlphaWords>(a, S, words, S.ew);
-      unsigned long long word;
-      const bool ok = res_receive<kAlphaWords>(a, words, word, ds);
-      if (ok) res_alpha(a, S, word, Sj, eu, e, j, leader, G, ds);
+      unsigned long long *maxima = sy.wmax[j & 1], word;
+      res_send<kAlphaWords>(a, S, words, maxima, a.tag0 + j);
+      const bool ok = res_receive<kAlphaWords>(a, words, word, ds) &&
+                      res_alpha(a, S, word, Sj, umax, maxima, a.tag0 + j, e, j, leader, G, ds);
       if (lane == 0) S.go = ok ? 1 : 0;
     }
     __syncthreads();
@@ -513,14 +538,17 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
           }
         }
       }
-      if (!FIX) te_fix_encode128(nr, S.k2, lo, hi);
-      int limb[kNormWords - 2];
+      if (!FIX) {
+        te_fix_encode128(nr, S.k2, lo, hi);
+        if (te_fix_hiword(nr) >= kNonFinite) mx = kNonFinite;
+      }
+      int limb[kNormWords];
       limb[0] = (int)(lo & 0xffffffull);
       limb[1] = (int)((lo >> 24) & 0xffffffull);
       limb[2] = (int)(((lo >> 48) | (hi << 16)) & 0xffffffull);
       limb[3] = (int)((hi >> 8) & 0xffffffull);
       limb[4] = (int)((hi >> 32) & 0xffffffull);
-      warp_limbs<kNormWords - 2>(limb, S.part[warp]);
+      warp_limbs<kNormWords>(limb, S.part[warp]);
       mx = __reduce_max_sync(0xffffffffu, mx);
       if (lane == 0) S.pmax[warp] = mx;
     }
@@ -528,18 +556,18 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
     const bool last = j + 1 == m;
     if (spare) {
       fence_gpu();  // the rows this block stored, before its sums
-      res_send<kNormWords>(a, S, words + 16, S.eu);
-      unsigned long long word;
+      unsigned long long *maxima = sy.umax[(j + 1) & 1], word;
+      res_send<kNormWords>(a, S, words + 16, maxima, a.tag0 + j + 1);
       bool ok = true;
       if (!last || leader) {
         ok = res_receive<kNormWords>(a, words + 16, word, ds);
         fence_gpu();  // the other blocks' rows, after their sums
+        if (ok) norm2 = res_norm(S, word, G);
       }
-      if (ok && (!last || leader)) {
-        const int en = res_norm(S, word, G, norm2);
-        eup = eu;
-        eu = en;
-        if (last && lane == 0) {
+      if (last && leader && ok) {
+        ok = res_max(a, maxima, a.tag0 + m, res_fetch(maxima), umax, ds);
+        if (umax >= kNonFinite) norm2 = __longlong_as_double(0x7ff8000000000000ll);
+        if (lane == 0) {
           S.cws[m] = Sj * norm2;
           S.norm2[m] = norm2;
         }
@@ -567,7 +595,7 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
 // change nothing (61.4, 59.4 us), nor does a value table per lane (62.1).
 // Measured on GB300 per iteration: Bose-Hubbard L=12 (dim 1 352 078, 113 values)
 // 85.6 us in two passes, 61.4 us here; complex, dim 1 000 003, 49 M entries: 293
-// -> 216 us.  In the L=12 iteration's 124 000 cycles the row sums take 85 000,
+// -> 214 us.  In the L=12 iteration's 124 000 cycles the row sums take 85 000,
 // the update 22 000, the two exchanges with their scalars 16 000.
 template <int FMT, int U>
 __device__ __forceinline__ void stream_slots(const TeResidentArgs& a, const int2* tab, int s, const int4* X,
@@ -630,7 +658,7 @@ __global__ void __launch_bounds__((kStreamWarps<FMT> + 1) * 32, 1)
   const bool spare = warp == W;
   const uint32_t n32 = (uint32_t)a.n;
   double Sj = 1.0, norm2 = 1.0;  // the spare warp's, as in the resident kernel
-  int eu = exp_above(ds->fx_umax[0]), eup = -4000;
+  unsigned int umax = ds->fx_umax[0];
   int xs = ds->fx_xs[0];
   const double bd2 = (ds->tol_rate / e) * (ds->tol_rate / e);
   int last_j = m;
@@ -642,23 +670,7 @@ __global__ void __launch_bounds__((kStreamWarps<FMT> + 1) * 32, 1)
     const double2 *uj = a.u[j], *up = a.u[j > 0 ? j - 1 : 0];
     double dr = 0.0, di = 0.0;
     unsigned int mx = 0;
-    if (spare) {
-      const double cw = j > 0 ? Sj * norm2 : 0.0;  // (beta_j / e)^2
-      const bool go = !(cw < bd2) || j == 0;       // else the lucky breakdown (:551-555)
-      const int ecw = j > 0 ? exp_above(cw) : -4000;
-      if (lane == 0) {
-        S.cw = cw;
-        S.go_start = go ? 1 : 0;
-        const int ex = j == 0 ? 2 * eu + a.n_exp : exp_above(norm2);
-        S.k1 = 82 - ex - max(a.r_exp, (ecw + 2) / 2);
-        S.ew = max(a.r_exp + eu, ecw + eup) + 1;
-        if (leader && j > 0) {
-          S.norm2[j] = norm2;
-          S.cws[j] = cw;
-        }
-      }
-      if (j > 0) Sj = 1.0 / norm2;
-    }
+    if (spare) res_start_call(a, S, j, leader, bd2, umax, Sj, norm2, ds);
     // apply; the first chunk's row sums before the scalars are needed
     bool first = true;
     double cw = 0.0;
@@ -688,7 +700,7 @@ __global__ void __launch_bounds__((kStreamWarps<FMT> + 1) * 32, 1)
         if (first) {  // the spare warp's scalars
           asm volatile("bar.sync 1, %0;" ::"r"((W + 1) * 32) : "memory");
           first = false;
-          if (!S.go_start) break;
+          if (S.go_start != 1) break;
           cw = S.cw;
         }
         if (live) {
@@ -708,28 +720,24 @@ __global__ void __launch_bounds__((kStreamWarps<FMT> + 1) * 32, 1)
       }
     }
     if (first) asm volatile("bar.sync 1, %0;" ::"r"((W + 1) * 32) : "memory");
-    if (!S.go_start) {
+    if (S.go_start < 0) return;
+    if (S.go_start == 0) {
       last_j = j;
       broke = true;
       break;
     }
     if (!spare) {
-      int limb[8];
-      unsigned long long lo, hi;
-      te_fix_encode128(dr, S.k1, lo, hi);
-      limbs4(lo, hi, limb);
-      te_fix_encode128(di, S.k1, lo, hi);
-      limbs4(lo, hi, limb + 4);
-      warp_limbs<8>(limb, S.part[warp]);
+      warp_limbs_signed(dr, S.k1, S.part[warp], mx);
+      warp_limbs_signed(di, S.k1, S.part[warp] + kLimbs, mx);
       mx = __reduce_max_sync(0xffffffffu, mx);
       if (lane == 0) S.pmax[warp] = mx;
     }
     __syncthreads();
     if (spare) {
-      unsigned long long word;
-      res_send<kAlphaWords>(a, S, words, S.ew);
-      const bool ok = res_receive<kAlphaWords>(a, words, word, ds);
-      if (ok) res_alpha(a, S, word, Sj, eu, e, j, leader, G, ds);
+      unsigned long long *maxima = sy.wmax[j & 1], word;
+      res_send<kAlphaWords>(a, S, words, maxima, a.tag0 + j);
+      const bool ok = res_receive<kAlphaWords>(a, words, word, ds) &&
+                      res_alpha(a, S, word, Sj, umax, maxima, a.tag0 + j, e, j, leader, G, ds);
       if (lane == 0) S.go = ok ? 1 : 0;
     }
     __syncthreads();
@@ -762,13 +770,13 @@ __global__ void __launch_bounds__((kStreamWarps<FMT> + 1) * 32, 1)
           hi += lo < sq ? 1ull : 0ull;
         }
       }
-      int limb[kNormWords - 2];
+      int limb[kNormWords];
       limb[0] = (int)(lo & 0xffffffull);
       limb[1] = (int)((lo >> 24) & 0xffffffull);
       limb[2] = (int)(((lo >> 48) | (hi << 16)) & 0xffffffull);
       limb[3] = (int)((hi >> 8) & 0xffffffull);
       limb[4] = (int)((hi >> 32) & 0xffffffull);
-      warp_limbs<kNormWords - 2>(limb, S.part[warp]);
+      warp_limbs<kNormWords>(limb, S.part[warp]);
       mx = __reduce_max_sync(0xffffffffu, mx);
       if (lane == 0) S.pmax[warp] = mx;
     }
@@ -776,18 +784,18 @@ __global__ void __launch_bounds__((kStreamWarps<FMT> + 1) * 32, 1)
     const bool last = j + 1 == m;
     if (spare) {
       fence_gpu();  // the rows this block stored, before its sums
-      res_send<kNormWords>(a, S, words + 16, S.eu);
-      unsigned long long word;
+      unsigned long long *maxima = sy.umax[(j + 1) & 1], word;
+      res_send<kNormWords>(a, S, words + 16, maxima, a.tag0 + j + 1);
       bool ok = true;
       if (!last || leader) {
         ok = res_receive<kNormWords>(a, words + 16, word, ds);
         fence_gpu();  // the other blocks' rows, after their sums
+        if (ok) norm2 = res_norm(S, word, G);
       }
-      if (ok && (!last || leader)) {
-        const int en = res_norm(S, word, G, norm2);
-        eup = eu;
-        eu = en;
-        if (last && lane == 0) {
+      if (last && leader && ok) {
+        ok = res_max(a, maxima, a.tag0 + m, res_fetch(maxima), umax, ds);
+        if (umax >= kNonFinite) norm2 = __longlong_as_double(0x7ff8000000000000ll);
+        if (lane == 0) {
           S.cws[m] = Sj * norm2;
           S.norm2[m] = norm2;
         }
@@ -829,7 +837,7 @@ ResKernel res_kernel(int fmt, int cpw) {
 // w' of a block's rows and the value table fit its shared memory (1.55 million
 // rows on 152 SMs), fixed-point form built.
 bool te_stream_fits(const TeSell& A) {
-  if (A.n_long > 0 || A.fix_nblk > 0 || te_num_sms() > 255 || A.slots >= ((int64_t)1 << 31) - 256) return false;
+  if (A.n_long > 0 || A.fix_nblk > 0 || te_num_sms() > kResMaxBlocks || A.slots >= ((int64_t)1 << 31) - 256) return false;
   const int64_t most = (A.n_chunks + te_num_sms() - 1) / te_num_sms();
   return (size_t)most * 512 + sizeof(int2) * A.fix_nvals <= kStreamSmem;
 }
@@ -837,7 +845,7 @@ bool te_stream_fits(const TeSell& A) {
 // Rows that fit the registers of one block per SM: kResWarps warps of
 // kResMaxCpw chunks (369 664 rows on 152 SMs).
 bool te_resident_fits(const TeSell& A) {
-  if (A.n_long > 0 || A.n < 1 || A.fix_nblk > 0 || te_num_sms() > 255) return false;
+  if (A.n_long > 0 || A.n < 1 || A.fix_nblk > 0 || te_num_sms() > kResMaxBlocks) return false;
   if (A.slots >= ((int64_t)1 << 31) - 256) return false;  // 32-bit slot counters
   return A.n_chunks <= (int64_t)te_num_sms() * kResWarps * kResMaxCpw;
 }
@@ -873,7 +881,7 @@ bool te_launch_lanczos_resident(const TeSell& A, bool is_real, bool fixed, doubl
   a.X = fixed ? X : nullptr;
   a.sync = sync;
   a.parity = (int)(launch & 1u);
-  a.epoch = launch + 1u;
+  a.tag0 = (launch + 1u) * 128u;
   a.spin_limit = spin_limit;
   a.arrivals = (unsigned int)G + extra_arrivals;
   for (int j = 0; j < TE_MMAX; ++j) a.u[j] = j < m ? cols[j] : nullptr;
