@@ -186,3 +186,33 @@ def test_streamed_exchange_timeout(te_gpu):
     exact = scipy.sparse.linalg.expm_multiply(-3j * _scipy(diag, hop), v)
     assert np.linalg.norm(ev.time_evolve()["state"] - exact) < TOL
     ev.close()
+
+
+@pytest.mark.parametrize("scale", [1e20, 1e100, 1e154, 1e200, 1e299])
+@pytest.mark.parametrize("n,fixed", FORMS)
+def test_overflow_is_an_error(te_gpu, n, fixed, scale):
+    """The norms of the unnormalised basis grow with ||H||^m: beyond the range of
+    a double the evolution ends with an error (no step size or no eigenvalues),
+    not with a state."""
+    diag, hop = _tridiagonal(n, n)
+    M, v = _matrix(te_gpu, scale * diag, scale * hop), _random(n, 3)
+    for fused in (1, 0):
+        ev = _evolver(te_gpu, M, v, 1.0, fused, fixed)
+        with pytest.raises(te_gpu.TeError) as e:
+            ev.time_evolve()
+        assert e.value.code in (-5, -6)
+        ev.close()
+
+
+@pytest.mark.parametrize("scale", [1e-6, 1e-5, 1e5])
+@pytest.mark.parametrize("n", [RESIDENT, STREAMED])
+def test_units_of_energy(te_gpu, n, scale):
+    """The same evolution in other units; at 1e-6 the basis's squared norms leave
+    the range of a double after 26 iterations, which ends the step as a lucky
+    breakdown would."""
+    diag, hop = _tridiagonal(n, n)
+    M, v = _matrix(te_gpu, scale * diag, scale * hop), _random(n, 3)
+    exact = scipy.sparse.linalg.expm_multiply(-3j * _scipy(diag, hop), v)
+    for fused in (1, 0):
+        out = _run(te_gpu, M, v, 3.0 / scale, fused, 1, m=40 if scale < 1e-5 else 28)
+        assert np.linalg.norm(out["state"] - exact) < TOL

@@ -100,7 +100,8 @@ __device__ __forceinline__ double te_i64_to_double(int64_t v, int e2) {
 }
 
 // (hi:lo) 2^e2 for an unsigned 128-bit value, rounded to the nearest double
-// (ties to even), integers only; results below the normal range flush to zero.
+// (ties to even), integers only; results below the normal range flush to zero,
+// those beyond it are infinite.
 __device__ __forceinline__ double te_u128_to_double(unsigned long long hi, unsigned long long lo, int e2) {
   if ((hi | lo) == 0ull) return 0.0;
   const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
@@ -124,6 +125,7 @@ __device__ __forceinline__ double te_u128_to_double(unsigned long long hi, unsig
     ++ex;
   }
   if (ex < -1022) return 0.0;
+  if (ex > 1023) return __longlong_as_double(0x7ff0000000000000ll);
   return __longlong_as_double((long long)(((uint64_t)(ex + 1023) << 52) | (mant & 0xfffffffffffffull)));
 }
 

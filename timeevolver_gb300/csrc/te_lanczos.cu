@@ -502,11 +502,13 @@ __global__ void __launch_bounds__(TE_THREADS) lanczos_update_kernel(int64_t n, c
       const double U = te_fix_upper(ds->fx_umax[j]);
       const double B = (W + (fabs(alpha.x * ie) + fabs(alpha.y * ie)) * U) * (1.0 + 1e-12);
       const int x = te_fix_scale(B);
+      // beyond the scale's range (or not finite): no coefficients rather than wrong ones
+      const double one = B < 1e300 ? 1.0 : __longlong_as_double(0x7ff8000000000000ll);
       scratch[0] = alpha.x * ie;
       scratch[1] = alpha.y * ie;
       scratch[2] = (double)x;
       if (blockIdx.x == 0) {
-        ds->alpha[j] = alpha;
+        ds->alpha[j] = make_double2(one * alpha.x, one * alpha.y);
         ds->upd_gr = alpha.x * ie;
         ds->upd_gi = alpha.y * ie;
         ds->fx_xs[j + 1] = x;

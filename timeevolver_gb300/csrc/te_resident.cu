@@ -107,10 +107,10 @@ __device__ __forceinline__ void warp_limbs(const int (&limb)[N], unsigned long l
 __device__ __forceinline__ void warp_limbs_signed(double x, int k, unsigned long long* out, unsigned int& mx) {
   unsigned long long lo = 0ull, hi = 0ull;
   const unsigned int h = te_fix_hiword(x);
-  if (h < kNonFinite && exp_above(h) + k < 24 * kLimbs)
-    te_fix_encode128(x, k, lo, hi);
-  else
+  if (h >= kNonFinite || (h >= 0x100000u && exp_above(h) + k >= 24 * kLimbs))
     mx = kNonFinite;
+  else
+    te_fix_encode128(x, k, lo, hi);  // 0 for a zero and subnormals
   const int limb[kLimbs] = {(int)(lo & 0xffffffull), (int)((lo >> 24) & 0xffffffull),
                             (int)(((lo >> 48) | (hi << 16)) & 0xffffffull), (int)((hi >> 8) & 0xffffffull),
                             (int)(hi >> 32)};
