@@ -216,3 +216,34 @@ def test_units_of_energy(te_gpu, n, scale):
     for fused in (1, 0):
         out = _run(te_gpu, M, v, 3.0 / scale, fused, 1, m=40 if scale < 1e-5 else 28)
         assert np.linalg.norm(out["state"] - exact) < TOL
+
+
+def test_same_route_in_every_run(te_gpu):
+    """What a run finds on the matrix from earlier ones (timed lanes per row, a
+    column-blocked fixed-point form) does not change its route: the same launches
+    and the same state, bit for bit."""
+    n, band = RESIDENT, 64  # rows long enough for several lanes each
+    rng = np.random.default_rng(1)
+    sides = [rng.standard_normal(n - k) / band for k in range(1, band)]
+    A = scipy.sparse.diags_array(sides + sides, offsets=[*range(1, band), *range(-1, -band, -1)], format="csr")
+    v = _random(n, 3)
+
+    def matrix():
+        return te_gpu.Matrix.from_csr(n, A.indptr, A.indices, A.data.astype(np.complex128))
+
+    def run(M, fixed):
+        out = _run(te_gpu, M, v, 3.0, 1, fixed)
+        return out["launches"], out["state"]
+
+    timed = matrix()
+    timed.set_spmv_lanes(-1)
+    runs = [run(timed, fixed) for fixed in (1, 0, 0, 1)]
+    assert timed.spmv_lanes(tune=False) > 1
+    for a, b in ((0, 3), (1, 2)):
+        assert runs[a][0] == runs[b][0] and np.array_equal(runs[a][1], runs[b][1])
+    blocked = matrix()
+    before = run(blocked, 0)
+    blocked.set_fixed_blocks(2)
+    run(blocked, 1)
+    after = run(blocked, 0)
+    assert before[0] == after[0] and np.array_equal(before[1], after[1])

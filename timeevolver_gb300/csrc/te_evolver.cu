@@ -65,7 +65,7 @@ struct te_evolver_s {
   double* partials = nullptr;
   double* results = nullptr;  // n_obs x n_samples
   int max_batch = 1;
-  int fused_lanczos = 1;  // TE_OPT_FUSED_LANCZOS: 0 never, 1 automatic, 2 always
+  int fused_lanczos = 1;  // TE_OPT_FUSED_LANCZOS: 0 passes, 1 automatic, 2 with FP64 rows
   int fixed_spmv = 1;     // TE_OPT_FIXED_SPMV: 0 FP64 SpMV, 1 fixed-point SpMV
   unsigned int barrier_spins = 1u << 22;  // TE_OPT_BARRIER_SPIN_LIMIT (~seconds of polling)
   unsigned int barrier_extra = 0;         // TE_OPT_BARRIER_EXTRA_ARRIVALS
@@ -351,23 +351,14 @@ int run(te_evolver ev, te_result* out) {
   int m = ev->m;
   double err_prev = 0.0, t_prev = 0.0;
   int64_t guard = 0;
-  // fixed-point SpMV in the folded three-term passes (te_fixed.cuh) for
-  // matrices large enough for the per-iteration passes
-  // (its own schedule, one lane per row); otherwise the FP64 passes, whose
-  // lanes per row are tuned once per matrix on first use
-  // all m iterations in one launch: the small matrices' kernel below 2048
-  // chunks, the resident kernel from there on for every matrix that fits,
-  // unless the caller pinned another number of lanes per row.  (per step of
-  // 40 iterations: see te_step.cu, te_resident.cu)
   const TeSell& sell = ev->H->sell;
-  const bool one_launch = ev->fused_lanczos != 0 && ev->p.reorth == 0 && ev->p.exp_factor != 0.0 && sell.n_long == 0 &&
-                          (sell.lanes == 1 || !(sell.lanes_pinned || sell.lanes_timed));
-  const bool small = one_launch && sell.n_chunks < 2048;
-  bool fix = ev->fixed_spmv != 0 && ev->p.reorth == 0 && ev->p.exp_factor != 0.0 && sell.n_chunks >= 2048 &&
-             ev->fused_lanczos != 2;
+  const bool three_term = ev->p.reorth == 0 && ev->p.exp_factor != 0.0;
+  // fixed-point SpMV (te_fixed.cuh) of the three-term iterations, passes or one
+  // launch, from 2048 chunks on; its own schedule, one lane per row
+  bool fix = ev->fixed_spmv != 0 && three_term && sell.n_chunks >= 2048 && ev->fused_lanczos != 2;
   if (fix) {
     // the fixed-point form and its vectors; without memory for them the
-    // evolution runs the FP64 passes instead
+    // evolution runs with FP64 rows instead
     rc = te_sell_build_fixed(ev->H);
     if (rc == TE_OK && !ev->X) rc = te_cuda_check(te_malloc(&ev->X, sizeof(int4) * n * ev->m), "fixed-point basis");
     if (rc == TE_OK && ev->H->sell.fix_nblk > 0 && !ev->fx_acc)
@@ -379,14 +370,22 @@ int run(te_evolver ev, te_result* out) {
       return rc;
     }
   }
+  // the FP64 passes' lanes per row, chosen once per matrix on first use
   if (!fix && (rc = te_tune_sell_lanes(ev->H)) != TE_OK) return rc;
+  // All m iterations in one launch (te_step.cu below 2048 chunks, te_resident.cu
+  // from there on).  The FP64 kernels take one lane per row: a caller's or the
+  // timed choice of another number keeps the passes, in every run alike (hence
+  // after the choice); a caller's choice does so for the fixed-point rows too.
+  const bool one_lane = sell.lanes == 1 || !(sell.lanes_pinned || (sell.lanes_timed && !fix));
+  const bool one_launch = ev->fused_lanczos != 0 && three_term && sell.n_long == 0 && one_lane;
+  const bool small = one_launch && sell.n_chunks < 2048;
   // These round alpha differently from the passes.  Up to 40 iterations a step that
   // stays below 1e-11 of the state's norm and 4e-9 of any component (evolutions
   // of random states at dims 92378 to 1352078); by 45 the extremal Ritz values
   // converge and carry a rounding to 6e-10 of the norm, 3e-7 of one component.
   constexpr int kResidentIterations = 40;
   const bool resident = one_launch && !small && ev->resident && ev->m <= kResidentIterations &&
-                        (te_resident_fits(sell) || (fix && te_stream_fits(sell)));
+                        (te_resident_fits(sell, fix) || (fix && te_stream_fits(sell)));
   if (small && !ev->step_sync) {
     TE_CUDA(te_malloc(&ev->step_sync, sizeof(TeStepSync)));
     TE_CUDA(cudaMemsetAsync(ev->step_sync, 0, sizeof(TeStepSync), st));

@@ -408,7 +408,7 @@ struct TeResidentSync {
   unsigned long long words[2][TE_MMAX][32];     // sums, by launch parity and iteration
   unsigned long long wmax[2][160], umax[2][160];  // tagged max|w'|, max|u_j| of the blocks, by parity of j
 };
-bool te_resident_fits(const TeSell& A);
+bool te_resident_fits(const TeSell& A, bool fixed);
 // Larger matrices, fixed point: rows streamed, w' in shared memory
 // (launched by te_launch_lanczos_resident).
 bool te_stream_fits(const TeSell& A);

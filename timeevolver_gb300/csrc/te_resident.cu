@@ -844,8 +844,8 @@ bool te_stream_fits(const TeSell& A) {
 
 // Rows that fit the registers of one block per SM: kResWarps warps of
 // kResMaxCpw chunks (369 664 rows on 152 SMs).
-bool te_resident_fits(const TeSell& A) {
-  if (A.n_long > 0 || A.n < 1 || A.fix_nblk > 0 || te_num_sms() > kResMaxBlocks) return false;
+bool te_resident_fits(const TeSell& A, bool fixed) {
+  if (A.n_long > 0 || A.n < 1 || (fixed && A.fix_nblk > 0) || te_num_sms() > kResMaxBlocks) return false;
   if (A.slots >= ((int64_t)1 << 31) - 256) return false;  // 32-bit slot counters
   return A.n_chunks <= (int64_t)te_num_sms() * kResWarps * kResMaxCpw;
 }
@@ -853,7 +853,7 @@ bool te_resident_fits(const TeSell& A) {
 bool te_launch_lanczos_resident(const TeSell& A, bool is_real, bool fixed, double norm1, double2* const* cols, int m,
                                 int4* X, TeDevState* ds, TeResidentSync* sync, unsigned int launch, cudaStream_t st,
                                 unsigned int spin_limit, unsigned int extra_arrivals) {
-  const bool stream = !te_resident_fits(A);
+  const bool stream = !te_resident_fits(A, fixed);
   if (m < 1 || m > TE_MMAX || (stream && !(fixed && te_stream_fits(A)))) return false;
   const int G = stream ? te_num_sms() : (int)std::min<int64_t>(te_num_sms(), A.n_chunks);
   const int per_block = (int)((A.n_chunks + G - 1) / G);
