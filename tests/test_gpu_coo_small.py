@@ -1,6 +1,8 @@
 """Matrices from 2^14 entries in row order are laid out on the device; the same
 entries with the rows out of order are converted on the host.  Each row keeps
 its entries' order either way, so products are equal bit for bit."""
+import time
+
 import numpy as np
 import pytest
 
@@ -32,3 +34,27 @@ def test_bad_entries_are_refused(te_gpu):
         bad_row[-1], bad_col[-1] = max(r, row[-1]), c or col[-1]
         with pytest.raises(Exception, match="out of range"):
             te_gpu.Matrix(n, bad_row, bad_col, np.ones(nnz, dtype=np.complex128))
+
+
+@pytest.mark.parametrize("last", [False, True])
+def test_a_long_row_stays_quick(te_gpu, last):
+    """A long row among the sorted ones (an arrow matrix of 260 000 entries: the
+    device would take a thread's time for each of its 86 666, 28 times the host's
+    in all): the creation takes no longer than from rows out of order, which the
+    host converts, but for what the rest of the creation varies (a factor 2)."""
+    nnz = 260_000
+    n = nnz // 3
+    row = np.sort(np.r_[np.full(n, n - 1 if last else 0), np.arange(nnz - n) % n])
+    col = np.arange(nnz) % n
+    val = np.ones(nnz, dtype=np.complex128)
+    moved = np.argsort(-row, kind="stable")
+
+    def best(r, c):
+        times = []
+        for _ in range(6):
+            start = time.perf_counter()
+            te_gpu.Matrix(n, r, c, val).close()
+            times.append(time.perf_counter() - start)
+        return min(times)
+
+    assert best(row, col) <= 2 * best(row[moved], col[moved])

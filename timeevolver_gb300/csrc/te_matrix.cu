@@ -1418,14 +1418,25 @@ int create_coo_device(int64_t n_rows, int64_t n_cols, int64_t nnz, const uint64_
 // scan before the host takes over.
 const int64_t kDeviceCooMinEntries = (int64_t)1 << 18;
 // A smaller input goes there where it is known to be sorted (the host's check
-// stops at the first row out of order) and no gap between its rows is long.
-// us per matrix, host / device: 230229 entries 2700 / 1145 (complex 2895 /
-// 1441), 54482 1471 / 1170, 12803 1213 / 1105, 2981 1106 / 1082, 685 864 / 1078.
+// stops at the first row out of order) and no row is long: one thread reads a
+// row's entries, ~1.3 us each.  us per matrix, host / device: 230229 entries 2700 /
+// 1145 (complex 2895 / 1441), 54482 1471 / 1170, 12803 1213 / 1105, 2981 1106 /
+// 1082, 685 864 / 1078; with a row of 512 / 1024 / 4096 entries among 17000 1120 /
+// 1168, 1160 / 1824, 1217 / 5232, of 1024 / 2048 among 130000 2164 / 2107, 2157 /
+// 3514, of 1024 / 2048 / 4096 among 262000 3622 / 2194, 3620 / 3614, 3565 / 6424;
+// an arrow with a row of 87333 4101 / 118497.  A gap between the rows costs
+// little: 200000 rows of 262000 5476 / 2487, without a gap 5869 / 1714.
 const int64_t kDeviceCooSortedEntries = (int64_t)1 << 14;
 
-bool coo_on_device(int64_t n_rows, int64_t nnz, const uint64_t* row_index) {
+bool coo_on_device(int64_t n_rows, int64_t nnz, const uint64_t* row) {
   if (nnz >= kDeviceCooMinEntries) return true;
-  return nnz >= kDeviceCooSortedEntries && n_rows <= nnz && std::is_sorted(row_index, row_index + nnz);
+  if (nnz < kDeviceCooSortedEntries || n_rows > nnz || !std::is_sorted(row, row + nnz)) return false;
+  // the host is as fast from rows of about this many entries on (up to 128 more
+  // go unnoticed)
+  const int64_t longest = std::max<int64_t>(512, nnz / 128);
+  for (int64_t i = 0; i + longest < nnz; i += 128)
+    if (row[i] == row[i + longest]) return false;
+  return true;
 }
 
 }  // namespace
