@@ -12,7 +12,8 @@ roofline: the Lanczos apply kernel (SELL-32 SpMV with the fused recurrence
 epilogue): the algorithmic bytes of one complex128 CSR SpMV (20 nnz +
 4 (n + 1) + 32 n) over the kernel's event-timed mean duration; the bytes of
 the stored format (4 per entry with the value dictionary) and their fraction
-are given beside it, and `traffic` is the DRAM bytes ncu measured per launch.
+are given beside it, and `traffic` is the DRAM bytes of a launch as measured by
+ncu (for the one-launch kernel a launch of 12 iterations, scaled to 40).
 
 --impl reference: the CPU restatement of the reference algorithm (the oracle,
 OpenMP on all host cores), every step one whole solve of the same workload,

@@ -374,8 +374,8 @@ int te_evolver_krylov_matrix(te_evolver ev, double* diag, double* offdiag, doubl
  * round differently).  0: never; 1 (default): for every matrix without long
  * rows whose rows fit the kernels' registers (369 664 rows on 152 SMs) and,
  * with the fixed-point SpMV, whose rows stream through them (about 1.5 million;
- * measured on GB300, per iteration: 31 against 11.5 us at dim 92378, 85.6
- * against 61.4 at 1.35 million), both from 2048 chunks of 32 rows on up to 40
+ * measured on GB300, per iteration: 31 against 11.3 us at dim 92378, 85.6
+ * against 61.1 at 1.35 million), both from 2048 chunks of 32 rows on up to 40
  * Krylov dimensions; 2: the first with the FP64 SpMV, whatever
  * TE_OPT_FIXED_SPMV says. */
 #define TE_OPT_FUSED_LANCZOS 1

@@ -4,9 +4,10 @@
 // and timeEvolve() (:261-512).  The control flow of the reference's main loop
 // runs on the device (Lanczos coefficients, step-size search, sampling cursor
 // and status counters live in TeDevState); the host only enqueues one Krylov
-// step at a time (2m Lanczos passes, one Krylov-space kernel, one combine
-// pass, one observable pass), reads back a few scalars and decides whether a
-// further sample batch or step is needed.  Observables are evaluated for a
+// step at a time (one Lanczos launch, or 2m passes where the one-launch kernels
+// do not apply, one Krylov-space kernel, one combine pass, one observable pass),
+// reads back a few scalars and decides whether a further sample batch or step is
+// needed.  Observables are evaluated for a
 // whole batch of samples per launch; host callbacks see one sample at a time.
 #include <cfloat>
 #include <cstddef>
@@ -379,10 +380,15 @@ int run(te_evolver ev, te_result* out) {
   const bool one_lane = sell.lanes == 1 || !(sell.lanes_pinned || (sell.lanes_timed && !fix));
   const bool one_launch = ev->fused_lanczos != 0 && three_term && sell.n_long == 0 && one_lane;
   const bool small = one_launch && sell.n_chunks < 2048;
-  // These round alpha differently from the passes.  Up to 40 iterations a step that
-  // stays below 1e-11 of the state's norm and 4e-9 of any component (evolutions
-  // of random states at dims 92378 to 1352078); by 45 the extremal Ritz values
-  // converge and carry a rounding to 6e-10 of the norm, 3e-7 of one component.
+  // te_resident.cu rounds alpha differently from the passes, so the results of the
+  // two lie apart by what the recurrence makes of a rounding; that grows where
+  // Ritz values converge within a step.  Their errors against exact states do not
+  // differ: within 9% of each other for m = 30 .. 64, random, Mott and Fock starts
+  // of Bose-Hubbard chains of dims 92378 to 1352078, U = 1 and 8, tol 1e-8 and
+  // 1e-10.  The limit is there for users who compare runs of the two: up to it they
+  // lie at most 7e-11 of the state's norm apart over t = 3 at tol 1e-8, at m = 48
+  // 1.3e-9 (over longer times, at m = 45, up to 3e-7 of single components), at tol
+  // 1e-10 5e-12 for every m.
   constexpr int kResidentIterations = 40;
   const bool resident = one_launch && !small && ev->resident && ev->m <= kResidentIterations &&
                         (te_resident_fits(sell, fix) || (fix && te_stream_fits(sell)));

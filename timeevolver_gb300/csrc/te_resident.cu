@@ -586,15 +586,15 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
 // chunks in turn (the same ones in every iteration), w' of its rows stays in
 // shared memory, u_j and u_{j-1} are read back. Against the two passes an
 // iteration saves w' through memory, two launches and the serial FP64 start of
-// every block (square root and divisions on the spare warp here).  What bounds
-// it is a warp's own chain per chunk (offsets, words, gathers, rows: 9 000
-// cycles) at 31 warps an SM, then the rows' FP64 recurrence (39% of the pipe's
-// cycles); the slot loop has no predicates (groups of U, then 4, 2, 1) and
+// every block (square root and divisions on the spare warp here).  No unit is
+// full (L1 data pipe 51%, integer multiplies 40%, FP64 39%, issue 36% of their
+// cycles): what bounds it is a warp's own chain per chunk (offsets, words, gathers,
+// products, rows: 9 000 cycles) at 31 warps an SM; the slot loop has no predicates (groups of U, then 4, 2, 1) and
 // 32-bit counters, since predicated groups with the next words fetched ahead
 // doubled the instructions (95 us).  Gathers made coalesced, or all from L1,
 // change nothing (61.4, 59.4 us), nor does a value table per lane (62.1).
 // Measured on GB300 per iteration: Bose-Hubbard L=12 (dim 1 352 078, 113 values)
-// 85.6 us in two passes, 61.4 us here; complex, dim 1 000 003, 49 M entries: 293
+// 85.6 us in two passes, 61.1 us here; complex, dim 1 000 003, 49 M entries: 293
 // -> 214 us.  In the L=12 iteration's 124 000 cycles the row sums take 85 000,
 // the update 22 000, the two exchanges with their scalars 16 000.
 template <int FMT, int U>
