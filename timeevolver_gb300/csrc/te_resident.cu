@@ -51,6 +51,7 @@ constexpr int kResWarps = 19;     // worker warps per block at most
 constexpr int kResMaxCpw = 4;     // chunks per worker warp at most
 constexpr int kMaxPerLane = 5;    // blocks whose maximum a lane reads
 constexpr int kResMaxBlocks = 32 * kMaxPerLane;
+static_assert(sizeof(TeResidentSync::wmax) == 2 * kResMaxBlocks * sizeof(unsigned long long), "a word per block");
 constexpr int kStreamMaxWarps = 31;        // worker warps per block of the streaming kernel at most
 // Its dynamic shared memory at most.  The L1 has the rest of the SM's 256 KB, and
 // the gathers in flight need it: us per iteration, passes / streamed, random
@@ -78,7 +79,7 @@ __device__ __forceinline__ int exp_above(unsigned int hiword) { return (int)((hi
 __device__ __forceinline__ int exp_above(double v) { return exp_above(te_fix_hiword(v)); }
 
 struct ResShared {
-  unsigned long long part[kStreamMaxWarps][kAlphaWords];  // per-warp limb sums
+  int part[kStreamMaxWarps][kAlphaWords];  // per-warp limb sums
   unsigned int pmax[kStreamMaxWarps];
   double cw, gr, gi;
   int k1, k2, xs;  // units of the two sums, fixed-point scale of u_{j+1}
@@ -89,22 +90,22 @@ struct ResShared {
 
 // A warp's sum of limbs (24 bits each); lane l < N keeps limb l.
 template <int N>
-__device__ __forceinline__ void warp_limbs(const int (&limb)[N], unsigned long long* out) {
+__device__ __forceinline__ void warp_limbs(const int (&limb)[N], int* out) {
   const int lane = threadIdx.x & 31;
-  long long mine = 0;
+  int mine = 0;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     const int s = __reduce_add_sync(0xffffffffu, limb[i]);
     if (lane == i) mine = s;
   }
-  if (lane < N) out[lane] = (unsigned long long)mine;
+  if (lane < N) out[lane] = mine;
 }
 
 // A warp's sum of the lanes' x in units of 2^-k, as limbs (the top one signed).
 // The caller's units keep a top limb below 2^23; an x beyond (not finite, or a
 // matrix whose norm is beyond the units' range) counts as zero here and as
 // non-finite in mx, so that no limb runs into the count of blocks.
-__device__ __forceinline__ void warp_limbs_signed(double x, int k, unsigned long long* out, unsigned int& mx) {
+__device__ __forceinline__ void warp_limbs_signed(double x, int k, int* out, unsigned int& mx) {
   unsigned long long lo = 0ull, hi = 0ull;
   const unsigned int h = te_fix_hiword(x);
   if (h >= kNonFinite || (h >= 0x100000u && exp_above(h) + k >= 24 * kLimbs))
@@ -231,7 +232,7 @@ __device__ __forceinline__ void res_send(const TeResidentArgs& a, const ResShare
   unsigned long long v = 0;
   unsigned int mx = 0;
   for (int w = 0; w < a.n_workers; ++w) {
-    if (l < N) v += S.part[w][l];
+    if (l < N) v += (unsigned long long)(long long)S.part[w][l];
     mx = max(mx, S.pmax[w]);
   }
   if (lane == 31) st_relaxed(maxima + blockIdx.x, ((unsigned long long)tag << 32) | mx);
