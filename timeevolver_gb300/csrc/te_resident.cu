@@ -300,15 +300,31 @@ __device__ __forceinline__ bool res_max(const TeResidentArgs& a, const unsigned 
   }
 }
 
+// The same as a call, from the fetch on.
+__device__ __noinline__ bool res_max_call(const TeResidentArgs& a, const unsigned long long* maxima, unsigned int tag,
+                                          unsigned int& hiword, TeDevState* ds) {
+  return res_max(a, maxima, tag, res_fetch(maxima), hiword, ds);
+}
+template <bool CALL>
+__device__ __forceinline__ bool res_grid_max(const TeResidentArgs& a, const unsigned long long* maxima,
+                                             unsigned int tag, unsigned int& hiword, TeDevState* ds) {
+  if constexpr (CALL)
+    return res_max_call(a, maxima, tag, hiword, ds);
+  else
+    return res_max(a, maxima, tag, res_fetch(maxima), hiword, ds);
+}
+
 // Spare warp, from the grid's words of <u_j, w'> and its maxima: alpha_j / e =
 // S_j <u_j, w'>, the fixed-point scale of u_{j+1} from B = (W + (|Re| + |Im|)
 // (alpha_j / e) U)(1 + 1e-12) (W >= max|w'|, U >= max|u_j|, as in
 // lanczos_update_kernel), and the units of its norm.  False: the wait for the
-// maxima gave up.
+// maxima gave up.  EARLY: the maxima are on their way while alpha_j is formed.
+template <bool EARLY, bool CALL>
 __device__ __forceinline__ bool res_alpha(const TeResidentArgs& a, ResShared& S, unsigned long long word, double Sj,
                                           unsigned int umax, const unsigned long long* maxima, unsigned int tag,
                                           double e, int j, bool leader, int G, TeDevState* ds) {
-  const ResMaxima r = res_fetch(maxima);
+  ResMaxima r{};
+  if constexpr (EARLY) r = res_fetch(maxima);
   // the even lanes join re, the odd lanes im
   const int lane = threadIdx.x & 31, im = lane & 1;
   unsigned long long t[kLimbs], lo, hi;
@@ -317,7 +333,7 @@ __device__ __forceinline__ bool res_alpha(const TeResidentArgs& a, ResShared& S,
   limbs_join<kLimbs>(t, (unsigned long long)G * kTopBias, lo, hi);
   double g = Sj * te_i128_to_double(lo, hi, -S.k1);
   unsigned int wmax = 0;
-  if (!res_max(a, maxima, tag, r, wmax, ds)) return false;
+  if (!(EARLY ? res_max(a, maxima, tag, r, wmax, ds) : res_grid_max<CALL>(a, maxima, tag, wmax, ds))) return false;
   const double go = __shfl_xor_sync(0xffffffffu, g, 1);
   const double B = fma(fabs(g) + fabs(go), te_fix_upper(umax), te_fix_upper(wmax)) * (1.0 + 1e-12);
   const int xs = te_fix_scale(B);
@@ -351,13 +367,14 @@ __device__ __forceinline__ double res_norm(const ResShared& S, unsigned long lon
 // Start of iteration j on the spare warp, while the others gather: max|u_j|,
 // then the scalars that the rows and the sum of <u_j, w'> need.  umax: the
 // high word of max|u_j|, known at j = 0 on the fixed-point path.
+template <bool CALL>
 __device__ __forceinline__ void res_start(const TeResidentArgs& a, ResShared& S, int j, bool leader, double bd2,
                                           unsigned int& umax, double& Sj, double& norm2, TeDevState* ds) {
   const int lane = threadIdx.x & 31;
   bool ok = true;
   if (j > 0 || !a.X) {
     const unsigned long long* maxima = a.sync->umax[j & 1];
-    ok = res_max(a, maxima, a.tag0 + j, res_fetch(maxima), umax, ds);
+    ok = res_grid_max<CALL>(a, maxima, a.tag0 + j, umax, ds);
     if (umax >= kNonFinite) norm2 = __longlong_as_double(0x7ff8000000000000ll);
   }
   const double cw = j > 0 ? Sj * norm2 : 0.0;  // (beta_j / e)^2
@@ -377,13 +394,27 @@ __device__ __forceinline__ void res_start(const TeResidentArgs& a, ResShared& S,
   }
   if (j > 0) Sj = 1.0 / norm2;
 }
-// The same as a call, for the streaming kernel: inlined, its registers come out
-// of the others' slots in flight there (complex, dim 1 000 003: 225 us an iteration
-// against 214; the resident kernel loses by the call: L=10 11.7 us against 11.4).
+// The same as a call.
 __device__ __noinline__ void res_start_call(const TeResidentArgs& a, ResShared& S, int j, bool leader, double bd2,
                                             unsigned int& umax, double& Sj, double& norm2, TeDevState* ds) {
-  res_start(a, S, j, leader, bd2, umax, Sj, norm2, ds);
+  res_start<false>(a, S, j, leader, bd2, umax, Sj, norm2, ds);
 }
+
+// The spare warp's registers come out of the others' loads in flight, so where its
+// code is a call and when it fetches the maxima was measured per format and chunks
+// per warp.  us per iteration, all inlined and early / with this choice / (before
+// the maxima were exchanged, the fewest registers): start as a call, 90 000 rows of
+// up to 256 real 38.6 / 36.5 / (37.1), 150 000 complex 122 / 103 / (122), 220 000
+// complex 143 / 119 / (145), streamed complex 1 000 003 225 / 214 / (217); inlined
+// for the dictionary, Bose-Hubbard L=10 11.3 (a call 11.7) / (11.5); 4 chunks:
+// maxima as a call, 369 000 complex 163 / 154 / (160); late, 369 000 real FP64 53.0 /
+// 51.9 / (51.9).
+template <int FMT, int CPW>
+constexpr bool kStartCall = CPW == 4 ? FMT == 1 || FMT == 4 : FMT != 1;
+template <int FMT, int CPW>
+constexpr bool kMaxCall = CPW == 4 && FMT == 2;
+template <int FMT, int CPW>
+constexpr bool kEarly = CPW < 4 || FMT == 1 || FMT == 4;
 
 // End of a launch, first block: the step's coefficients beta_j = |e| sqrt((beta_j
 // / e)^2), s_j = +-1 / ||u_j|| (s_j = e s_{j-1} / beta_j); the last one is h, or
@@ -464,7 +495,10 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
 #pragma unroll
       for (int i = 0; i < CPW; ++i) w[i] = res_row<FMT, CPW == 1 ? 8 : 4>(a, tab, s0[i], s1[i], x, a.sh + xs);
     } else {
-      res_start(a, S, j, leader, bd2, umax, Sj, norm2, ds);
+      if constexpr (kStartCall<FMT, CPW>)
+        res_start_call(a, S, j, leader, bd2, umax, Sj, norm2, ds);
+      else
+        res_start<kMaxCall<FMT, CPW>>(a, S, j, leader, bd2, umax, Sj, norm2, ds);
     }
     __syncthreads();
     if (S.go_start < 0) return;
@@ -503,7 +537,8 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
       unsigned long long *maxima = sy.wmax[j & 1], word;
       res_send<kAlphaWords>(a, S, words, maxima, a.tag0 + j);
       const bool ok = res_receive<kAlphaWords>(a, words, word, ds) &&
-                      res_alpha(a, S, word, Sj, umax, maxima, a.tag0 + j, e, j, leader, G, ds);
+                      res_alpha<kEarly<FMT, CPW>, kMaxCall<FMT, CPW>>(a, S, word, Sj, umax, maxima, a.tag0 + j, e, j,
+                                                                      leader, G, ds);
       if (lane == 0) S.go = ok ? 1 : 0;
     }
     __syncthreads();
@@ -566,7 +601,7 @@ __global__ void __launch_bounds__((kResWarps + 1) * 32, 1) lanczos_resident_kern
         if (ok) norm2 = res_norm(S, word, G);
       }
       if (last && leader && ok) {
-        ok = res_max(a, maxima, a.tag0 + m, res_fetch(maxima), umax, ds);
+        ok = res_grid_max<kMaxCall<FMT, CPW>>(a, maxima, a.tag0 + m, umax, ds);
         if (umax >= kNonFinite) norm2 = __longlong_as_double(0x7ff8000000000000ll);
         if (lane == 0) {
           S.cws[m] = Sj * norm2;
@@ -738,7 +773,7 @@ __global__ void __launch_bounds__((kStreamWarps<FMT> + 1) * 32, 1)
       unsigned long long *maxima = sy.wmax[j & 1], word;
       res_send<kAlphaWords>(a, S, words, maxima, a.tag0 + j);
       const bool ok = res_receive<kAlphaWords>(a, words, word, ds) &&
-                      res_alpha(a, S, word, Sj, umax, maxima, a.tag0 + j, e, j, leader, G, ds);
+                      res_alpha<true, false>(a, S, word, Sj, umax, maxima, a.tag0 + j, e, j, leader, G, ds);
       if (lane == 0) S.go = ok ? 1 : 0;
     }
     __syncthreads();
@@ -794,7 +829,7 @@ __global__ void __launch_bounds__((kStreamWarps<FMT> + 1) * 32, 1)
         if (ok) norm2 = res_norm(S, word, G);
       }
       if (last && leader && ok) {
-        ok = res_max(a, maxima, a.tag0 + m, res_fetch(maxima), umax, ds);
+        ok = res_grid_max<false>(a, maxima, a.tag0 + m, umax, ds);
         if (umax >= kNonFinite) norm2 = __longlong_as_double(0x7ff8000000000000ll);
         if (lane == 0) {
           S.cws[m] = Sj * norm2;
